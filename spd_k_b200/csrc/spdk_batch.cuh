@@ -53,7 +53,7 @@ __device__ __forceinline__ const Item& batch_item(const Item* __restrict__ items
 }
 
 template <typename R, int D, int P, int TX, int TY, int TZ, int MODE>
-__global__ void __launch_bounds__(kThreads, kPicardBlocksPerSM<R, D, P, MODE>)
+__global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_blocks<R, D, P, TX, TY, TZ, MODE>())
     picard_batched(const BatchItem<PicardArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
     long long b;
     const BatchItem<PicardArgsT<R>>& it = batch_item(items, n, &b);
@@ -97,19 +97,27 @@ struct BatchSetT {
     void (*flux)(const BatchItem<PicardArgsT<R>>*, int, DevMatsT<R>) = nullptr;
     void (*detect)(const BatchItem<DetectArgs>*, int) = nullptr;
     void (*update)(const BatchItem<FallbackArgsT<R>>*, int, DevMatsT<R>) = nullptr;
-    size_t picard_smem = 0, update_smem = 0;
-    int tile[3] = {1, 1, 1};
+    size_t picard_smem[3] = {0, 0, 0}, update_smem = 0;  // predict, correct, flux
+    int picard_threads = kThreads;
+    int picard_tile[3] = {1, 1, 1};  // a Picard block's elements (may hang over a domain's edge)
+    int tile[3] = {1, 1, 1};         // a detect / update block's elements
 };
 
 template <typename R, int P, int TX, int TY>
 BatchSetT<R> make_batch_set() {
     BatchSetT<R> k;
-    k.predict = picard_batched<R, 2, P, TX, TY, 1, kPredict>;
-    k.correct = picard_batched<R, 2, P, TX, TY, 1, kCorrect>;
-    k.flux = picard_batched<R, 2, P, TX, TY, 1, kFlux>;
+    constexpr int PX = kLineTX<P>, PY = kLineTY<P>;
+    k.predict = picard_batched<R, 2, P, PX, PY, 1, kPredict>;
+    k.correct = picard_batched<R, 2, P, PX, PY, 1, kCorrect>;
+    k.flux = picard_batched<R, 2, P, PX, PY, 1, kFlux>;
+    k.picard_threads = picard_threads<R, 2, P, PX, PY>();
+    k.picard_tile[0] = PX;
+    k.picard_tile[1] = PY;
     k.detect = detect_batched<R, 2, P, TX, TY, 1>;
     k.update = update_batched<R, 2, P, TX, TY, 1>;
-    k.picard_smem = picard_smem_bytes<R, 2, P, TX, TY, 1>();
+    k.picard_smem[kPredict] = picard_smem_bytes<R, 2, P, PX, PY, 1, kPredict>();
+    k.picard_smem[kCorrect] = picard_smem_bytes<R, 2, P, PX, PY, 1, kCorrect>();
+    k.picard_smem[kFlux] = picard_smem_bytes<R, 2, P, PX, PY, 1, kFlux>();
     k.update_smem = UpdateSmem<R, 2, P, TX, TY, 1>::bytes;
     k.tile[0] = TX;
     k.tile[1] = TY;

@@ -103,14 +103,18 @@ template <typename R>
 int plan_group(spdk_batch* b, Group& g) {
     free_tables(g);
     const int n = (int)g.members.size();
-    std::vector<long long> first(n);
-    long long total = 0;
+    // first block of every member, in the Picard and the detect / update launches
+    std::vector<long long> pfirst(n), first(n);
+    long long ptotal = 0, total = 0;
+    const int* ptile = set_of<R>(g).picard_tile;
     for (int q = 0; q < n; q++) {
         const spdk_hydro* h = b->probs[g.members[q]];
+        pfirst[q] = ptotal;
+        ptotal += tile_blocks(2, h->G.N, ptile);
         first[q] = total;
         total += (long long)(h->G.N[0] / g.tile) * (h->G.N[1] / g.tile);
     }
-    const unsigned blocks = (unsigned)total;
+    const unsigned pblocks = (unsigned)ptotal, blocks = (unsigned)total;
     const int nt = b->probs[g.members[0]]->nt;
     std::vector<const R*> in(n);
     std::vector<int> in_slices(n, 1);
@@ -121,7 +125,7 @@ int plan_group(spdk_batch* b, Group& g) {
         it.G = h->G;
         it.G.elem_trouble = nullptr;  // no per-step labels in the batch
         it.G.elem_pred = nullptr;
-        it.first = first[q];
+        it.first = pfirst[q];
         it.A.u = (const R*)h->u;
         it.A.dt = h->dt;
         return it;
@@ -138,7 +142,7 @@ int plan_group(spdk_batch* b, Group& g) {
             in[q] = (const R*)h->ua[i % 2];
             in_slices[q] = nt;
         }
-        rc = upload_pass(g, kPassPredict, blocks, items);
+        rc = upload_pass(g, kPassPredict, pblocks, items);
     }
     if (rc) return rc;
     if (!b->fallback) {
@@ -155,7 +159,7 @@ int plan_group(spdk_batch* b, Group& g) {
             items[q].A.wcv = (R*)h->wcv;
             items[q].A.dtmin = h->dtmin;
         }
-        return upload_pass(g, kPassCorrect, blocks, items);
+        return upload_pass(g, kPassCorrect, pblocks, items);
     }
     {
         std::vector<BatchItem<PicardArgsT<R>>> items(n);
@@ -169,7 +173,7 @@ int plan_group(spdk_batch* b, Group& g) {
             items[q].A.rp_old = h->rpo;
             items[q].A.rp_new = h->rpn;
         }
-        if ((rc = upload_pass(g, kPassFlux, blocks, items))) return rc;
+        if ((rc = upload_pass(g, kPassFlux, pblocks, items))) return rc;
     }
     for (int t = 0; t < nt && !rc; t++) {
         std::vector<BatchItem<DetectArgs>> det(n);
@@ -179,10 +183,10 @@ int plan_group(spdk_batch* b, Group& g) {
             const BatchItem<PicardArgsT<R>> bq = base(q);
             det[q].G = bq.G;
             if (b->labels) det[q].G.elem_trouble = h->elem_trouble;
-            det[q].first = bq.first;
+            det[q].first = first[q];
             det[q].A = DetectArgs{h->rpo, h->rpn, h->trouble};
             up[q].G = bq.G;
-            up[q].first = bq.first;
+            up[q].first = first[q];
             FallbackArgsT<R>& F = up[q].A;
             F = FallbackArgsT<R>{};
             F.ucv_in = (R*)h->ucv[t % 2];
@@ -215,8 +219,9 @@ int plan_group(spdk_batch* b, Group& g) {
 template <typename R>
 int set_batch_attributes(const BatchSetT<R>& k) {
     const void* fns[] = {(const void*)k.predict, (const void*)k.correct, (const void*)k.flux};
-    for (const void* f : fns) {
-        BCUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.picard_smem));
+    for (int m = 0; m < 3; m++) {
+        const void* f = fns[m];
+        BCUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.picard_smem[m]));
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
     BCUDA(cudaFuncSetAttribute((const void*)k.update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.update_smem));
@@ -251,9 +256,9 @@ int launch_group_t(spdk_batch* b, const Group& g, cudaStream_t st) {
         const DI* di = static_cast<const DI*>(p.items);
         const UI* ui = static_cast<const UI*>(p.items);
         switch (p.kind) {
-        case kPassPredict: k.predict<<<p.blocks, kThreads, k.picard_smem, st>>>(pi, p.n, dm); break;
-        case kPassCorrect: k.correct<<<p.blocks, kThreads, k.picard_smem, st>>>(pi, p.n, dm); break;
-        case kPassFlux: k.flux<<<p.blocks, kThreads, k.picard_smem, st>>>(pi, p.n, dm); break;
+        case kPassPredict: k.predict<<<p.blocks, k.picard_threads, k.picard_smem[kPredict], st>>>(pi, p.n, dm); break;
+        case kPassCorrect: k.correct<<<p.blocks, k.picard_threads, k.picard_smem[kCorrect], st>>>(pi, p.n, dm); break;
+        case kPassFlux: k.flux<<<p.blocks, k.picard_threads, k.picard_smem[kFlux], st>>>(pi, p.n, dm); break;
         case kPassDetect: k.detect<<<p.blocks, kThreads, 0, st>>>(di, p.n); break;
         case kPassUpdate: k.update<<<p.blocks, kThreads, k.update_smem, st>>>(ui, p.n, dm); break;
         }

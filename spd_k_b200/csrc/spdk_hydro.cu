@@ -94,16 +94,12 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-unsigned grid_blocks(const spdk_hydro* h) {
-    long long b = 1;
-    for (int d = 0; d < h->D; d++) b *= h->G.N[d] / h->tile[d];
-    return (unsigned)b;
-}
-
 // launches of one step, recorded on h->stream (also used for capture)
 template <typename R>
 int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm) {
-    const unsigned blocks = grid_blocks(h);
+    const unsigned pblocks = tile_blocks(h->D, h->G.N, k.picard_tile);
+    const unsigned blocks = tile_blocks(h->D, h->G.N, k.tile);
+    const dim3 pthreads(k.picard_threads);
     int launches = 0;
     // viscous face fluxes of a pass's input, written just before the pass
     auto viscous = [&](PicardArgsT<R>& A) -> int {
@@ -148,7 +144,7 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.ua_out = ua[it % 2];
             if (int rc = viscous(A)) return rc;
             prof_begin(h);
-            SPDK_CUDA(launch_pdl(k.predict, dim3(blocks), dim3(kThreads), k.picard_smem, h->stream, h->G, dm, A));
+            SPDK_CUDA(launch_pdl(k.predict, dim3(pblocks), pthreads, k.picard_smem[kPredict], h->stream, h->G, dm, A));
             prof_end(h, SPDK_KERNEL_PREDICT);
             launches++;
             in = ua[it % 2];
@@ -165,7 +161,7 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.wcv = (R*)h->wcv;
             A.dtmin = h->dtmin;
             prof_begin(h);
-            SPDK_CUDA(launch_pdl(k.correct, dim3(blocks), dim3(kThreads), k.picard_smem, h->stream, h->G, dm, A));
+            SPDK_CUDA(launch_pdl(k.correct, dim3(pblocks), pthreads, k.picard_smem[kCorrect], h->stream, h->G, dm, A));
             prof_end(h, SPDK_KERNEL_CORRECT);
             launches++;
         } else {
@@ -174,7 +170,7 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.rp_old = h->rpo;
             A.rp_new = h->rpn;
             prof_begin(h);
-            SPDK_CUDA(launch_pdl(k.flux, dim3(blocks), dim3(kThreads), k.picard_smem, h->stream, h->G, dm, A));
+            SPDK_CUDA(launch_pdl(k.flux, dim3(pblocks), pthreads, k.picard_smem[kFlux], h->stream, h->G, dm, A));
             prof_end(h, SPDK_KERNEL_FLUX);
             launches++;
             if (h->join_pending) {
@@ -311,9 +307,10 @@ __global__ void narrow_kernel(const double* __restrict__ a, float* __restrict__ 
 template <typename R>
 int set_attributes(const KernelSetT<R>& ks) {
     const void* fns[] = {(const void*)ks.predict, (const void*)ks.correct, (const void*)ks.flux};
-    for (const void* f : fns) {
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem) != cudaSuccess)
-            return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(ks.picard_smem) + " bytes");
+    for (int m = 0; m < 3; m++) {
+        const void* f = fns[m];
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem[m]) != cudaSuccess)
+            return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(ks.picard_smem[m]) + " bytes");
         // the whole unified L1/shared array as shared memory: residency is
         // limited by shared memory, not by L1 (staging goes through TMA)
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -400,11 +397,6 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
         delete h;
         return fail(SPDK_E_ARG, "no kernel instantiation for this ndim/p");
     }
-    // the step kernels' tile (their launch grid): the kernel set of the run's
-    // arithmetic; the FP64 set of an FP32 run only serves the element-local
-    // set-up kernels, and the two sets may choose different tiles
-    for (int d = 0; d < 3; d++)
-        h->tile[d] = h->prec == SPDK_PRECISION_FP32 ? h->ks32.tile[d] : h->ks64.tile[d];
     int rc = cudaSetDevice(c.device) == cudaSuccess ? 0 : fail(SPDK_E_CUDA, "cudaSetDevice failed");
     if (rc) { delete h; return rc; }
     build_matrices(c.p, ader, &h->mats);
@@ -430,6 +422,7 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
         const double* src = (const double*)&h->dm64;
         float* dst = (float*)&h->dm32;
         for (size_t q = 0; q < sizeof(h->dm64) / sizeof(double); q++) dst[q] = (float)src[q];
+        for (int q = 0; q < h->nt * h->nt; q++) h->dm32.pred[q] = h->dm32.invader[q] * h->dm32.wt[q % h->nt];
     }
     // grid
     DevGrid& G = h->G;
@@ -437,16 +430,10 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
     for (int d = 0; d < 3; d++) {
         G.N[d] = N[d];
         G.bc[d] = c.bc[d];
-        G.h[d] = h->ax[d].h;
-        int ex = 0;
-        const double m = std::frexp(G.h[d], &ex);
-        G.pow2[d] = (m == 0.5) ? 1 : 0;
-        G.rh[d] = G.pow2[d] ? std::ldexp(1.0, 1 - ex) : 0.0;
         G.g[d] = c.g[d];
     }
-    G.uniform_pow2 = 1;
-    for (int d = 0; d < D; d++)
-        if (!G.pow2[d] || G.h[d] != G.h[0]) G.uniform_pow2 = 0;
+    const double width[3] = {h->ax[0].h, h->ax[1].h, h->ax[2].h};
+    set_spacing(G, D, width, h->dm64.dfp_to_sp, n * nf);
     G.gm = c.gamma;
     G.cfl = c.cfl;
     G.grav = (c.g[0] != 0.0 || c.g[1] != 0.0 || c.g[2] != 0.0) ? 1 : 0;

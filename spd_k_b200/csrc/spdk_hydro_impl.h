@@ -30,7 +30,6 @@ struct spdk_hydro {
     DevGrid G{};
     KernelSetT<double> ks64;           // FP64 kernels (also the FP32 form's set-up)
     KernelSetT<float> ks32;
-    int tile[3] = {1, 1, 1};
     cudaStream_t stream = nullptr;
     // state buffers hold doubles (plain form) or floats (precision form)
     void *u = nullptr, *ua[2] = {nullptr, nullptr}, *u0 = nullptr, *ucv[2] = {nullptr, nullptr};

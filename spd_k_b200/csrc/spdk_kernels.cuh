@@ -35,6 +35,7 @@ struct DevMatsT {
     R cv_to_sp[kMaxNd * kMaxNd];
     R invader[kMaxNd * kMaxNd];     // [nt][nt]
     R wt[kMaxNd];
+    R pred[kMaxNd * kMaxNd];        // invader(t,l) w_l (precision form)
 };
 using DevMats = DevMatsT<double>;
 
@@ -42,6 +43,8 @@ struct DevGrid {
     int N[3];
     int bc[3];
     double h[3], rh[3];
+    double ih[3], ihl[3];  // 1/h rounded to nearest, and what it lacks of 1/h
+    int safe_div;          // the derivative coefficients allow divisions by h from ih, ihl (div_const)
     int pow2[3];
     int uniform_pow2;  // all active h equal and a power of two
     double gm, cfl;
@@ -226,7 +229,7 @@ __device__ __forceinline__ double point_dt(const DevGrid& G, const R* wr, int n)
 // block-wide min of positive doubles, then one atomic per block (the order
 // of a min never changes its value)
 __device__ __forceinline__ void block_min_dt(double v, unsigned long long* out) {
-    __shared__ double red[kThreads / 32];
+    __shared__ double red[32];
     for (int o = 16; o > 0; o >>= 1) v = smin(v, __shfl_xor_sync(0xffffffffu, v, o));
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     if (l == 0) red[w] = v;
@@ -520,26 +523,12 @@ __device__ __forceinline__ void picard_face_item(const DevGrid& G, const DevMats
     }
 }
 
-// resident blocks per SM the register allocation is sized for: 2 (128
-// registers a thread); for the FP32 form in 2D, whose per-point slices take
-// half the registers of FP64, 4 (64) at p <= 2, 5 (48) at p = 3 and 3 (80)
-// above, where
-// the extra resident warps outweigh a few spilled registers (measured on
-// B200: 159 us against 178 us per predictor pass at 256^2 going from 2 to
-// 4 blocks; from 4 to 5 blocks, 16 / 8 bytes of spills in the predictor /
-// corrector, 0.798 against 0.812 ms per FP32 blast step at 256^2; p = 2 at
-// 4 blocks and p = 5 at 3, without spills: blast steps 0.328 -> 0.285 ms
-// at 192^2 p=2, 1.635 -> 1.340 ms at 128^2 p=5, the first 16 problems of
-// the batched ensemble 43.6 -> 37.6 ms). The
-// flux pass keeps no per-slice registers (FP32 5 blocks: 159 against 167
-// us; FP64 3 blocks: 338 against 376 us). The FP64 2D predictor and
-// corrector at p = 3 take 3 blocks too (80 registers, 184 / 88 bytes of
-// spills): 1.704 against 1.717 ms per plain FP64 step at 256^2. The FP32
-// 3D passes at p <= 3 (2x1x1 tiles, 23-52 KB of shared memory) take 3
-// blocks (80 registers, at most 52 bytes of spills): steps 7.30 -> 6.42 ms
-// (40^3 p=2 blast), 3.58 -> 3.43 ms (24^3 p=3 KH), 4.63 -> 4.60 ms (32^3
-// p=3 blast).
-// In 3D at p = 5 the FP64 passes' 161 KB of shared memory admit one block
+// resident blocks per SM the register allocation of the 3D pass is sized
+// for: 2 (128 registers a thread). The FP32 passes at p <= 3 (2x1x1 tiles,
+// 23-52 KB of shared memory) take 3 (80 registers, at most 52 bytes of
+// spills): steps 7.30 -> 6.42 ms (40^3 p=2 blast), 3.58 -> 3.43 ms (24^3 p=3
+// KH), 4.63 -> 4.60 ms (32^3 p=3 blast).
+// At p = 5 the FP64 passes' 161 KB of shared memory admit one block
 // per SM anyway, so they take the whole register file instead of spilling
 // at 128 registers.
 // The FP64 3D passes on 2x2x1-element tiles (p = 2, 3) are compiled for one
@@ -551,12 +540,8 @@ __device__ __forceinline__ void picard_face_item(const DevGrid& G, const DevMats
 // staging and disabling the first-pass shortcut did not change the spilled
 // build's results; the tile index arithmetic was checked against the
 // oracle at p = 1 and p = 3 on the same tiles.
-template <typename R, int D, int P, int MODE, int NE = 1>
-constexpr int kPicardBlocksPerSM = (sizeof(R) == 4 && D == 2)
-                                       ? (P == 3 ? 5 : (P == 2 ? 4 : 3))
-                                       : (sizeof(R) == 8 && D == 3 && (P >= 5 || (NE >= 4 && P >= 2)))
-                                             ? 1
-                                             : (D == 2 && P == 3 ? 3 : ((sizeof(R) == 4 && D == 3 && P <= 3) ? 3 : 2));
+template <typename R, int P, int NE>
+constexpr int kPicard3BlocksPerSM = sizeof(R) == 8 ? ((P >= 5 || (NE >= 4 && P >= 2)) ? 1 : 2) : (P <= 3 ? 3 : 2);
 
 // flux-point buffers of a Picard pass (alternated between slices when 2)
 template <typename R>
@@ -1018,21 +1003,35 @@ __device__ __forceinline__ void picard_kernel_body(const DevGrid& G, const DevMa
 
 namespace spdk {
 
+// threads and resident blocks of a pass: the 2D pass by its lines, the 3D
+// pass kThreads
+template <typename R, int D, int P, int TX, int TY>
+constexpr int picard_threads() {
+    if constexpr (D == 2) return Line2<R, P, TX, TY, kFlux>::threads;
+    else return kThreads;
+}
+template <typename R, int D, int P, int TX, int TY, int TZ, int MODE>
+constexpr int picard_blocks() {
+    if constexpr (D == 2) return kLineBlocksPerSM<R, P, MODE>;
+    else return kPicard3BlocksPerSM<R, P, TX * TY * TZ>;
+}
+
 // VISC: instantiation that adds the viscous interface fluxes (hydro/nu > 0);
 // the inviscid kernels carry none of that code. 2D runs take the
 // line-organised pass of spdk_picard2d.cuh.
 template <typename R, int D, int P, int TX, int TY, int TZ, int MODE, bool VISC = false>
-__global__ void __launch_bounds__(kThreads, kPicardBlocksPerSM<R, D, P, MODE, TX * TY * TZ>) picard_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
+__global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_blocks<R, D, P, TX, TY, TZ, MODE>())
+    picard_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
     pdl_wait();
     if (gate_closed(G)) return;
     if constexpr (D == 2) picard2d_body<R, P, TX, TY, MODE, VISC>(G, M, A, blockIdx.x);
     else picard_kernel_body<R, D, P, TX, TY, TZ, MODE, VISC>(G, M, A, blockIdx.x);
 }
 
-template <typename R, int D, int P, int TX, int TY, int TZ>
+template <typename R, int D, int P, int TX, int TY, int TZ, int MODE>
 constexpr size_t picard_smem_bytes() {
     if constexpr (D == 2) {
-        return Smem2<R, P, TX, TY>::bytes;
+        return Line2<R, P, TX, TY, MODE>::bytes;
     } else {
         using S = Shape<D, P>;
         using TL = Tile<D, TX, TY, TZ>;

@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "spdk_fallback.cuh"
 #include "spdk_kernels.cuh"
 #include "spdk_viscous.cuh"
@@ -140,8 +142,10 @@ struct KernelSetT {
     void (*init)(DevGrid, DevMatsT<R>, const R*, R*, unsigned long long*) = nullptr;
     void (*derive)(DevGrid, DevMatsT<R>, const R*, R*, unsigned long long*) = nullptr;
     void (*visc)(DevGrid, DevMatsT<R>, ViscArgsT<R>) = nullptr;
-    size_t picard_smem = 0, update_smem = 0;
-    int tile[3] = {1, 1, 1};
+    size_t picard_smem[3] = {0, 0, 0}, update_smem = 0;  // predict, correct, flux
+    int picard_threads = kThreads;
+    int picard_tile[3] = {1, 1, 1};  // elements of a Picard pass's block (2D: may hang over the domain's edge)
+    int tile[3] = {1, 1, 1};         // elements of a detect / update block
     int visc_epb = 1;  // elements per block of the viscous face kernel
 };
 using KernelSet = KernelSetT<double>;
@@ -149,21 +153,58 @@ using KernelSet = KernelSetT<double>;
 template <typename R, int D, int P, int TX, int TY, int TZ, bool VISC = false>
 KernelSetT<R> make_set() {
     KernelSetT<R> k;
-    k.predict = picard_kernel<R, D, P, TX, TY, TZ, kPredict, VISC>;
-    k.correct = picard_kernel<R, D, P, TX, TY, TZ, kCorrect, VISC>;
-    k.flux = picard_kernel<R, D, P, TX, TY, TZ, kFlux, VISC>;
+    constexpr int PX = D == 2 ? kLineTX<P> : TX, PY = D == 2 ? kLineTY<P> : TY;
+    k.predict = picard_kernel<R, D, P, PX, PY, TZ, kPredict, VISC>;
+    k.correct = picard_kernel<R, D, P, PX, PY, TZ, kCorrect, VISC>;
+    k.flux = picard_kernel<R, D, P, PX, PY, TZ, kFlux, VISC>;
+    k.picard_threads = picard_threads<R, D, P, PX, PY>();
+    k.picard_tile[0] = PX;
+    k.picard_tile[1] = PY;
+    k.picard_tile[2] = TZ;
     k.detect = fv_detect_kernel<R, D, P, TX, TY, TZ>;
     k.update = fv_update_kernel<R, D, P, TX, TY, TZ>;
     k.init = init_state_kernel<R, D, P>;
     k.derive = derive_kernel<R, D, P>;
     k.visc = visc_face_kernel<R, D, P>;
     k.visc_epb = ViscShape<R, D, P>::EPB;
-    k.picard_smem = picard_smem_bytes<R, D, P, TX, TY, TZ>();
+    k.picard_smem[kPredict] = picard_smem_bytes<R, D, P, PX, PY, TZ, kPredict>();
+    k.picard_smem[kCorrect] = picard_smem_bytes<R, D, P, PX, PY, TZ, kCorrect>();
+    k.picard_smem[kFlux] = picard_smem_bytes<R, D, P, PX, PY, TZ, kFlux>();
     k.update_smem = UpdateSmem<R, D, P, TX, TY, TZ>::bytes;
     k.tile[0] = TX;
     k.tile[1] = TY;
     k.tile[2] = TZ;
     return k;
+}
+
+// blocks of tiles that cover the domain
+inline unsigned tile_blocks(int D, const int N[3], const int tile[3]) {
+    long long b = 1;
+    for (int d = 0; d < D; d++) b *= (N[d] + tile[d] - 1) / tile[d];
+    return (unsigned)b;
+}
+
+// element widths, their reciprocals and powers of two (G.N, D and the box
+// lengths given), and whether every derivative coefficient is zero or far
+// from under- and overflow (div_const)
+inline void set_spacing(DevGrid& G, int D, const double h[3], const double* dfp_to_sp, int coefs) {
+    G.uniform_pow2 = 1;
+    G.safe_div = 1;
+    for (int d = 0; d < 3; d++) {
+        G.h[d] = h[d];
+        int ex = 0;
+        const double m = std::frexp(h[d], &ex);
+        G.pow2[d] = m == 0.5 ? 1 : 0;
+        G.rh[d] = G.pow2[d] ? std::ldexp(1.0, 1 - ex) : 0.0;
+        G.ih[d] = 1.0 / h[d];
+        G.ihl[d] = std::fma(-h[d], G.ih[d], 1.0) * G.ih[d];
+        if (d < D && (!G.pow2[d] || h[d] != h[0])) G.uniform_pow2 = 0;
+        if (d < D && !(h[d] > 1e-30 && h[d] < 1e30)) G.safe_div = 0;
+    }
+    for (int q = 0; q < coefs; q++) {
+        const double a = std::fabs(dfp_to_sp[q]);
+        if (a != 0.0 && !(a > 1e-30 && a < 1e30)) G.safe_div = 0;
+    }
 }
 
 // Tile choice: the largest instantiated tile that divides the element counts.

@@ -83,8 +83,9 @@ int setup_device(int dev, const KernelSet& ks, void** base) {
     }
     // per-kernel attributes (idempotent, not an allocation)
     const void* fns[] = {(const void*)ks.predict, (const void*)ks.correct};
-    for (const void* f : fns) {
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem);
+    for (int m = 0; m < 2; m++) {
+        const void* f = fns[m];
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem[m]);
         if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
@@ -157,16 +158,10 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
     for (int d = 0; d < 3; d++) {
         G.N[d] = N[d];
         G.bc[d] = c.bc[d];
-        G.h[d] = c.L[d] / N[d];
-        int ex = 0;
-        const double m = std::frexp(G.h[d], &ex);
-        G.pow2[d] = (m == 0.5) ? 1 : 0;
-        G.rh[d] = G.pow2[d] ? std::ldexp(1.0, 1 - ex) : 0.0;
         G.g[d] = c.g[d];
     }
-    G.uniform_pow2 = 1;
-    for (int d = 0; d < D; d++)
-        if (!G.pow2[d] || G.h[d] != G.h[0]) G.uniform_pow2 = 0;
+    const double width[3] = {c.L[0] / N[0], c.L[1] / N[1], c.L[2] / N[2]};
+    set_spacing(G, D, width, dm.dfp_to_sp, n * nf);
     G.gm = c.gamma;
     G.cfl = c.cfl;
     G.grav = (c.g[0] != 0.0 || c.g[1] != 0.0 || c.g[2] != 0.0) ? 1 : 0;
@@ -175,8 +170,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
     G.status = status;
 
     cudaStream_t s = (cudaStream_t)stream;
-    long long blocks = 1;
-    for (int d = 0; d < D; d++) blocks *= N[d] / ks.tile[d];
+    const unsigned blocks = tile_blocks(D, N, ks.picard_tile);
     noalloc_arm<<<1, 1, 0, s>>>(dtmin, status);
     double rk_a[3] = {0, 0, 0};
     if (c.rk_order == 2) rk_a[1] = 0.5;
@@ -192,7 +186,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
             A.ua_in = in;
             A.in_slices = in_slices;
             A.ua_out = ua[it % 2];
-            ks.predict<<<(unsigned)blocks, kThreads, ks.picard_smem, s>>>(G, dm, A);
+            ks.predict<<<blocks, ks.picard_threads, ks.picard_smem[kPredict], s>>>(G, dm, A);
             in = ua[it % 2];
             in_slices = nt;
         }
@@ -202,7 +196,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
         A.final_stage = 1;
         A.wcv = wcv_out;
         A.dtmin = dtmin;
-        ks.correct<<<(unsigned)blocks, kThreads, ks.picard_smem, s>>>(G, dm, A);
+        ks.correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
     } else {
         double* stage_in = work;
         double* u0 = work + (size_t)E * V * NPT;
@@ -224,7 +218,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
             A.wcv = wcv_out;
             A.dtmin = dtmin;
             A.dt = dt_inout;
-            ks.correct<<<(unsigned)blocks, kThreads, ks.picard_smem, s>>>(G, dm, A);
+            ks.correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
             cur = u_out;
         }
     }

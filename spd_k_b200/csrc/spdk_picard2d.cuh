@@ -1,146 +1,189 @@
-// Fused Picard pass of 2D runs: balanced interface / interior flux points
-// and a register-blocked flux divergence.
+// Fused Picard pass of 2D runs: one thread per solution-point line.
 //
-// Same inputs, outputs and arithmetic as picard_kernel_body (spdk_kernels.cuh),
-// reorganised so that operands are read once:
+// Same inputs, outputs and FP64 arithmetic as picard_kernel_body
+// (spdk_kernels.cuh), organised by lines:
 //
-// * Phase A (fluxes at the flux points of one slice). Interfaces (both
-//   sides extrapolated, ghost image at a non-periodic edge, LLF) take one
-//   thread each; interior flux points are shared by the remaining threads,
-//   ordered by (direction, flux point) so that a warp's points read the same
-//   interpolation coefficients (one broadcast shared-memory word); x lines
-//   are loaded as 16-byte vectors.
-// * Phase B (divergence at the solution points). A thread owns a BX x BY block
-//   of solution points of one variable of one element, for the whole pass:
-//   every x-flux value it reads serves BX points, every y-flux value BY
-//   points; items are ordered block-major, so a warp's derivative
-//   coefficients are broadcast words too. Each point's sum keeps the
-//   reference's order (flux points outer, directions inner:
+// * Phase A (fluxes at the flux points of one slice). A thread takes one x or
+//   y line of an element, all variables: the line's low interface (its own
+//   trace, and the neighbour's from the neighbour's line) and its interior
+//   flux points. The interpolation coefficients are compile-time offsets of
+//   the kernel parameters, and a line is read twice instead of once per flux
+//   point. The interfaces on the tile's high edges, which no line of the tile
+//   owns, go to one more warp or two, so that no thread solves two.
+// * Phase B (divergence at the solution points). A thread owns one row of
+//   points of V / H variables of one element for the whole pass: the x
+//   fluxes of the row and all y fluxes of the element are read as vectors,
+//   the x coefficients are constant bank operands. Each point's sum keeps
+//   the reference's order (flux points outer, directions inner:
 //   src/transforms.cpp:296-303), so the FP64 plain form is unchanged bit for
-//   bit.
-// * Epilogues. The step-start state of the tile is staged point-major by
-//   coalesced loads while slice 0 arrives; results are assembled in shared
-//   memory and written back with coalesced 16-byte stores.
+//   bit; the precision form scales the sum once.
+// * Rows are contiguous in memory, so the step-start state is read and the
+//   slices are written straight from registers (16-byte vectors where a row
+//   is whole vectors).
+// * Tiles at the high edges may hang over the domain: their outside elements
+//   are staged as periodic images (or not at all), take part in nothing
+//   that is stored, and any element counts run on the same tiles.
+//
+// What bounds it: instruction issue (the point-per-thread pass before it read
+// every line nf - 2 + 2 times through shared memory with its coefficients,
+// and ran 2.2 of 4 issue slots).
 #pragma once
 #include <type_traits>
 
 namespace spdk {
 
-// point block of the 2D divergence: BX x BY points of one variable per thread
-template <int n>
-struct DivBlock2 {
-    static constexpr int BX = n == 2 ? 2 : n == 3 ? 3 : n == 4 ? 2 : n == 5 ? 5 : n == 6 ? 3 : n == 7 ? 1 : 2;
-    static constexpr int BY = (n == 4 || n == 8) ? 2 : 1;
-    static constexpr int NBX = n / BX, NBY = n / BY;
-    static constexpr int NB = NBX * NBY;
-};
+// 16-byte vector of R
+template <typename R> struct Vec16;
+template <> struct Vec16<float> { using T = float4; };
+template <> struct Vec16<double> { using T = double2; };
 
-// interfaces of a TX x TY tile per direction: (faces along d) x (rows or columns) x n
-template <int P, int TX, int TY>
-struct Lines2 {
-    static constexpr int n = P + 1;
-    static constexpr int L0 = (TX + 1) * TY * n;
-    static constexpr int L1 = (TY + 1) * TX * n;
-};
+// the widest vector (in values) that divides a row of n values: 16 or 8 bytes, or single values
+template <typename R, int n>
+constexpr int kRowVec = sizeof(R) == 4 ? (n % 4 == 0 ? 4 : (n % 2 == 0 ? 2 : 1)) : (n % 2 == 0 ? 2 : 1);
 
-// shared-memory layout of the 2D pass (in elements of R): staging buffers,
-// flux-point buffers; the epilogues' buffers reuse that space. Values that
-// phase-B threads read or write (their lanes run over element x variable at
-// a common point) sit point-major, [point][element x variable + pad], so
-// that those lanes hit distinct banks, and so do the copy-out lanes running
-// over points. The step-start state of the tile follows at the end.
-template <typename R, int P, int TX, int TY>
-struct Smem2 {
-    static constexpr int n = P + 1, NPT = n * n, V = 4, NE = TX * TY;
-    static constexpr int NS = Tile<2, TX, TY, 1>::NS;
-    static constexpr int nt = P + 1;
-    static constexpr int KS = NE * V + (sizeof(R) == 4 ? 2 : 1);  // point stride of a point-major tile
-    static constexpr size_t tsz = (size_t)NPT * KS;                // one point-major tile
-    static constexpr size_t stage = 2 * (size_t)NS * PicardPad<2, P, R>::SS;
-    static constexpr size_t fx = (size_t)kFxBuffers<R> * 2 * NE * V * PicardPad<2, P, R>::FXS;
-    static constexpr size_t out = (size_t)nt * tsz;                           // predictor slices
-    static constexpr size_t epi = 2 * (size_t)NE * V * NPT + tsz;             // corrector W_sp, scratch, U - du
-    static constexpr size_t main0 = stage + fx > out ? stage + fx : out;
-    static constexpr size_t main1 = main0 > epi ? main0 : epi;
-    static constexpr size_t ubuf = main1;                                     // point-major U of the tile
-    static constexpr size_t total = ubuf + tsz;
-    static constexpr size_t bytes = total * sizeof(R);
-};
-
-// the n values of one line of one variable's point block into registers:
-// x lines are contiguous (16-byte vectors when they are whole vectors), y
-// lines strided by n
-template <typename R, int n, int d>
-__device__ __forceinline__ void load_line(const R* src, int tp, R (&u)[n]) {
-    constexpr int VW = 16 / (int)sizeof(R);
-    if constexpr (d == 0 && n % VW == 0) {
-        using VT = typename std::conditional<sizeof(R) == 4, float4, double2>::type;
-        const VT* p = reinterpret_cast<const VT*>(src + n * tp);
+// n consecutive values between memory and registers
+template <typename R, int n>
+__device__ __forceinline__ void row_load(const R* p, R* out) {
+    constexpr int W = kRowVec<R, n>;
+    if constexpr (W == 1) {
 #pragma unroll
-        for (int c = 0; c < n / VW; c++) {
-            __align__(16) R t[VW];
-            *reinterpret_cast<VT*>(t) = p[c];
-#pragma unroll
-            for (int w = 0; w < VW; w++) u[c * VW + w] = t[w];
-        }
+        for (int i = 0; i < n; i++) out[i] = p[i];
     } else {
+        using VT = typename std::conditional<W * sizeof(R) == 16, typename Vec16<R>::T, float2>::type;
 #pragma unroll
-        for (int l = 0; l < n; l++) u[l] = src[d == 0 ? l + n * tp : tp + n * l];
+        for (int c = 0; c < n / W; c++) {
+            __align__(16) R t[W];
+            *reinterpret_cast<VT*>(t) = reinterpret_cast<const VT*>(p)[c];
+#pragma unroll
+            for (int w = 0; w < W; w++) out[c * W + w] = t[w];
+        }
+    }
+}
+template <typename R, int n>
+__device__ __forceinline__ void row_store(R* p, const R* in) {
+    constexpr int W = kRowVec<R, n>;
+    if constexpr (W == 1) {
+#pragma unroll
+        for (int i = 0; i < n; i++) p[i] = in[i];
+    } else {
+        using VT = typename std::conditional<W * sizeof(R) == 16, typename Vec16<R>::T, float2>::type;
+#pragma unroll
+        for (int c = 0; c < n / W; c++) {
+            __align__(16) R t[W];
+#pragma unroll
+            for (int w = 0; w < W; w++) t[w] = in[c * W + w];
+            reinterpret_cast<VT*>(p)[c] = *reinterpret_cast<const VT*>(t);
+        }
     }
 }
 
-// one element interface of direction d (phase A): the face between the
-// elements at positions f-1 and f of row/column r, at transverse point tp;
-// both sides extrapolated to the face, the ghost image at a non-periodic
-// domain edge (src/boundary.cpp:48-113), the LLF flux written to the
-// adjacent flux points of the tile's elements
-template <typename R, int P, int TX, int TY, int d, bool VISC>
-__device__ __forceinline__ void face_item2(const DevGrid& G, const DevMatsT<R>& M, const R* Ss, R* FX, const int o[3],
-                                           int q, const R* vg, const long long* sl_elem, int vt) {
-    using TL = Tile<2, TX, TY, 1>;
-    constexpr int n = P + 1, nf = P + 2, V = 4, NPT = n * n, NE = TL::NE;
-    constexpr int SS = PicardPad<2, P, R>::SS, FXS = PicardPad<2, P, R>::FXS;
-    constexpr int Td = d == 0 ? TX : TY, Tt = d == 0 ? TY : TX;
-    constexpr int NTP = n;
-    const int tp = q % n;
-    const int r = (q / n) % Tt;
-    const int f = q / (n * Tt);
-    int lL[2], lR[2];
-    lL[d] = f - 1;
-    lR[d] = f;
-    lL[1 - d] = r;
-    lR[1 - d] = r;
-    const int sL = TL::slot(lL[0], lL[1], 0), sR = TL::slot(lR[0], lR[1], 0);
-    const int gface = o[d] + f;
-    const bool ghostL = gface == 0 && G.bc[d] != kPeriodic;
-    const bool ghostR = gface == G.N[d] && G.bc[d] != kPeriodic;
-    // offset of flux point ll of the line inside a variable's flux-point block
-    auto fpo = [&](int ll) { return d == 0 ? ll + nf * tp : tp + n * ll; };
-    R uL[V], uR[V];
-    if (!ghostR) {
-        const R* src = Ss + sR * SS;
-#pragma unroll
-        for (int v = 0; v < V; v++) {
-            R ul[n];
-            load_line<R, n, d>(src + v * NPT, tp, ul);
-            R a = 0;
-#pragma unroll
-            for (int l = 0; l < n; l++) a += ul[l] * M.sp_to_fp[l];
-            uR[v] = a;
-        }
+// element stride of a flux-point array: V * NFP plus the pad (whole 16-byte
+// units) that leaves the fewest bank conflicts when a warp's lanes run over
+// the n lines of an element, then over elements
+template <typename R, int n>
+constexpr int flux_stride() {
+    constexpr int nf = n + 1, V = 4, W = (int)sizeof(R) / 4, lanes = 32 / W;
+    constexpr int base = V * n * nf;
+    int best = 0, best_c = 1 << 30;
+    for (int pad = 0; pad < 32 / W; pad += 4 / W) {
+        int cnt[32] = {};
+        for (int l = 0; l < lanes; l++) cnt[(((l % n) * nf + (l / n) * (base + pad)) * W) % 32]++;
+        int c = 0;
+        for (int b = 0; b < 32; b++) c = cnt[b] > c ? cnt[b] : c;
+        c = c * 64 + pad;
+        if (c < best_c) { best_c = c; best = pad; }
     }
-    if (!ghostL) {
-        const R* src = Ss + sL * SS;
+    return base + best;
+}
+
+// Thread organisation and shared memory of the 2D pass on TX x TY elements.
+// Phase A: the x lines, then the y lines (each padded to whole warps, so that
+// a warp runs one direction), then the interfaces on the tile's high edges.
+// Phase B: rows of points x H groups of variables.
+// A thread has registers for either the predictor's sums or the flux
+// evaluation at the occupancy that hides its latency, so the predictor keeps
+// the sums in shared memory (one private column per thread) and pays for it
+// with single staging and flux-point buffers: the next slice's copy starts
+// when phase A is over and runs under phase B. Measured per predictor pass at
+// 256^2, p = 3 (the average of a step's three): FP64 260 us with the sums in
+// registers (3 blocks, 356 bytes of spills), 198 us in shared memory (3
+// blocks); FP32 87 us in registers (4 blocks), 84 us in shared memory (6).
+template <typename R, int P, int TX, int TY, int MODE>
+struct Line2 {
+    static constexpr int n = P + 1, nf = P + 2, V = 4, NPT = n * n, NFP = n * nf, NE = TX * TY;
+    static constexpr int NS = Tile<2, TX, TY, 1>::NS;
+    static constexpr int warps(int items) { return (items + 31) / 32 * 32; }
+    static constexpr int H = P <= 3 ? 2 : 4;
+    static constexpr int VB = V / H;                           // variables of a phase-B thread
+    static constexpr int LINES = NE * n;                       // lines of one direction
+    static constexpr int LW = warps(LINES);
+    static constexpr int EDGE0 = TY * n, EDGE1 = TX * n;       // interfaces on the high x / y edge
+    static constexpr int ROWS = NE * n * H;                    // phase-B threads
+    static constexpr int A = 2 * LW + warps(EDGE0 + EDGE1);
+    static constexpr int threads = A > warps(ROWS) ? A : warps(ROWS);
+    static constexpr bool shared_sums = MODE == kPredict;
+    static constexpr int fbufs = (sizeof(R) == 8 || MODE == kPredict) ? 1 : 2;  // staging and flux-point buffers
+    static constexpr int stages = fbufs;
+    static constexpr int SS = PicardPad<2, P, R>::SS;          // staged element
+    static constexpr int FE = flux_stride<R, n>();             // flux points of an element, one direction
+    static constexpr size_t stage = (size_t)stages * NS * SS;
+    static constexpr size_t fx = (size_t)fbufs * 2 * NE * FE;
+    static constexpr size_t sums = shared_sums ? (size_t)VB * n * n * ROWS : 0;
+    static constexpr size_t grav = MODE == kPredict ? (size_t)n * 3 * NE * NPT : 0;  // predictor slices of rho, m (gravity)
+    static constexpr size_t epi = 2 * (size_t)NE * V * NPT;         // W_sp / U_sp and sweep scratch
+    static constexpr size_t m0 = stage + fx > grav ? stage + fx : grav;
+    static constexpr size_t m1 = m0 > epi ? m0 : epi;
+    static constexpr size_t bytes = (m1 + sums) * sizeof(R);
+};
+
+// tile of the 2D pass: 4 x 4 elements up to p = 3 and 4 x 2 above (160
+// threads at p = 2, 3 and 4, 192 at p = 5)
+template <int P> constexpr int kLineTX = 4;
+template <int P> constexpr int kLineTY = P <= 3 ? 4 : 2;
+
+// resident blocks per SM the 2D pass's registers are sized for
+// (threads x blocks leave 64 registers a thread at p = 3 in FP32 and 96 to 128
+// in FP64, where spills stay below 40 bytes; FP64 flux pass at p = 3: 347 us
+// at 3 blocks, 304 us at 4; FP32 predictor at p = 5: 98 us with the sums in
+// registers, 91 / 88 us in shared memory at 5 / 4 blocks)
+template <typename R, int P, int MODE>
+constexpr int kLineBlocksPerSM =
+    sizeof(R) == 4 ? (P == 1 ? 8 : P <= 3 ? (MODE == kPredict ? 6 : 5) : P == 4 ? 5 : P == 5 ? 4 : 2)
+                   : (P == 1 ? 5 : P <= 4 ? (MODE == kPredict ? 3 : 4) : P == 5 ? (MODE == kPredict ? 2 : 3) : 2);
+
+// the values of one line of one variable's point block: x lines are
+// contiguous, y lines strided by n
+template <typename R, int n, int d>
+__device__ __forceinline__ void load_line(const R* src, int tp, R (&u)[n]) {
+    if constexpr (d == 0) row_load<R, n>(src + n * tp, u);
+    else {
 #pragma unroll
-        for (int v = 0; v < V; v++) {
-            R ul[n];
-            load_line<R, n, d>(src + v * NPT, tp, ul);
-            R a = 0;
-#pragma unroll
-            for (int l = 0; l < n; l++) a += ul[l] * M.sp_to_fp[(nf - 1) * n + l];
-            uL[v] = a;
-        }
+        for (int l = 0; l < n; l++) u[l] = src[tp + n * l];
     }
+}
+
+// the state at a line's end: E = 0 low, 1 high
+template <typename R, int P, int d, int END>
+__device__ __forceinline__ void trace2(const DevMatsT<R>& M, const R* src, int tp, R (&t)[4]) {
+    constexpr int n = P + 1, NPT = n * n, o = END ? (P + 1) * n : 0;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        R ul[n];
+        load_line<R, n, d>(src + v * NPT, tp, ul);
+        R a = 0;
+#pragma unroll
+        for (int l = 0; l < n; l++) a += ul[l] * M.sp_to_fp[o + l];
+        t[v] = a;
+    }
+}
+
+// interface flux between the states of the two sides: the ghost image at a
+// non-periodic domain edge (src/boundary.cpp:48-113), LLF, and in viscous
+// runs the interface sum of the sides' viscous fluxes (src/hydro.cpp:420-455)
+template <typename R, int P, int d, bool VISC>
+__device__ __forceinline__ void interface2(const DevGrid& G, R (&uL)[4], R (&uR)[4], bool ghostL, bool ghostR, R (&F)[4],
+                                           const R* vg, int eL, int eR, int vt, int tp) {
+    constexpr int V = 4, NTP = P + 1;
     if (ghostL) {
 #pragma unroll
         for (int v = 0; v < V; v++) uL[v] = uR[v];
@@ -151,18 +194,16 @@ __device__ __forceinline__ void face_item2(const DevGrid& G, const DevMatsT<R>& 
         for (int v = 0; v < V; v++) uR[v] = uL[v];
         if (G.bc[d] == kReflective) uR[1 + d] = -uR[1 + d];
     }
-    R F[V];
     riemann_llf<2>(F, uL, uR, d, (R)G.gm);
     if constexpr (VISC) {
-        // viscous interface flux (src/hydro.cpp:420-455), as in picard_face_item
         R gL[V], gR[V];
         if (!ghostL) {
-            const R* g = vg + ((((long long)vt * G.E + sl_elem[sL]) * 2 + 1) * V) * NTP + tp;
+            const R* g = vg + ((((long long)vt * G.E + eL) * 2 + 1) * V) * NTP + tp;
 #pragma unroll
             for (int v = 0; v < V; v++) gL[v] = g[v * NTP];
         }
         if (!ghostR) {
-            const R* g = vg + ((((long long)vt * G.E + sl_elem[sR]) * 2 + 0) * V) * NTP + tp;
+            const R* g = vg + ((((long long)vt * G.E + eR) * 2 + 0) * V) * NTP + tp;
 #pragma unroll
             for (int v = 0; v < V; v++) gR[v] = g[v * NTP];
         }
@@ -179,136 +220,23 @@ __device__ __forceinline__ void face_item2(const DevGrid& G, const DevMatsT<R>& 
 #pragma unroll
         for (int v = 0; v < V; v++) F[v] += wind_mix(gR[v], gL[v], R(-0.5));
     }
-    if (f >= 1) {
-        R* dst = FX + (d * NE + sL) * V * FXS + fpo(nf - 1);
-#pragma unroll
-        for (int v = 0; v < V; v++) dst[v * FXS] = F[v];
-    }
-    if (f < Td) {
-        R* dst = FX + (d * NE + sR) * V * FXS + fpo(0);
-#pragma unroll
-        for (int v = 0; v < V; v++) dst[v * FXS] = F[v];
-    }
 }
 
-// interior flux point ll (1..nf-2) of direction d at transverse point tp of
-// tile element el (phase A): interpolation, primitives, Euler flux. The
-// coefficients come from the shared copy of sp_to_fp; a warp's items share
-// ll, so every lane reads the same word.
-template <typename R, int P, int TX, int TY, int d>
-__device__ __forceinline__ void interior_item2(const DevGrid& G, const R* Msf, const R* Ss, R* FX, int el, int ll,
-                                               int tp) {
-    constexpr int n = P + 1, nf = P + 2, V = 4, NPT = n * n, NE = TX * TY;
-    constexpr int SS = PicardPad<2, P, R>::SS, FXS = PicardPad<2, P, R>::FXS;
-    const R* src = Ss + el * SS;
-    R m[n];
-#pragma unroll
-    for (int l = 0; l < n; l++) m[l] = Msf[ll * n + l];
-    R u[V], w[V], fl[V];
-#pragma unroll
-    for (int v = 0; v < V; v++) {
-        R ul[n];
-        load_line<R, n, d>(src + v * NPT, tp, ul);
-        R a = 0;
-#pragma unroll
-        for (int l = 0; l < n; l++) a += ul[l] * m[l];
-        u[v] = a;
-    }
-    primitives<2>(u, w, (R)G.gm);
-    euler_flux<2>(u, w, fl, d);
-    R* dst = FX + (d * NE + el) * V * FXS + (d == 0 ? ll + nf * tp : tp + n * ll);
-#pragma unroll
-    for (int v = 0; v < V; v++) dst[v * FXS] = fl[v];
+// x / h for a step-constant h from its correctly rounded reciprocal y and
+// y's own remainder: q is a faithful quotient, and the exact remainder
+// x - h q times y rounds it correctly (Markstein's theorem for a quotient
+// with a fused multiply-add), for x = 0 or x far from under- and overflow
+__device__ __forceinline__ double div_const(double x, double h, double y, double yl) {
+    const double q = __fma_rn(x, y, __dmul_rn(x, yl));
+    return __fma_rn(__fma_rn(-h, q, x), y, q);
 }
-
-// divergence of one BX x BY point block of one variable (phase B): dd[j][i]
-// at point (bx0 + i, by0 + j). The sum over the flux points ll takes the
-// x term, then the y term, at each ll (the reference's order). The
-// derivative coefficients come from the shared copy of dfp_to_sp; a warp's
-// items share their block, so every lane reads the same word.
-template <typename R, int P>
-__device__ __forceinline__ void div_block2(const DevGrid& G, const R* Mdf, const R* Fx, const R* Fy, int bx0, int by0,
-                                           R (&dd)[DivBlock2<P + 1>::BY][DivBlock2<P + 1>::BX]) {
-    using DB = DivBlock2<P + 1>;
-    constexpr int n = P + 1, nf = P + 2, BX = DB::BX, BY = DB::BY;
-#pragma unroll
-    for (int j = 0; j < BY; j++)
-#pragma unroll
-        for (int i = 0; i < BX; i++) dd[j][i] = 0;
-    const bool uni = G.uniform_pow2 != 0;
-    const bool p2x = G.pow2[0] != 0, p2y = G.pow2[1] != 0;
-    const R hx = (R)G.h[0], hy = (R)G.h[1], rhx = (R)G.rh[0], rhy = (R)G.rh[1];
-#pragma unroll
-    for (int ll = 0; ll < nf; ll++) {
-        R fx[BY], fy[BX], cx[BX], cy[BY];
-#pragma unroll
-        for (int j = 0; j < BY; j++) {
-            fx[j] = Fx[ll + nf * (by0 + j)];
-            cy[j] = Mdf[(by0 + j) * nf + ll];
-        }
-#pragma unroll
-        for (int i = 0; i < BX; i++) {
-            fy[i] = Fy[(bx0 + i) + n * ll];
-            cx[i] = Mdf[(bx0 + i) * nf + ll];
-        }
-        if (uni) {
-            // every active h is the same power of two: the scaling of each
-            // term by 1/h is exact and commutes with the rounding of the sum
-#pragma unroll
-            for (int j = 0; j < BY; j++)
-#pragma unroll
-                for (int i = 0; i < BX; i++) {
-                    dd[j][i] += fx[j] * cx[i];
-                    dd[j][i] += fy[i] * cy[j];
-                }
-        } else {
-#pragma unroll
-            for (int j = 0; j < BY; j++)
-#pragma unroll
-                for (int i = 0; i < BX; i++) {
-                    dd[j][i] += div_h(fx[j] * cx[i], hx, rhx, p2x);
-                    dd[j][i] += div_h(fy[i] * cy[j], hy, rhy, p2y);
-                }
-        }
-    }
-    if (uni)
-#pragma unroll
-        for (int j = 0; j < BY; j++)
-#pragma unroll
-            for (int i = 0; i < BX; i++) dd[j][i] *= rhx;
+// whether a flux value's products with the derivative coefficients lie in
+// that range: zero, or an exponent within 700 of 1's
+__device__ __forceinline__ bool div_range(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) & 0x7ff00000u;
+    return (e - ((1023u - 700u) << 20)) < (1400u << 20) || x == 0.0;
 }
-
-// 16-byte vector of R
-template <typename R> struct Vec16;
-template <> struct Vec16<float> { using T = float4; };
-template <> struct Vec16<double> { using T = double2; };
-
-// W consecutive values (W = 1 or a 16-byte vector) between memory and registers
-template <typename R, int W>
-__device__ __forceinline__ void vload(const R* p, R* out) {
-    if constexpr (W == 1) {
-        out[0] = p[0];
-    } else {
-        using VT = typename Vec16<R>::T;
-        static_assert(W * sizeof(R) == 16, "W is one 16-byte vector");
-        __align__(16) R t[W];
-        *reinterpret_cast<VT*>(t) = *reinterpret_cast<const VT*>(p);
-#pragma unroll
-        for (int w = 0; w < W; w++) out[w] = t[w];
-    }
-}
-template <typename R, int W>
-__device__ __forceinline__ void vstore(R* p, const R* in) {
-    if constexpr (W == 1) {
-        p[0] = in[0];
-    } else {
-        using VT = typename Vec16<R>::T;
-        __align__(16) R t[W];
-#pragma unroll
-        for (int w = 0; w < W; w++) t[w] = in[w];
-        *reinterpret_cast<VT*>(p) = *reinterpret_cast<const VT*>(t);
-    }
-}
+__device__ __forceinline__ bool div_range(float) { return true; }
 
 template <typename R, int P, int TX, int TY, int MODE, bool VISC>
 __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R>& M, const PicardArgsT<R>& A,
@@ -316,55 +244,51 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
     constexpr int D = 2;
     using S = Shape<2, P>;
     using TL = Tile<2, TX, TY, 1>;
-    using DB = DivBlock2<P + 1>;
-    using LN = Lines2<P, TX, TY>;
-    using SM = Smem2<R, P, TX, TY>;
-    using VT = typename Vec16<R>::T;
+    using LN = Line2<R, P, TX, TY, MODE>;
     constexpr int n = S::n, nf = S::nf, V = S::V, NPT = S::NPT, NFP = S::NFP;
-    constexpr int NE = TL::NE, NS = TL::NS;
+    constexpr int NE = TL::NE, NS = TL::NS, NTH = LN::threads;
     constexpr int NT = MODE == kFlux ? 1 : (P + 1);
-    constexpr int SS = PicardPad<2, P, R>::SS;
-    constexpr int FXS = PicardPad<2, P, R>::FXS;
-    constexpr int NFX = kFxBuffers<R>;
-    constexpr int BX = DB::BX, BY = DB::BY, BXY = BX * BY;
-    constexpr int ITEMS = NE * V * DB::NB;                 // phase-B items
-    constexpr int IPT = (ITEMS + kThreads - 1) / kThreads;  // items per thread
-    constexpr int VW = 16 / (int)sizeof(R);                  // values per 16-byte vector
-    constexpr int CH = V * NPT / VW;                         // vectors per element chunk
-    constexpr int PW = NPT % VW == 0 ? VW : 1;               // values per transfer of a variable's points
+    constexpr int ND = MODE == kPredict ? NT : 1;  // divergence values kept per point
+    constexpr int SS = LN::SS, FE = LN::FE, VB = LN::VB, ST = LN::stages;
+    constexpr int NFX = LN::fbufs;
+    constexpr int Q = 16 / (int)sizeof(R);
+    using VT = typename Vec16<R>::T;
     static_assert((V * NPT * sizeof(R)) % 16 == 0, "2D element chunks are whole 16-byte units");
-    static_assert(SM::out <= SM::ubuf && SM::epi <= SM::ubuf, "epilogue buffers overlap the step-start state");
+    static_assert((V * NFP * sizeof(R)) % 16 == 0 && FE % Q == 0, "flux blocks are whole 16-byte units");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     R* smem = reinterpret_cast<R*>(smem_raw);
-    R* Sbuf = smem;                       // 2 x [NS][SS]
-    R* FX0 = Sbuf + 2 * NS * SS;          // [NFX][2][NE][V][FXS]
-    R* Ubuf = smem + SM::ubuf;            // [NPT][KS]: U of the tile's elements, point-major
-    constexpr int KS = SM::KS;
-    __shared__ long long sl_elem[NS];
+    R* Sbuf = smem;                       // [stages][NS][SS]
+    R* FX0 = Sbuf + LN::stage;            // [NFX][2][NE][FE]
+    __shared__ int sl_elem[NS];           // staged element (a periodic image outside the domain), -1: none
+    __shared__ int el_own[NE];            // element of the tile, -1 outside the domain
     __shared__ uint64_t bar[2];
-    __shared__ R Mcv[S::n * S::n];
-    __shared__ R Msf[S::nf * S::n];   // sp_to_fp [nf][n]
-    __shared__ R Mdf[S::n * S::nf];   // dfp_to_sp [n][nf]
 
     const int tid = threadIdx.x;
-    for (int i = tid; i < S::n * S::n; i += kThreads) Mcv[i] = M.sp_to_cv[i];
-    for (int i = tid; i < S::nf * S::n; i += kThreads) {
-        Msf[i] = M.sp_to_fp[i];
-        Mdf[i] = M.dfp_to_sp[i];
-    }
-    int o[3];
+    int o[2];
     {
-        int b = (int)bidx;
-        const int tx = G.N[0] / TX;
-        o[0] = (b % tx) * TX;
-        o[1] = (b / tx) * TY;
-        o[2] = 0;
+        const int tx = (G.N[0] + TX - 1) / TX;
+        o[0] = ((int)bidx % tx) * TX;
+        o[1] = ((int)bidx / tx) * TY;
     }
-    for (int s = tid; s < NS; s += kThreads) {
+    for (int s = tid; s < NS; s += NTH) {
         int l[3];
         TL::coords(s, l);
-        sl_elem[s] = elem_of<2>(G, o, l);
+        int g[2];
+        bool none = false;
+#pragma unroll
+        for (int d = 0; d < 2; d++) {
+            g[d] = o[d] + l[d];
+            if (g[d] < 0 || g[d] >= G.N[d]) {
+                none |= G.bc[d] != kPeriodic;
+                g[d] = (g[d] + G.N[d]) % G.N[d];
+            }
+        }
+        sl_elem[s] = none ? -1 : g[1] * G.N[0] + g[0];
+        if (s < NE) {
+            const int gx = o[0] + l[0], gy = o[1] + l[1];
+            el_own[s] = gx < G.N[0] && gy < G.N[1] ? gy * G.N[0] + gx : -1;
+        }
     }
     if (tid == 0) {
         mbar_init(&bar[0], 1);
@@ -372,279 +296,412 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         mbar_fence_init();
     }
     const R dt = (R)(*A.dt);
-    const int nt = G.nt;
+    const int nt = MODE == kPredict ? P + 1 : G.nt;
     const long long E = G.E;
 
-    // phase-B items of this thread: element, variable and point block
-    // (items ordered block-major, so a warp's items share their block)
-    int it_el[IPT], it_v[IPT], it_b[IPT], it_bx[IPT], it_by[IPT];
-    bool it_ok[IPT];
+    // phase B: row br of variables bv .. bv + VB - 1 of element bel
+    const int bh = tid / (NE * n), bel = (tid / n) % NE, br = tid % n, bv = bh * VB;
+    const bool brow = tid < LN::ROWS;
+    // kPredict: du of every slice, summed as the slices pass (with gravity
+    // dudt per slice, which the source of the updated state still joins);
+    // kCorrect: du
+    R dreg[VB][n][LN::shared_sums ? 1 : ND];
+    R* sums = smem + LN::m1 + tid;
+    auto acc = [&](int k, int i, int tt) -> R& {
+        if constexpr (LN::shared_sums) return sums[((k * n + i) * ND + tt) * LN::ROWS];
+        else return dreg[k][i][tt];
+    };
+    // du of slice tt += dudt of slice ll, invader(tt,l) w_l dt times (the
+    // precision form takes invader(tt,l) w_l from one product and dt at the end)
+    auto add_term = [&](R& du, R dudt, int tt, int ll) {
+        if constexpr (sizeof(R) == 4) du += dudt * M.pred[tt * (P + 1) + ll];
+        else du += dudt * M.invader[tt * (P + 1) + ll] * M.wt[ll] * dt;
+    };
+    R cy[nf];           // derivative coefficients of the row
+    if (MODE != kFlux) {
 #pragma unroll
-    for (int k = 0; k < IPT; k++) {
-        const int it = tid + k * kThreads;
-        it_ok[k] = it < ITEMS;
-        const int itc = it_ok[k] ? it : 0;
-        const int b = itc / (NE * V), rem = itc % (NE * V);
-        it_el[k] = rem / V;
-        it_v[k] = rem % V;
-        it_b[k] = b;
-        it_bx[k] = (b % DB::NBX) * BX;
-        it_by[k] = (b / DB::NBX) * BY;
+        for (int k = 0; k < VB; k++)
+#pragma unroll
+            for (int i = 0; i < n; i++)
+#pragma unroll
+                for (int t = 0; t < ND; t++)
+                    if (!LN::shared_sums || brow) acc(k, i, t) = 0;
+#pragma unroll
+        for (int ll = 0; ll < nf; ll++) cy[ll] = M.dfp_to_sp[br * nf + ll];
+        if constexpr (sizeof(R) == 4) {
+            // the precision form scales the sum by 1/h_x alone
+            const R ratio = (R)(G.h[0] / G.h[1]);
+#pragma unroll
+            for (int ll = 0; ll < nf; ll++) cy[ll] *= ratio;
+        }
     }
-    R dreg[IPT][BXY][NT];  // kPredict: dudt per slice; kCorrect: du in [..][..][0]
-#pragma unroll
-    for (int k = 0; k < IPT; k++)
-#pragma unroll
-        for (int p = 0; p < BXY; p++)
-#pragma unroll
-            for (int t = 0; t < NT; t++) dreg[k][p][t] = 0;
-
     __syncthreads();
-    // one elected thread issues the bulk copies of slice t into buffer b
+    // the last warp issues the bulk copies of slice t into buffer b, one
+    // staged element per lane
     auto issue = [&](int t, int b) {
+        if (tid < NTH - 32) return;
+        const int lane = tid & 31;
         const R* src = A.in_slices > 1 ? A.ua_in + (long long)t * E * V * NPT : A.ua_in;
         R* dst = Sbuf + b * NS * SS;
-        if (tid == 0) {
-            uint32_t bytes = 0;
-            for (int s = 0; s < NS; s++)
-                if (sl_elem[s] >= 0) bytes += V * NPT * sizeof(R);
+        int cnt = 0;
+        for (int s = lane; s < NS; s += 32) cnt += sl_elem[s] >= 0;
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) {
             fence_proxy_async_smem();
-            mbar_expect_tx(&bar[b], bytes);
-            for (int s = 0; s < NS; s++)
-                if (sl_elem[s] >= 0) bulk_g2s(dst + s * SS, src + sl_elem[s] * V * NPT, V * NPT * sizeof(R), &bar[b]);
+            mbar_expect_tx(&bar[b], (uint32_t)(cnt * V * NPT * sizeof(R)));
         }
+        __syncwarp();
+        for (int s = lane; s < NS; s += 32)
+            if (sl_elem[s] >= 0)
+                bulk_g2s(dst + s * SS, src + (long long)sl_elem[s] * V * NPT, V * NPT * sizeof(R), &bar[b]);
     };
     const bool multi = A.in_slices > 1;
     const int nt_eval = (MODE == kPredict && !multi) ? 1 : nt;
     issue(0, 0);
-    // the step-start state of the tile's elements (predictor and corrector
-    // epilogues), point-major, by coalesced loads while slice 0 is staged
-    if (MODE != kFlux) {
-        for (int q = tid; q < NE * V * (NPT / PW); q += kThreads) {
-            const int c = q % (NPT / PW), k = q / (NPT / PW);
-            R w4[PW];
-            vload<R, PW>(A.u + sl_elem[k / V] * V * NPT + (k % V) * NPT + c * PW, w4);
-#pragma unroll
-            for (int w = 0; w < PW; w++) Ubuf[(c * PW + w) * KS + k] = w4[w];
-        }
-    }
     for (int t = 0; t < nt_eval; t++) {
-        const int b = multi ? (t & 1) : 0;
-        R* Ss = Sbuf + b * NS * SS;
-        R* FX = FX0 + (NFX == 1 ? 0 : (t & 1)) * (2 * NE * V * FXS);
-        if (multi && t + 1 < nt) issue(t + 1, b ^ 1);
-        if (t == 0 || multi) mbar_wait_bounded(&bar[b], multi ? ((t >> 1) & 1) : 0, G.status);
+        const int b = ST == 2 && multi ? (t & 1) : 0;
+        const R* Ss = Sbuf + b * NS * SS;
+        R* FX = FX0 + (NFX == 1 ? 0 : (t & 1)) * (2 * NE * FE);
+        if (ST == 2 && multi && t + 1 < nt) issue(t + 1, b ^ 1);
+        if (t == 0 || multi) mbar_wait_bounded(&bar[b], multi ? (ST == 2 ? (t >> 1) & 1 : t & 1) : 0, G.status);
         // ---- phase A: fluxes at every flux point of the slice ----
-        // interfaces (two extrapolations and an LLF solve, about twice an
-        // interior point's work) on the first NFT threads, one each; the
-        // interior points on the rest, ordered by (direction, flux point)
-        // so that a warp's points share both and take their coefficients
-        // from constant offsets
-        {
-            constexpr int NF0 = LN::L0, NF1 = LN::L1, NFT = NF0 + NF1;
-            constexpr int NPL = NE * n;                 // interior items per (direction, flux point)
-            constexpr int NINT = 2 * (nf - 2) * NPL;
-            constexpr int TI = kThreads - NFT;
-            const int vt = A.in_slices > 1 ? t : 0;
-            auto face = [&](int q) {
-                if (q < NF0) face_item2<R, P, TX, TY, 0, VISC>(G, M, Ss, FX, o, q, A.vg[0], sl_elem, vt);
-                else face_item2<R, P, TX, TY, 1, VISC>(G, M, Ss, FX, o, q - NF0, A.vg[1], sl_elem, vt);
+        bool bad = false;  // a flux value outside div_range
+        const bool check = MODE != kFlux && sizeof(R) == 8 && !G.uniform_pow2;
+        const int vt = multi ? t : 0;
+        auto line = [&](auto dir, int q) {
+            constexpr int d = decltype(dir)::value;
+            // x lines: 8 elements, then their rows (16-byte loads of 8 lanes
+            // fall into distinct banks); y lines: an element's columns first
+            int el, r;
+            if constexpr (d == 0 && NE % 8 == 0) { el = (q & 7) + 8 * (q / (8 * n)); r = (q >> 3) % n; }
+            else { el = q / n; r = q % n; }
+            const int lx = el % TX, ly = el / TX;
+            const int sN = d == 0 ? TL::slot(lx - 1, ly, 0) : TL::slot(lx, ly - 1, 0);
+            const int gface = o[d] + (d == 0 ? lx : ly);
+            // beyond the domain's edge, or in a row outside it: nothing reads it
+            if (gface > G.N[d] || o[1 - d] + (d == 0 ? ly : lx) >= G.N[1 - d]) return;
+            const bool edge = G.bc[d] != kPeriodic;
+            const bool ghostL = edge && gface == 0, ghostR = edge && gface == G.N[d];
+            const R* src = Ss + el * SS;
+            R* dst = FX + d * NE * FE + el * FE + (d == 0 ? r * nf : r);
+            constexpr int st = d == 0 ? 1 : n;  // stride between the line's flux points
+            // the plain form reads the line again after the interface instead
+            // of holding it across, for its registers
+            constexpr bool hold = sizeof(R) == 4;
+            R ul[V][n];
+            auto load = [&]() {
+#pragma unroll
+                for (int v = 0; v < V; v++) load_line<R, n, d>(src + v * NPT, r, ul[v]);
             };
-            auto interior = [&](int r) {
-                const int g = r / NPL, el = (r % NPL) / n, tp = r % n;
-                if (g < nf - 2) interior_item2<R, P, TX, TY, 0>(G, Msf, Ss, FX, el, 1 + g, tp);
-                else interior_item2<R, P, TX, TY, 1>(G, Msf, Ss, FX, el, 1 + g - (nf - 2), tp);
-            };
-            if constexpr (TI >= kThreads / 4) {
-                if (tid < NFT) face(tid);
-                else
-                    for (int r = tid - NFT; r < NINT; r += TI) interior(r);
-            } else {
-                for (int q = tid; q < NFT + NINT; q += kThreads) {
-                    if (q < NFT) face(q);
-                    else interior(q - NFT);
-                }
-            }
-        }
-        __syncthreads();
-        if (MODE != kFlux) {
-            // ---- phase B: divergence of the thread's point blocks ----
-#pragma unroll
-            for (int k = 0; k < IPT; k++) {
-                if (!it_ok[k]) continue;
-                const int el = it_el[k], v = it_v[k], bx0 = it_bx[k], by0 = it_by[k];
-                const R* Fx = FX + ((0 * NE + el) * V + v) * FXS;
-                const R* Fy = FX + ((1 * NE + el) * V + v) * FXS;
-                R dd[BY][BX];
-                div_block2<R, P>(G, Mdf, Fx, Fy, bx0, by0, dd);
-#pragma unroll
-                for (int j = 0; j < BY; j++)
-#pragma unroll
-                    for (int i = 0; i < BX; i++) {
-                        const int p = j * BX + i;
-                        if (MODE == kPredict) {
-#pragma unroll
-                            for (int tt = 0; tt < NT; tt++)
-                                if (tt == t || (!multi && tt < nt)) dreg[k][p][tt] = dd[j][i];
-                        } else {
-                            R dudt = dd[j][i];
-                            if (G.grav && v != 0) {
-                                const int pt = (bx0 + i) + n * (by0 + j);
-                                const R* uv = Ss + el * SS;
-                                R s;
-                                if (v <= D) s = uv[pt] * (R)G.g[v - 1];
-                                else s = uv[NPT + pt] * (R)G.g[0] + uv[2 * NPT + pt] * (R)G.g[1];
-                                dudt -= s;
-                            }
-                            dreg[k][p][0] += dudt * M.wt[t] * dt;
-                        }
-                    }
-            }
-        } else {
-            // ---- FV face fluxes of slice t (src/transforms.cpp:378-481) ----
-#pragma unroll
-            for (int d = 0; d < D; d++) {
-                R* out = A.ff[d];
-                const R* Fd = FX + d * NE * V * FXS;
-                for (int q = tid; q < NE * NFP; q += kThreads) {
-                    const int el = q / NFP, fi = q % NFP;
-                    int ll, cc;
-                    if (d == 0) { ll = fi % nf; cc = fi / nf; }
-                    else { cc = fi % n; ll = fi / n; }
-                    R* dst = out + (((long long)t * E + sl_elem[el]) * V) * NFP + fi;
-                    const R* srcb = Fd + el * V * FXS + (d == 0 ? ll : n * ll);
+            if (hold) load();
+            {
+                R uL[V], uR[V], F[V];
+                if constexpr (hold) {
 #pragma unroll
                     for (int v = 0; v < V; v++) {
-                        R f = 0;
+                        R a = 0;
 #pragma unroll
-                        for (int m = 0; m < n; m++) f += srcb[v * FXS + (d == 0 ? nf * m : m)] * Mcv[cc * n + m];
-                        dst[v * NFP] = f;
+                        for (int l = 0; l < n; l++) a += ul[v][l] * M.sp_to_fp[l];
+                        uR[v] = a;
+                    }
+                } else if (!ghostR) {
+                    trace2<R, P, d, 0>(M, src, r, uR);
+                }
+                if (!ghostL) trace2<R, P, d, 1>(M, Ss + sN * SS, r, uL);
+                interface2<R, P, d, VISC>(G, uL, uR, ghostL, ghostR, F, A.vg[d], VISC ? sl_elem[sN] : 0,
+                                          VISC ? sl_elem[el] : 0, vt, r);
+                R* dl = FX + d * NE * FE + sN * FE + (d == 0 ? r * nf : r) + (nf - 1) * st;
+                const bool inside = d == 0 ? lx > 0 : ly > 0;
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    dst[v * NFP] = F[v];
+                    if (inside) dl[v * NFP] = F[v];
+                    if (check) bad |= !div_range(F[v]);
+                }
+            }
+            if (gface == G.N[d]) return;  // the domain's high edge: only the interface is inside
+            if (!hold) load();
+#pragma unroll
+            for (int ll = 1; ll < nf - 1; ll++) {
+                R u[V], w[V], f[V];
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    R a = 0;
+#pragma unroll
+                    for (int l = 0; l < n; l++) a += ul[v][l] * M.sp_to_fp[ll * n + l];
+                    u[v] = a;
+                }
+                primitives<2>(u, w, (R)G.gm);
+                euler_flux<2>(u, w, f, d);
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    dst[v * NFP + ll * st] = f[v];
+                    if (check) bad |= !div_range(f[v]);
+                }
+            }
+        };
+        auto edge = [&](auto dir, int q) {
+            constexpr int d = decltype(dir)::value;
+            const int r = q % n, k = q / n;
+            const int el = d == 0 ? (TX - 1) + TX * k : k + TX * (TY - 1);
+            const int sN = d == 0 ? TL::slot(TX, k, 0) : TL::slot(k, TY, 0);
+            const int gface = o[d] + (d == 0 ? TX : TY);
+            if (gface > G.N[d] || o[1 - d] + k >= G.N[1 - d]) return;
+            const bool ghostR = G.bc[d] != kPeriodic && gface == G.N[d];
+            R uL[V], uR[V], F[V];
+            trace2<R, P, d, 1>(M, Ss + el * SS, r, uL);
+            if (!ghostR) trace2<R, P, d, 0>(M, Ss + sN * SS, r, uR);
+            interface2<R, P, d, VISC>(G, uL, uR, false, ghostR, F, A.vg[d], VISC ? sl_elem[el] : 0,
+                                      VISC ? sl_elem[sN] : 0, vt, r);
+            R* dst = FX + d * NE * FE + el * FE + (d == 0 ? r * nf + nf - 1 : r + n * (nf - 1));
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                dst[v * NFP] = F[v];
+                if (check) bad |= !div_range(F[v]);
+            }
+        };
+        using D0 = std::integral_constant<int, 0>;
+        using D1 = std::integral_constant<int, 1>;
+        if (tid < LN::LW) {
+            if (LN::LW == LN::LINES || tid < LN::LINES) line(D0{}, tid);
+        } else if (tid < 2 * LN::LW) {
+            if (LN::LW == LN::LINES || tid < LN::LW + LN::LINES) line(D1{}, tid - LN::LW);
+        } else if (tid < 2 * LN::LW + LN::EDGE0) {
+            edge(D0{}, tid - 2 * LN::LW);
+        } else if (tid < 2 * LN::LW + LN::EDGE0 + LN::EDGE1) {
+            edge(D1{}, tid - 2 * LN::LW - LN::EDGE0);
+        }
+        // spacings that are no power of two: the FP64 form divides every term
+        // by h, from h's reciprocal unless some flux value of the tile is so
+        // small or large that the quotient could under- or overflow
+        bool slow = false;
+        if (check) slow = __syncthreads_or(bad || !G.safe_div);
+        else __syncthreads();
+        // one staging buffer: the next slice's copy may start, unless phase B
+        // still reads this slice's state
+        const bool reads = MODE == kCorrect && G.grav;
+        if (ST == 1 && multi && t + 1 < nt && !reads) issue(t + 1, 0);
+        if constexpr (MODE != kFlux) {
+            // ---- phase B: divergence of the thread's rows ----
+            if (brow) {
+#pragma unroll
+                for (int k = 0; k < VB; k++) {
+                    const int v = bv + k;
+                    const R* Fx = FX + bel * FE + v * NFP + br * nf;
+                    const R* Fy = FX + NE * FE + bel * FE + v * NFP;
+                    R dd[n];
+                    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+                        for (int i = 0; i < n; i++) dd[i] = 0;
+#pragma unroll
+                        for (int ll = 0; ll < nf; ll++) {
+                            R fy[n];
+                            row_load<R, n>(Fy + n * ll, fy);
+                            const R fx = Fx[ll];
+#pragma unroll
+                            for (int i = 0; i < n; i++) {
+                                dd[i] += fx * M.dfp_to_sp[i * nf + ll];
+                                dd[i] += fy[i] * cy[ll];
+                            }
+                        }
+                        // (the predictor without gravity scales at the end)
+                        if (MODE != kPredict || G.grav) {
+                            const R ihx = (R)G.ih[0];
+#pragma unroll
+                            for (int i = 0; i < n; i++) dd[i] *= ihx;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < n; i++) dd[i] = 0;
+                        auto sum = [&](auto term) {
+#pragma unroll
+                            for (int ll = 0; ll < nf; ll++) {
+                                R fy[n];
+                                row_load<R, n>(Fy + n * ll, fy);
+                                const R fx = Fx[ll];
+#pragma unroll
+                                for (int i = 0; i < n; i++) {
+                                    dd[i] += term(fx * M.dfp_to_sp[i * nf + ll], 0);
+                                    dd[i] += term(fy[i] * cy[ll], 1);
+                                }
+                            }
+                        };
+                        if (G.uniform_pow2) {
+                            // every active h is the same power of two: the
+                            // scaling of each term by 1/h is exact and
+                            // commutes with the rounding of the sum
+                            sum([](R x, int) { return x; });
+#pragma unroll
+                            for (int i = 0; i < n; i++) dd[i] *= G.ih[0];
+                        } else if (!slow) {
+                            sum([&](R x, int d) { return div_const(x, G.h[d], G.ih[d], G.ihl[d]); });
+                        } else {
+                            sum([&](R x, int d) { return x / G.h[d]; });
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < n; i++) {
+                        if constexpr (MODE == kPredict) {
+                            if (G.grav) {
+#pragma unroll
+                                for (int tt = 0; tt < ND; tt++)
+                                    if (tt == t || !multi) acc(k, i, tt) = dd[i];
+                            } else if (multi) {
+#pragma unroll
+                                for (int tt = 0; tt < ND; tt++) add_term(acc(k, i, tt), dd[i], tt, t);
+                            } else {
+#pragma unroll
+                                for (int tt = 0; tt < ND; tt++)
+#pragma unroll
+                                    for (int ll = 0; ll < ND; ll++) add_term(acc(k, i, tt), dd[i], tt, ll);
+                            }
+                        } else {
+                            R dudt = dd[i];
+                            if (G.grav && v != 0) {
+                                const R* uv = Ss + bel * SS + br * n + i;
+                                R s;
+                                if (v <= D) s = uv[0] * (R)G.g[v - 1];
+                                else s = uv[NPT] * (R)G.g[0] + uv[2 * NPT] * (R)G.g[1];
+                                dudt -= s;
+                            }
+                            acc(k, i, 0) += dudt * M.wt[t] * dt;
+                        }
                     }
                 }
             }
-        }
-        // with one FX buffer the next slice's phase A overwrites this
-        // slice's fluxes; the corrector's gravity source reads this slice's
-        // staging buffer, which the next slice's prefetch overwrites
-        if (NFX == 1 || (MODE == kCorrect && G.grav)) __syncthreads();
-    }
-    __syncthreads();
-
-    if (MODE == kPredict) {
-        // ---- ADER predictor (src/transforms.cpp:309-323) ----
-        __shared__ R Cw[NT * NT];
-        if constexpr (sizeof(R) == 4) {
-            for (int i = tid; i < NT * NT; i += kThreads) {
-                const int tt = i / NT, ll = i % NT;
-                Cw[i] = (tt < nt && ll < nt) ? M.invader[tt * nt + ll] * M.wt[ll] * dt : R(0);
+        } else {
+            // ---- FV face fluxes of slice t (src/transforms.cpp:378-481):
+            // the averages across each set of transverse points replace the
+            // points in place, then the element blocks are copied out ----
+            constexpr int ITEMS = NE * V * nf;
+            for (int q = tid; q < 2 * ITEMS; q += NTH) {
+                const int d = q >= ITEMS, w = d ? q - ITEMS : q;
+                const int ll = w % nf, k = w / nf;  // k = element x variable
+                R* src = FX + d * NE * FE + (k / V) * FE + (k % V) * NFP + (d ? n * ll : ll);
+                const int st = d ? 1 : nf;
+                R in[n];
+#pragma unroll
+                for (int m = 0; m < n; m++) in[m] = src[st * m];
+#pragma unroll
+                for (int c = 0; c < n; c++) {
+                    R f = 0;
+#pragma unroll
+                    for (int m = 0; m < n; m++) f += in[m] * M.sp_to_cv[c * n + m];
+                    src[st * c] = f;
+                }
+            }
+            __syncthreads();
+            constexpr int CF = V * NFP / Q;  // vectors per element block
+            for (int q = tid; q < 2 * NE * CF; q += NTH) {
+                const int d = q >= NE * CF, w = d ? q - NE * CF : q;
+                const int el = w / CF, c = w - el * CF;
+                const int ge = el_own[el];
+                if (ge >= 0)
+                    reinterpret_cast<VT*>(A.ff[d] + ((long long)t * E + ge) * V * NFP)[c] =
+                        reinterpret_cast<const VT*>(FX + d * NE * FE + el * FE)[c];
             }
         }
-        __syncthreads();
-        R* O = smem;  // [slice][point][KS], point-major
+        // with one flux buffer the next slice's phase A overwrites this
+        // slice's fluxes; the corrector's gravity source reads this slice's
+        // staging buffer, which the next slice's prefetch overwrites
+        if (NFX == 1 || reads) __syncthreads();
+        if (ST == 1 && multi && t + 1 < nt && reads) issue(t + 1, 0);
+    }
+    __syncthreads();
+    const int bge = brow ? el_own[bel] : -1;
+
+    if constexpr (MODE == kPredict) {
+        // ---- ADER predictor (src/transforms.cpp:309-323) ----
         // with gravity the source of a momentum (energy) slot uses the
         // updated density (momenta) of the same point and slice
         // (src/transforms.cpp:16-27 on U_ader being written): variables are
-        // finished in three rounds that read the earlier rounds' results
+        // finished in three rounds that pass those on through shared memory
+        R* O = smem;  // [slice][rho, m_x, m_y][element][point]
         const int rounds = G.grav ? 3 : 1;
         for (int round = 0; round < rounds; round++) {
+            if (brow) {
 #pragma unroll
-            for (int k = 0; k < IPT; k++) {
-                if (!it_ok[k]) continue;
-                const int el = it_el[k], v = it_v[k], kk = el * V + v;
-                if (G.grav && (v == 0 ? 0 : (v <= D ? 1 : 2)) != round) continue;
+                for (int k = 0; k < VB; k++) {
+                    const int v = bv + k;
+                    if (G.grav && (v == 0 ? 0 : (v <= D ? 1 : 2)) != round) continue;
+                    R uo[n];
+                    if (bge >= 0) row_load<R, n>(A.u + ((long long)bge * V + v) * NPT + br * n, uo);
+                    else {
 #pragma unroll
-                for (int j = 0; j < BY; j++)
+                        for (int i = 0; i < n; i++) uo[i] = 0;
+                    }
+                    if (G.grav && v != 0) {
 #pragma unroll
-                    for (int i = 0; i < BX; i++) {
-                        const int p = j * BX + i;
-                        const int pt = (it_bx[k] + i) + n * (it_by[k] + j);
-                        const R u_old = Ubuf[pt * KS + kk];
-                        R dudt[NT];
+                        for (int tt = 0; tt < NT; tt++)
 #pragma unroll
-                        for (int tt = 0; tt < NT; tt++) {
-                            dudt[tt] = dreg[k][p][tt];
-                            if (G.grav && v != 0 && tt < nt) {
-                                const R* nw = O + (tt * NPT + pt) * KS + el * V;
+                            for (int i = 0; i < n; i++) {
+                                const R* nw = O + ((tt * 3) * NE + bel) * NPT + br * n + i;
                                 R s;
                                 if (v <= D) s = nw[0] * (R)G.g[v - 1];
-                                else s = nw[1] * (R)G.g[0] + nw[2] * (R)G.g[1];
-                                dudt[tt] -= s;
+                                else s = nw[NE * NPT] * (R)G.g[0] + nw[2 * NE * NPT] * (R)G.g[1];
+                                acc(k, i, tt) -= s;
                             }
-                        }
+                    }
 #pragma unroll
-                        for (int tt = 0; tt < NT; tt++) {
-                            if (tt >= nt) break;
+                    for (int tt = 0; tt < NT; tt++) {
+                        R val[n];
+#pragma unroll
+                        for (int i = 0; i < n; i++) {
                             R du = 0;
-                            if constexpr (sizeof(R) == 4) {
+                            if (G.grav) {
 #pragma unroll
-                                for (int ll = 0; ll < NT; ll++)
-                                    if (ll < nt) du += dudt[ll] * Cw[tt * NT + ll];
+                                for (int ll = 0; ll < NT; ll++) add_term(du, acc(k, i, ll), tt, ll);
                             } else {
-#pragma unroll
-                                for (int ll = 0; ll < NT; ll++)
-                                    if (ll < nt) du += dudt[ll] * M.invader[tt * nt + ll] * M.wt[ll] * dt;
+                                du = acc(k, i, tt);
                             }
-                            O[(tt * NPT + pt) * KS + kk] = u_old - du;
+                            if constexpr (sizeof(R) == 4) du *= G.grav ? dt : dt * (R)G.ih[0];
+                            val[i] = uo[i] - du;
+                        }
+                        if (bge >= 0) row_store<R, n>(A.ua_out + (((long long)tt * E + bge) * V + v) * NPT + br * n, val);
+                        if (G.grav && v <= D) {
+#pragma unroll
+                            for (int i = 0; i < n; i++) O[((tt * 3 + v) * NE + bel) * NPT + br * n + i] = val[i];
                         }
                     }
+                }
             }
             if (G.grav) __syncthreads();
         }
-        __syncthreads();
-        // coalesced write-back of every slice: consecutive threads take
-        // consecutive points of an element's variable rows
-        for (int q = tid; q < NE * V * (NPT / PW); q += kThreads) {
-            const int c = q % (NPT / PW), k = q / (NPT / PW);
-            R* dst = A.ua_out + sl_elem[k / V] * V * NPT + (k % V) * NPT + c * PW;
-            const R* src = O + c * PW * KS + k;
-            for (int tt = 0; tt < nt; tt++) {
-                R w4[PW];
-#pragma unroll
-                for (int w = 0; w < PW; w++) w4[w] = src[w * KS];
-                vstore<R, PW>(dst, w4);
-                dst += E * V * NPT;
-                src += NPT * KS;
-            }
-        }
-    } else if (MODE == kCorrect) {
+    } else if constexpr (MODE == kCorrect) {
         // ---- corrector / RK stage (src/transforms.cpp:327-374, 252-261) ----
         R* Wsp = smem;                     // [NE][V][NPT]
         R* Tmp = smem + NE * V * NPT;
-        R* Tu = smem + 2 * NE * V * NPT;   // [NPT][KS]: U - du, point-major
+        if (brow) {
 #pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            if (!it_ok[k]) continue;
-            const int kk = it_el[k] * V + it_v[k];
+            for (int k = 0; k < VB; k++) {
+                const int v = bv + k;
+                const long long g = ((long long)bge * V + v) * NPT + br * n;
+                R val[n];
+                if (bge >= 0) {
+                    row_load<R, n>(A.u + g, val);
 #pragma unroll
-            for (int j = 0; j < BY; j++)
+                    for (int i = 0; i < n; i++) val[i] -= acc(k, i, 0);
+                    if (A.rk_a > 0) {
+                        const R ra = (R)A.rk_a;
+                        R u0[n];
+                        row_load<R, n>(A.u0 + g, u0);
 #pragma unroll
-                for (int i = 0; i < BX; i++) {
-                    const int pt = (it_bx[k] + i) + n * (it_by[k] + j);
-                    Tu[pt * KS + kk] = Ubuf[pt * KS + kk] - dreg[k][j * BX + i][0];
+                        for (int i = 0; i < n; i++) val[i] = ra * u0[i] + ((R)1.0 - ra) * val[i];
+                    }
+                    row_store<R, n>(A.u_out + g, val);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < n; i++) val[i] = 1;
                 }
-        }
-        __syncthreads();
-        // RK convex combination and the write of U, coalesced; W_sp's
-        // element-major copy for the final stage's primitives and sweeps
-        for (int q = tid; q < NE * V * (NPT / PW); q += kThreads) {
-            const int c = q % (NPT / PW), k = q / (NPT / PW);
-            const long long g = sl_elem[k / V] * V * NPT + (k % V) * NPT + c * PW;
-            R val[PW];
 #pragma unroll
-            for (int w = 0; w < PW; w++) val[w] = Tu[(c * PW + w) * KS + k];
-            if (A.rk_a > 0) {
-                const R ra = (R)A.rk_a;
-                R u0[PW];
-                vload<R, PW>(A.u0 + g, u0);
-#pragma unroll
-                for (int w = 0; w < PW; w++) val[w] = ra * u0[w] + ((R)1.0 - ra) * val[w];
+                for (int i = 0; i < n; i++) Wsp[(bel * V + v) * NPT + br * n + i] = val[i];
             }
-            vstore<R, PW>(A.u_out + g, val);
-            vstore<R, PW>(Wsp + k * NPT + c * PW, val);
         }
         if (A.final_stage) {
+            __shared__ R Mcv[S::n * S::n];
+            for (int i = tid; i < S::n * S::n; i += NTH) Mcv[i] = M.sp_to_cv[i];
             __syncthreads();
-            for (int q = tid; q < NE * NPT; q += kThreads) {
+            for (int q = tid; q < NE * NPT; q += NTH) {
                 const int el = q / NPT, pt = q % NPT;
                 R un[V], w[V];
 #pragma unroll
@@ -660,9 +717,10 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             sweep_smem<D, P, R>(Tmp, Wsp, Mcv, 1, NE * V * NPT);
             __syncthreads();
             double dtl = 1.7976931348623157e308;
-            for (int q = tid; q < NE * NPT; q += kThreads) {
+            for (int q = tid; q < NE * NPT; q += NTH) {
                 const int el = q / NPT, pt = q % NPT;
-                const long long ge = sl_elem[el];
+                const long long ge = el_own[el];
+                if (ge < 0) continue;
                 R w[V];
 #pragma unroll
                 for (int v = 0; v < V; v++) w[v] = Wsp[(el * V + v) * NPT + pt];
@@ -675,11 +733,16 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         }
     } else {
         // ---- U_cv = sp_to_cv(U) and the slice-0 FV candidate ----
+        __shared__ R Mcv[S::n * S::n];
+        constexpr int CH = V * NPT / Q;  // vectors per element
         R* Ut = Sbuf;
         R* Tmp = Sbuf + NE * V * NPT;
-        for (int q = tid; q < NE * CH; q += kThreads) {
+        for (int i = tid; i < S::n * S::n; i += NTH) Mcv[i] = M.sp_to_cv[i];
+        for (int q = tid; q < NE * CH; q += NTH) {
             const int el = q / CH, c = q % CH;
-            reinterpret_cast<VT*>(Ut + el * V * NPT)[c] = reinterpret_cast<const VT*>(A.u + sl_elem[el] * V * NPT)[c];
+            if (el_own[el] >= 0)
+                reinterpret_cast<VT*>(Ut + el * V * NPT)[c] =
+                    reinterpret_cast<const VT*>(A.u + (long long)el_own[el] * V * NPT)[c];
         }
         __syncthreads();
         sweep_smem<D, P, R>(Ut, Tmp, Mcv, 0, NE * V * NPT);
@@ -687,13 +750,16 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         sweep_smem<D, P, R>(Tmp, Ut, Mcv, 1, NE * V * NPT);
         __syncthreads();
         const R* src = Ut;
-        for (int q = tid; q < NE * CH; q += kThreads) {
+        for (int q = tid; q < NE * CH; q += NTH) {
             const int el = q / CH, c = q % CH;
-            reinterpret_cast<VT*>(A.ucv + sl_elem[el] * V * NPT)[c] = reinterpret_cast<const VT*>(src + el * V * NPT)[c];
+            if (el_own[el] >= 0)
+                reinterpret_cast<VT*>(A.ucv + (long long)el_own[el] * V * NPT)[c] =
+                    reinterpret_cast<const VT*>(src + el * V * NPT)[c];
         }
-        for (int q = tid; q < NE * NPT; q += kThreads) {
+        for (int q = tid; q < NE * NPT; q += NTH) {
             const int el = q / NPT, pt = q % NPT;
-            const long long ge = sl_elem[el];
+            const long long ge = el_own[el];
+            if (ge < 0) continue;
             R uo[V], un[V];
 #pragma unroll
             for (int v = 0; v < V; v++) uo[v] = src[(el * V + v) * NPT + pt];

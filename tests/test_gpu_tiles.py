@@ -1,0 +1,78 @@
+"""Element counts that no tile divides: the 2D Picard pass runs 4 x 4 (above
+p = 3: 4 x 2) element tiles that hang over the domain's high edges, and
+spacings that are no power of two take the division by h from its reciprocal.
+The plain form against the oracle, bit for bit; the precision form against
+the plain form."""
+import zlib
+
+import numpy as np
+import pytest
+
+from helpers import gpu_config, oracle_active, oracle_config, rel_l1, same_bits
+from test_gpu_parity import load_oracle_state, random_state, solver
+
+pytestmark = pytest.mark.gpu
+
+# one element past a tile, one short of it, less than one tile, whole tiles
+SIZES = [(2, 2), (3, 5), (5, 3), (4, 6), (9, 7)]
+EDGES = ["periodic", "gradfree", "reflective"]
+
+
+def overrides(p, nx, ny, bc, fallback=True, integrator="ader"):
+    return [f"mesh/p={p}", f"mesh/nx1={nx}", f"mesh/nx2={ny}", "mesh/nx3=1", f"mesh/x1_bc={bc[0]}",
+            f"mesh/x2_bc={bc[1]}", f"job/fallback={str(fallback).lower()}", f"time/integrator={integrator}"]
+
+
+def against_oracle(ov, mine, ref5, D, steps=2):
+    from oracle import oracle as O
+    g, o = solver(ov), O.Oracle(oracle_config(ov))
+    g.write_u(mine)
+    load_oracle_state(o, ref5, D)
+    dt = o.compute_dt()
+    assert g.dt() == dt
+    for step in range(steps):
+        o.step(dt)
+        g.step()
+        dt = o.compute_dt()
+        assert g.dt() == dt, step
+        for name, field in (("U_sp", 0), ("W_cv", 1)):
+            wo, wg = oracle_active(o, name), g.to_reference_slots(g.field_array(field))
+            assert same_bits(wg, wo), (step, name, rel_l1(wo, wg))
+    g.close()
+
+
+@pytest.mark.parametrize("p", range(1, 8))
+@pytest.mark.parametrize("size", SIZES)
+def test_ragged_counts_match_the_oracle(p, size):
+    k = zlib.crc32(repr((p, size)).encode())
+    bc = (EDGES[k % 3], EDGES[(k // 3) % 3])
+    integrator = ["ader", "ader", "rk2"][(k // 9) % 3]
+    ov = overrides(p, *size, bc, fallback=k % 2 == 0, integrator=integrator)
+    if integrator == "ader" and k % 5 == 0:
+        ov.append("hydro/g2=-0.3")
+    against_oracle(ov, *random_state(gpu_config(ov), seed=k))
+
+
+@pytest.mark.parametrize("scale", [1e-160, 1e-300, 1e80])
+def test_fluxes_too_small_or_large_for_the_reciprocal(scale):
+    """momenta (and with them flux values) of this size leave the range in
+    which a quotient from 1/h is exact: the tile divides"""
+    ov = overrides(3, 5, 6, ("periodic", "gradfree"), fallback=False)
+    mine, ref5, D = random_state(gpu_config(ov), seed=3)
+    mine[:, :, :, 1:3] *= scale
+    ref5[1:3] *= scale
+    against_oracle(ov, mine, ref5, D, steps=1)
+
+
+@pytest.mark.parametrize("p,size", [(2, (7, 6)), (3, (6, 5)), (5, (5, 7))])
+def test_precision_form_on_ragged_counts(p, size):
+    """FP32 round-off only (as the aligned counts): smooth flow, 4 steps"""
+    ov = overrides(p, *size, ("periodic", "periodic"), fallback=False) + ["time/cfl=0.4"]
+    g64, g32 = solver(ov, precision="fp64"), solver(ov, precision="fp32")
+    for _ in range(4):
+        g64.step()
+        g32.step()
+    a, b = g64.field_array(0), g32.field_array(0)
+    assert max(np.abs(b[v] - a[v]).sum() / np.abs(a[v]).sum() for v in range(4)) < 3e-6
+    g64.close()
+    g32.close()
