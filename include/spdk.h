@@ -160,8 +160,8 @@ enum {
     SPDK_KERNEL_CORRECT = 1,  /* corrector / RK stage + W_cv + dt */
     SPDK_KERNEL_FLUX = 2,     /* last Picard pass writing FV face fluxes */
     SPDK_KERNEL_DETECT = 3,   /* NAD/SED/PAD */
-    SPDK_KERNEL_THETA = 4,    /* theta blending (computed inside the update kernel: no launches) */
-    SPDK_KERNEL_UPDATE = 5,   /* fallback fluxes + FV update (+ W_cv, dt) */
+    SPDK_KERNEL_THETA = 4,    /* theta blending and the fallback fluxes of the faces it reaches */
+    SPDK_KERNEL_UPDATE = 5,   /* FV update (+ W_cv, dt) */
     SPDK_KERNEL_OTHER = 6,    /* dt hand-over */
     SPDK_KERNEL_KINDS = 7
 };

@@ -9,11 +9,6 @@
 
 namespace spdk {
 
-struct DetectArgs {
-    const double2* rpo;
-    const double2* rpn;
-    uint8_t* T;
-};
 struct DtArgs {
     double* dt;
     unsigned long long* dtmin;
@@ -61,30 +56,33 @@ __global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_bloc
     else picard_kernel_body<R, D, P, TX, TY, TZ, MODE>(it.G, M, it.A, b);
 }
 
-// the batched detect and update take one block per SM more than the
-// single-problem kernels (the FP64 update excepted: it would spill 350
-// bytes a thread): the groups' many small members leave the single-problem
-// sizing's occupancy unused (measured on the first 16 problems of the
-// ensemble, FP32: 44.7 -> 43.6 ms per step; the single 256^2 blast is
-// 0.3 % slower with the same sizing, so it keeps its own)
+// the batched detect takes one block per SM more than the single-problem
+// kernel in 2D: the groups' many small members leave its sizing's occupancy
+// unused (measured on the first 16 problems of the ensemble, FP32)
 template <int D>
 constexpr int kDetectBlocksPerSMBatched = D == 2 ? 5 : kDetectBlocksPerSM<D>;
-template <typename R, int D, int P>
-constexpr int kUpdateBlocksPerSMBatched = (D == 2 && sizeof(R) == 4) ? 6 : kUpdateBlocksPerSM<D, P>;
 
 template <typename R, int D, int P, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(kThreads, kDetectBlocksPerSMBatched<D>) detect_batched(const BatchItem<DetectArgs>* __restrict__ items, int n) {
     long long b;
     const BatchItem<DetectArgs>& it = batch_item(items, n, &b);
-    fv_detect_kernel_body<R, D, P, TX, TY, TZ>(it.G, it.A.rpo, it.A.rpn, it.A.T, nullptr, b);
+    fv_detect_kernel_body<R, D, P, TX, TY, TZ>(it.G, it.A, b);
 }
 
 template <typename R, int D, int P, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSMBatched<R, D, P>)
+__global__ void __launch_bounds__(kThreads, kBlendBlocksPerSM<R, D>)
+    blend_batched(const BatchItem<BlendArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
+    long long b;
+    const BatchItem<BlendArgsT<R>>& it = batch_item(items, n, &b);
+    fv_blend_kernel_body<R, D, P, TX, TY, TZ>(it.G, M, it.A, b);
+}
+
+template <typename R, int D, int P>
+__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D>)
     update_batched(const BatchItem<FallbackArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
     long long b;
     const BatchItem<FallbackArgsT<R>>& it = batch_item(items, n, &b);
-    fv_update_kernel_body<R, D, P, TX, TY, TZ>(it.G, M, it.A, b);
+    fv_update_kernel_body<R, D, P>(it.G, M, it.A, b);
 }
 
 // dt hand-over of every problem of the batch: one thread per problem
@@ -96,11 +94,14 @@ struct BatchSetT {
     void (*correct)(const BatchItem<PicardArgsT<R>>*, int, DevMatsT<R>) = nullptr;
     void (*flux)(const BatchItem<PicardArgsT<R>>*, int, DevMatsT<R>) = nullptr;
     void (*detect)(const BatchItem<DetectArgs>*, int) = nullptr;
+    void (*blend)(const BatchItem<BlendArgsT<R>>*, int, DevMatsT<R>) = nullptr;
     void (*update)(const BatchItem<FallbackArgsT<R>>*, int, DevMatsT<R>) = nullptr;
-    size_t picard_smem[3] = {0, 0, 0}, update_smem = 0;  // predict, correct, flux
+    size_t picard_smem[3] = {0, 0, 0}, blend_smem = 0, update_smem = 0;  // predict, correct, flux
     int picard_threads = kThreads;
     int picard_tile[3] = {1, 1, 1};  // a Picard block's elements (may hang over a domain's edge)
-    int tile[3] = {1, 1, 1};         // a detect / update block's elements
+    int tile[3] = {1, 1, 1};         // a detect block's elements
+    int blend_tile[3] = {1, 1, 1};
+    int update_elems = 1;            // consecutive elements of an update block
 };
 
 template <typename R, int P, int TX, int TY>
@@ -114,11 +115,17 @@ BatchSetT<R> make_batch_set() {
     k.picard_tile[0] = PX;
     k.picard_tile[1] = PY;
     k.detect = detect_batched<R, 2, P, TX, TY, 1>;
-    k.update = update_batched<R, 2, P, TX, TY, 1>;
+    using BT = BlendTile<2, P>;
+    k.blend = blend_batched<R, 2, P, BT::X, BT::Y, 1>;
+    k.blend_smem = BlendSmem<R, 2, P, BT::X, BT::Y, 1>::bytes;
+    k.blend_tile[0] = BT::X;
+    k.blend_tile[1] = BT::Y;
+    k.update = update_batched<R, 2, P>;
+    k.update_elems = UpdateBlock<2, P>::NE;
     k.picard_smem[kPredict] = picard_smem_bytes<R, 2, P, PX, PY, 1, kPredict>();
     k.picard_smem[kCorrect] = picard_smem_bytes<R, 2, P, PX, PY, 1, kCorrect>();
     k.picard_smem[kFlux] = picard_smem_bytes<R, 2, P, PX, PY, 1, kFlux>();
-    k.update_smem = UpdateSmem<R, 2, P, TX, TY, 1>::bytes;
+    k.update_smem = UpdateSmem<R, 2, P>::bytes;
     k.tile[0] = TX;
     k.tile[1] = TY;
     return k;

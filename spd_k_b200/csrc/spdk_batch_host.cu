@@ -34,7 +34,7 @@ __global__ void dt_batched(const DtArgs* __restrict__ a, int n) {
 
 namespace {
 
-enum { kPassPredict, kPassCorrect, kPassFlux, kPassDetect, kPassUpdate };
+enum { kPassPredict, kPassCorrect, kPassFlux, kPassDetect, kPassBlend, kPassUpdate };
 
 struct Pass {
     int kind;
@@ -103,16 +103,20 @@ template <typename R>
 int plan_group(spdk_batch* b, Group& g) {
     free_tables(g);
     const int n = (int)g.members.size();
-    // first block of every member, in the Picard and the detect / update launches
-    std::vector<long long> pfirst(n), first(n);
-    long long ptotal = 0, total = 0;
-    const int* ptile = set_of<R>(g).picard_tile;
+    // first block of every member in the Picard, detect, blend and update launches
+    std::vector<long long> pfirst(n), first(n), bfirst(n), ufirst(n);
+    long long ptotal = 0, total = 0, btotal = 0, utotal = 0;
+    const BatchSetT<R>& set = set_of<R>(g);
     for (int q = 0; q < n; q++) {
         const spdk_hydro* h = b->probs[g.members[q]];
         pfirst[q] = ptotal;
-        ptotal += tile_blocks(2, h->G.N, ptile);
+        ptotal += tile_blocks(2, h->G.N, set.picard_tile);
         first[q] = total;
-        total += (long long)(h->G.N[0] / g.tile) * (h->G.N[1] / g.tile);
+        total += tile_blocks(2, h->G.N, set.tile);
+        bfirst[q] = btotal;
+        btotal += tile_blocks(2, h->G.N, set.blend_tile);
+        ufirst[q] = utotal;
+        utotal += (h->E + set.update_elems - 1) / set.update_elems;
     }
     const unsigned pblocks = (unsigned)ptotal, blocks = (unsigned)total;
     const int nt = b->probs[g.members[0]]->nt;
@@ -177,6 +181,7 @@ int plan_group(spdk_batch* b, Group& g) {
     }
     for (int t = 0; t < nt && !rc; t++) {
         std::vector<BatchItem<DetectArgs>> det(n);
+        std::vector<BatchItem<BlendArgsT<R>>> bl(n);
         std::vector<BatchItem<FallbackArgsT<R>>> up(n);
         for (int q = 0; q < n; q++) {
             spdk_hydro* h = b->probs[g.members[q]];
@@ -184,22 +189,26 @@ int plan_group(spdk_batch* b, Group& g) {
             det[q].G = bq.G;
             if (b->labels) det[q].G.elem_trouble = h->elem_trouble;
             det[q].first = first[q];
-            det[q].A = DetectArgs{h->rpo, h->rpn, h->trouble};
+            det[q].A = DetectArgs{h->rpo, h->rpn, h->trouble, h->theta, h->elem_any};
+            bl[q].G = bq.G;
+            bl[q].first = bfirst[q];
+            BlendArgsT<R>& B = bl[q].A;
+            B = BlendArgsT<R>{};
+            B.ucv = (R*)h->ucv[t % 2];
+            B.trouble = h->trouble;
+            B.elem_any = h->elem_any;
+            B.theta = h->theta;
+            B.t = t;
+            B.dt = h->dt;
             up[q].G = bq.G;
-            up[q].first = first[q];
+            up[q].first = ufirst[q];
             FallbackArgsT<R>& F = up[q].A;
             F = FallbackArgsT<R>{};
             F.ucv_in = (R*)h->ucv[t % 2];
             F.ucv_out = (R*)h->ucv[(t + 1) % 2];
-            F.ff0 = (R*)h->ff[0];
-            F.ff1 = (R*)h->ff[1];
-            F.ff2 = (R*)h->ff[2];
-            F.rp_old = h->rpo;
-            F.rp_new = h->rpn;
+            for (int d = 0; d < 3; d++) B.ff[d] = F.ff[d] = (R*)h->ff[d];
             F.rp_old_next = h->rpo;
             F.rp_new_next = h->rpn;
-            F.trouble = h->trouble;
-            F.theta = h->theta;
             F.t = t;
             F.last = t == nt - 1;
             F.u = (R*)h->u;
@@ -211,7 +220,8 @@ int plan_group(spdk_batch* b, Group& g) {
             F.dt = h->dt;
         }
         rc = upload_pass(g, kPassDetect, blocks, det);
-        if (!rc) rc = upload_pass(g, kPassUpdate, blocks, up);
+        if (!rc) rc = upload_pass(g, kPassBlend, (unsigned)btotal, bl);
+        if (!rc) rc = upload_pass(g, kPassUpdate, (unsigned)utotal, up);
     }
     return rc;
 }
@@ -224,16 +234,14 @@ int set_batch_attributes(const BatchSetT<R>& k) {
         BCUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.picard_smem[m]));
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
+    BCUDA(cudaFuncSetAttribute((const void*)k.blend, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.blend_smem));
     BCUDA(cudaFuncSetAttribute((const void*)k.update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.update_smem));
+    cudaFuncSetAttribute((const void*)k.blend, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     cudaFuncSetAttribute((const void*)k.update, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return 0;
 }
 
 int select_group(spdk_batch* b, Group& g, int tile) {
-    for (int q : g.members) {
-        const spdk_hydro* h = b->probs[q];
-        if (h->G.N[0] % tile || h->G.N[1] % tile) return fail(SPDK_E_ARG, "tile does not divide an element count");
-    }
     const bool ok = b->prec == SPDK_PRECISION_FP32 ? batch_set(g.p, tile, &g.k32) : batch_set(g.p, tile, &g.k64);
     if (!ok) return fail(SPDK_E_ARG, "no batched kernels for this order / tile");
     g.tile = tile;
@@ -250,16 +258,19 @@ int launch_group_t(spdk_batch* b, const Group& g, cudaStream_t st) {
         b->prec == SPDK_PRECISION_FP32 ? (const void*)&h0->dm32 : (const void*)&h0->dm64);
     using PI = BatchItem<PicardArgsT<R>>;
     using DI = BatchItem<DetectArgs>;
+    using LI = BatchItem<BlendArgsT<R>>;
     using UI = BatchItem<FallbackArgsT<R>>;
     for (const Pass& p : g.passes) {
         const PI* pi = static_cast<const PI*>(p.items);
         const DI* di = static_cast<const DI*>(p.items);
+        const LI* li = static_cast<const LI*>(p.items);
         const UI* ui = static_cast<const UI*>(p.items);
         switch (p.kind) {
         case kPassPredict: k.predict<<<p.blocks, k.picard_threads, k.picard_smem[kPredict], st>>>(pi, p.n, dm); break;
         case kPassCorrect: k.correct<<<p.blocks, k.picard_threads, k.picard_smem[kCorrect], st>>>(pi, p.n, dm); break;
         case kPassFlux: k.flux<<<p.blocks, k.picard_threads, k.picard_smem[kFlux], st>>>(pi, p.n, dm); break;
         case kPassDetect: k.detect<<<p.blocks, kThreads, 0, st>>>(di, p.n); break;
+        case kPassBlend: k.blend<<<p.blocks, kThreads, k.blend_smem, st>>>(li, p.n, dm); break;
         case kPassUpdate: k.update<<<p.blocks, kThreads, k.update_smem, st>>>(ui, p.n, dm); break;
         }
     }

@@ -14,19 +14,26 @@
 
 namespace spdk {
 
+// Blended fluxes of one slice (blend kernel): the SD face fluxes of the faces
+// that the troubles reach are replaced in place
+template <typename R>
+struct BlendArgsT {
+    const R* ucv;             // U_cv at the start of slice t [E][V][NPT]
+    R* ff[3];                 // FV face fluxes of each direction, all slices
+    const uint8_t* trouble;   // [E][NPT]
+    const uint8_t* elem_any;  // [E]: any troubled sub-cell in the element
+    uint8_t* theta;           // [E][NPT], theta * 8 (zero on entry where no trouble is near)
+    int t;                    // slice
+    const double* dt;
+};
+
 template <typename R>
 struct FallbackArgsT {
     const R* ucv_in;        // U_cv at the start of slice t [E][V][NPT]
     R* ucv_out;             // U_cv after slice t
-    R* ff0;                 // FV face fluxes of each direction, all slices
-    R* ff1;
-    R* ff2;
-    const double2* rp_old;  // (rho, p) of U_old / U_new candidates of slice t
-    const double2* rp_new;
-    double2* rp_old_next;   // candidates of slice t+1
+    R* ff[3];               // FV face fluxes of each direction, all slices
+    double2* rp_old_next;   // (rho, p) of U_old / U_new candidates of slice t+1
     double2* rp_new_next;
-    uint8_t* trouble;       // [E][NPT]
-    uint8_t* theta;         // [E][NPT], theta * 8
     int t;                  // slice
     int last;               // last slice of the stage: U_sp = cv_to_sp(U_cv)
     R* u;                   // U_sp (written on the last slice)
@@ -36,7 +43,6 @@ struct FallbackArgsT {
     R* wcv;
     unsigned long long* dtmin;
     const double* dt;
-    int* any_trouble;       // diagnostic counter of troubled sub-cells (nullable)
     // learned indicator (nullable): after the final stage, the element means
     // of (rho, p) and the nodal part of each feature row (row length n_in)
     // of the new state, for the next step's a-priori flags
@@ -44,9 +50,16 @@ struct FallbackArgsT {
     float2* means;
     int n_in;
 };
-using FallbackArgs = FallbackArgsT<double>;
 
-// active FV cell -> (element, point) index of a [E][NPT] array
+// what a detect launch reads and writes
+struct DetectArgs {
+    const double2* rpo;  // (rho, p) of the U_old / U_new candidates
+    const double2* rpn;
+    uint8_t* T;          // troubles
+    uint8_t* theta;      // cleared for the blend kernel
+    uint8_t* elem_any;   // [E]: any troubled sub-cell
+};
+
 template <int D, int P>
 __device__ __forceinline__ long long cell_id(const DevGrid& G, const int a[3]) {
     constexpr int n = P + 1;
@@ -71,6 +84,66 @@ __device__ __forceinline__ long long cell_image(const DevGrid& G, const int a[3]
         m[d] = fv_image(a[d], G.N[d] * n, G.bc[d], &flips[d]);
     }
     return cell_id<D, P>(G, m);
+}
+
+// Cell numbers of a tile and its halo: the number of cell (x, y, z) of the
+// frame that begins H cells outside the tile is x0[x] + x1[y] + x2[z], each
+// part from the cell's image in that direction; a part is negative (kNoCell)
+// where there is none (outside the domain and its `layers` ghost layers), and
+// flip[d] marks reflective images. Formed once per block, so that a staged
+// cell costs two or three shared loads instead of the image arithmetic.
+constexpr int kNoCell = -(1 << 29);  // below minus any cell number (fewer than 2^29 cells fit the memory)
+template <int D, int P, int TX, int TY, int TZ, int H>
+struct CellMap {
+    static constexpr int n = P + 1;
+    static constexpr int Lx = TX * n + 2 * H, Ly = TY * n + 2 * H, Lz = D == 3 ? TZ * n + 2 * H : 1;
+    int x0[Lx], x1[Ly], x2[Lz];
+    uint8_t flip[Lx + Ly + Lz];
+    __device__ __forceinline__ void fill(const DevGrid& G, const int o[3], int layers) {
+        constexpr int NPT = Shape<D, P>::NPT;
+        for (int q = threadIdx.x; q < Lx + Ly + (D == 3 ? Lz : 0); q += blockDim.x) {
+            const int d = q < Lx ? 0 : (q < Lx + Ly ? 1 : 2);
+            const int i = q - (d == 0 ? 0 : (d == 1 ? Lx : Lx + Ly));
+            const int a = o[d] - H + i, na = G.N[d] * n;
+            const int g = G.bc[d] == kPeriodic ? layers : (layers < 2 ? layers : 2);
+            int part = kNoCell;
+            bool f = false;
+            if (a >= -g && a < na + g) {
+                const int m = fv_image(a, na, G.bc[d], &f), e = m / n, c = m - e * n;
+                if (d == 0) part = e * NPT + c;
+                else if (d == 1) part = e * G.N[0] * NPT + c * n;
+                else part = e * G.N[0] * G.N[1] * NPT + c * n * n;
+            }
+            (d == 0 ? x0 : (d == 1 ? x1 : x2))[i] = part;
+            flip[q] = f;
+        }
+        if (D == 2 && threadIdx.x == 0) x2[0] = 0;
+    }
+    // cell number, negative where the cell has no image
+    __device__ __forceinline__ int cell(int x, int y, int z) const {
+        return x0[x] + x1[y] + (D == 3 ? x2[z] : 0);
+    }
+};
+
+// a cell of the domain (tiles at the high edges may hang over it)
+template <int D, int P>
+__device__ __forceinline__ bool in_domain(const DevGrid& G, const int a[3]) {
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < D; d++) in &= a[d] < G.N[d] * (P + 1);
+    return in;
+}
+// a cell of the domain or of its first `layers` ghost layers (the ghost frame
+// of a non-periodic edge is two layers deep)
+template <int D, int P>
+__device__ __forceinline__ bool has_image(const DevGrid& G, const int a[3], int layers) {
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+        const int g = G.bc[d] == kPeriodic ? layers : (layers < 2 ? layers : 2);
+        in &= a[d] >= -g && a[d] < G.N[d] * (P + 1) + g;
+    }
+    return in;
 }
 
 __device__ __forceinline__ double rp_var(const double2 v, int k) { return k == 0 ? v.x : v.y; }
@@ -232,11 +305,10 @@ constexpr bool kSedStage3 =
 constexpr int kSedTileThreshold = 24;
 
 template <typename R, int D, int P, int TX, int TY, int TZ>
-__device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const double2* __restrict__ rpo,
-                                                            const double2* __restrict__ rpn,
-                                                            uint8_t* __restrict__ T, int* any_trouble, long long bidx) {
+__device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const DetectArgs& A, long long bidx) {
     constexpr int n = P + 1;
     constexpr int NPT = Shape<D, P>::NPT;
+    constexpr int NE = TX * TY * TZ;
     constexpr int Bx = TX * n, By = TY * n, Bz = D == 3 ? TZ * n : 1;
     constexpr int E1x = Bx + 2, E1y = By + 2, E1z = D == 3 ? Bz + 2 : 1;
     constexpr int NC = Bx * By * Bz;
@@ -244,33 +316,54 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const do
     static_assert(CPT <= 16, "NAD flag bits");
     constexpr int E3x = Bx + 6, E3y = By + 6, E3z = D == 3 ? Bz + 6 : 1;
     constexpr bool stage3 = kSedStage3<D, P, TX, TY, TZ>;
+    const double2* __restrict__ rpo = A.rpo;
+    const double2* __restrict__ rpn = A.rpn;
+    __shared__ int el_any[NE];
+    for (int e = threadIdx.x; e < NE; e += blockDim.x) el_any[e] = 0;
     __shared__ double2 Ro[E1x * E1y * E1z];
     __shared__ double2 Rn[D == 2 ? E3x * E3y : (stage3 ? E3x * E3y * E3z : 1)];
     __shared__ double Al[D == 2 ? 4 * E1x * E1y : 1];
+    __shared__ CellMap<D, P, TX, TY, TZ, 3> map;
     const int dz = D == 3 ? 1 : 0;
     int o[3];
     {
         int b = bidx;
-        const int tx = G.N[0] / TX, ty = G.N[1] / TY;
+        const int tx = (G.N[0] + TX - 1) / TX, ty = (G.N[1] + TY - 1) / TY;
         o[0] = (b % tx) * Bx;
         b /= tx;
         o[1] = (b % ty) * By;
         b /= ty;
         o[2] = D == 3 ? b * Bz : 0;
     }
+    map.fill(G, o, 3);
+    __syncthreads();
+    // this thread's cells, in memory order: element q / NPT, point q % NPT;
+    // cells of a tile that hangs over the domain: bit r is clear
+    auto place = [&](int q, int l[3]) {
+        const int el = q / NPT, pt = q % NPT;
+        l[0] = (el % TX) * n + pt % n;
+        l[1] = ((el / TX) % TY) * n + (pt / n) % n;
+        l[2] = D == 3 ? (el / (TX * TY)) * n + pt / (n * n) : 0;
+    };
+    unsigned mine = 0;
     double2 here_new[CPT];
 #pragma unroll
     for (int r = 0; r < CPT; r++) {
         const int q = threadIdx.x + r * kThreads;
+        here_new[r] = make_double2(1.0, 1.0);
         if (NC % kThreads == 0 || q < NC) {
-            int a[3] = {o[0] + q % Bx, o[1] + (q / Bx) % By, o[2] + q / (Bx * By)};
-            here_new[r] = rpn[cell_id<D, P>(G, a)];
+            int l[3];
+            place(q, l);
+            int a[3] = {o[0] + l[0], o[1] + l[1], o[2] + l[2]};
+            if (in_domain<D, P>(G, a)) {
+                mine |= 1u << r;
+                here_new[r] = rpn[map.cell(l[0] + 3, l[1] + 3, l[2] + 3 * dz)];
+            }
         }
     }
     for (int q = threadIdx.x; q < E1x * E1y * E1z; q += blockDim.x) {
-        int a[3] = {o[0] - 1 + q % E1x, o[1] - 1 + (q / E1x) % E1y, o[2] - dz + q / (E1x * E1y)};
-        bool fl[3];
-        Ro[q] = rpo[cell_image<D, P>(G, a, fl)];
+        const int id = map.cell(q % E1x + 2, (q / E1x) % E1y + 2, q / (E1x * E1y) + 2 * dz);
+        Ro[q] = id >= 0 ? rpo[id] : make_double2(1.0, 1.0);
     }
     __syncthreads();
     // NAD flags of this thread's cells: bit 2r + k for variable k of cell r
@@ -278,42 +371,46 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const do
 #pragma unroll
     for (int r = 0; r < CPT; r++) {
         const int q = threadIdx.x + r * kThreads;
-        if (NC % kThreads != 0 && q >= NC) break;
-        const int x = q % Bx, y = (q / Bx) % By, z = q / (Bx * By);
-        const int sc = (x + 1) + E1x * ((y + 1) + E1y * (z + dz));
+        if (!((mine >> r) & 1u)) continue;
+        int l[3];
+        place(q, l);
+        const int sc = (l[0] + 1) + E1x * ((l[1] + 1) + E1y * (l[2] + dz));
+        // extrema of both variables over the box (or the cross)
+        double2 mx = Ro[sc], mn = mx;
+        auto take = [&](const double2 u) {
+            mx.x = smax(mx.x, u.x);
+            mn.x = smin(mn.x, u.x);
+            mx.y = smax(mx.y, u.y);
+            mn.y = smin(mn.y, u.y);
+        };
+        if (G.nad_moore) {
+            for (int ok = -dz; ok <= dz; ok++)
+#pragma unroll
+                for (int oj = -1; oj <= 1; oj++)
+#pragma unroll
+                    for (int oi = -1; oi <= 1; oi++) take(Ro[sc + oi + E1x * (oj + E1y * ok)]);
+        } else {
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+                const int st = d == 0 ? 1 : (d == 1 ? E1x : E1x * E1y);
+                const double2 uL = Ro[sc - st], uR = Ro[sc + st];
+                mx = make_double2(smax(smax(uL.x, mx.x), uR.x), smax(smax(uL.y, mx.y), uR.y));
+                mn = make_double2(smin(smin(uL.x, mn.x), uR.x), smin(smin(uL.y, mn.y), uR.y));
+            }
+        }
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const double un = rp_var(here_new[r], k);
-            double mx = rp_var(Ro[sc], k), mn = mx;
-            if (G.nad_moore) {
-                for (int ok = -dz; ok <= dz; ok++)
-#pragma unroll
-                    for (int oj = -1; oj <= 1; oj++)
-#pragma unroll
-                        for (int oi = -1; oi <= 1; oi++) {
-                            const double u = rp_var(Ro[sc + oi + E1x * (oj + E1y * ok)], k);
-                            mx = smax(mx, u);
-                            mn = smin(mn, u);
-                        }
-            } else {
-#pragma unroll
-                for (int d = 0; d < D; d++) {
-                    const int st = d == 0 ? 1 : (d == 1 ? E1x : E1x * E1y);
-                    const double uL = rp_var(Ro[sc - st], k);
-                    const double uR = rp_var(Ro[sc + st], k);
-                    mx = smax(smax(uL, mx), uR);
-                    mn = smin(smin(uL, mn), uR);
-                }
-            }
+            double hi = rp_var(mx, k), lo = rp_var(mn, k);
             if (G.nad_delta) {
-                const double eps = G.nad_tol * (mx - mn);
-                mn -= eps;
-                mx += eps;
+                const double eps = G.nad_tol * (hi - lo);
+                lo -= eps;
+                hi += eps;
             } else {
-                mn -= fabs(mn) * G.nad_tol;
-                mx += fabs(mx) * G.nad_tol;
+                lo -= fabs(lo) * G.nad_tol;
+                hi += fabs(hi) * G.nad_tol;
             }
-            if (un > mx || un < mn) nad |= 1u << (2 * r + k);
+            if (un > hi || un < lo) nad |= 1u << (2 * r + k);
         }
     }
     // SED relaxation of the NAD flags (it can only clear one). In 2D, and
@@ -324,14 +421,9 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const do
     if (nflag) {
         if (D == 2 || stage3) {
             for (int q = threadIdx.x; q < E3x * E3y * E3z; q += blockDim.x) {
-                int a[3] = {o[0] - 3 + q % E3x, o[1] - 3 + (q / E3x) % E3y, o[2] - 3 * dz + q / (E3x * E3y)};
-                // three cells outside a non-periodic boundary: never read
-                bool outside = false;
-#pragma unroll
-                for (int d = 0; d < D; d++)
-                    outside |= G.bc[d] != kPeriodic && (a[d] < -2 || a[d] >= G.N[d] * n + 2);
-                bool fl[3];
-                Rn[q] = outside ? make_double2(0.0, 0.0) : rpn[cell_image<D, P>(G, a, fl)];
+                // (three cells outside a non-periodic boundary: never read)
+                const int id = map.cell(q % E3x, (q / E3x) % E3y, q / (E3x * E3y));
+                Rn[q] = id >= 0 ? rpn[id] : make_double2(0.0, 0.0);
             }
             __syncthreads();
         }
@@ -359,8 +451,9 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const do
 #pragma unroll
                     for (int r = 0; r < CPT; r++) {
                         if (!(nad & (1u << (2 * r + k)))) continue;
-                        const int q = threadIdx.x + r * kThreads;
-                        const int x = q % Bx, y = (q / Bx) % By, z = q / (Bx * By);
+                        int l[3];
+                        place(threadIdx.x + r * kThreads, l);
+                        const int x = l[0], y = l[1], z = l[2];
                         double alpha = 1;
 #pragma unroll
                         for (int d = 0; d < 3; d++) {
@@ -390,8 +483,9 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const do
 #pragma unroll
             for (int r = 0; r < CPT; r++) {
                 if (!(nad & (3u << (2 * r)))) continue;
-                const int q = threadIdx.x + r * kThreads;
-                int a[3] = {o[0] + q % Bx, o[1] + (q / Bx) % By, o[2] + q / (Bx * By)};
+                int l[3];
+                place(threadIdx.x + r * kThreads, l);
+                int a[3] = {o[0] + l[0], o[1] + l[1], o[2] + l[2]};
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
                     if (!(nad & (1u << (2 * r + k)))) continue;
@@ -424,34 +518,40 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const do
 #pragma unroll
     for (int r = 0; r < CPT; r++) {
         const int q = threadIdx.x + r * kThreads;
-        if (NC % kThreads != 0 && q >= NC) break;
-        int a[3] = {o[0] + q % Bx, o[1] + (q / Bx) % By, o[2] + q / (Bx * By)};
-        const long long cid = cell_id<D, P>(G, a);
+        if (!((mine >> r) & 1u)) continue;
+        int l[3];
+        place(q, l);
+        const int cid = map.cell(l[0] + 3, l[1] + 3, l[2] + 3 * dz);
         bool tr = (nad >> (2 * r)) & 3u;
         const double rho = here_new[r].x, p = here_new[r].y;
         if (rho < kRhoMin || rho > kRhoMax) tr = true;
         if (p < kPMin || p > kPMax) tr = true;
-        const long long el = cid / NPT;
+        const int el = cid / NPT;
         if (G.elem_trouble && tr) G.elem_trouble[el] = 1;  // a-posteriori label
         if (G.elem_pred && G.elem_pred[el]) tr = true;     // a-priori prediction
-        T[cid] = tr ? 1 : 0;
-        if (any_trouble && tr) atomicAdd(any_trouble, 1);
+        A.T[cid] = tr ? 1 : 0;
+        A.theta[cid] = 0;
+        if (tr) el_any[q / NPT] = 1;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < NE; e += blockDim.x) {
+        const int g0 = o[0] / n + e % TX, g1 = o[1] / n + (e / TX) % TY, g2 = o[2] / n + e / (TX * TY);
+        if (g0 < G.N[0] && g1 < G.N[1] && (D == 2 || g2 < G.N[2]))
+            A.elem_any[((long long)g2 * G.N[1] + g1) * G.N[0] + g0] = (uint8_t)el_any[e];
     }
 }
 
 template <typename R, int D, int P, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(kThreads, kDetectBlocksPerSM<D>) fv_detect_kernel(DevGrid G, const double2* __restrict__ rpo,
-                                                            const double2* __restrict__ rpn,
-                                                            uint8_t* __restrict__ T, int* any_trouble) {
+__global__ void __launch_bounds__(kThreads, kDetectBlocksPerSM<D>) fv_detect_kernel(DevGrid G, DetectArgs A) {
     pdl_wait();
     if (gate_closed(G)) return;
-    fv_detect_kernel_body<R, D, P, TX, TY, TZ>(G, rpo, rpn, T, any_trouble, blockIdx.x);
+    fv_detect_kernel_body<R, D, P, TX, TY, TZ>(G, A, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
 // theta = max over the Moore box of w(#offsets) * trouble, plus the 0.25 ring
 // (src/trouble_detection.cpp:191-242; theta_from_troubles without blending),
-// evaluated by the update kernel on its tile + 1 halo from the troubles on
+// evaluated by the blend kernel on its tile + 1 halo from the troubles on
 // the tile + 3 halo, in eighths: w * 8 = 8, 6, 4, 3 and the ring 2 (all
 // exact, as is theta * 8 of the reference's float weights).
 //
@@ -476,46 +576,23 @@ struct ThetaTile {
 
 // called by every thread of the block; `scratch` holds ThetaTile::scratch
 // bytes; th (tile + 1 halo) is complete after the caller's next barrier.
-// Returns (to every thread) whether any trouble lies within reach of the
-// tile: when none does, theta is zero on the tile + 1 halo and the blending
-// passes are skipped.
+// theta_out of the tile's cells was cleared by the detection.
 template <int D, int P, int TX, int TY, int TZ>
-__device__ __forceinline__ int theta_on_tile(const DevGrid& G, const uint8_t* __restrict__ T, const int o[3],
-                                             uint8_t* scratch, uint8_t* th, uint8_t* __restrict__ theta_out) {
+__device__ __forceinline__ void theta_on_tile(const DevGrid& G, const CellMap<D, P, TX, TY, TZ, 3>& map,
+                                              const uint8_t* __restrict__ T, const int o[3], uint8_t* scratch, uint8_t* th, uint8_t* __restrict__ theta_out) {
     using TT = ThetaTile<D, P, TX, TY, TZ>;
     constexpr int n = P + 1;
     const int dz = D == 3 ? 1 : 0;
     uint8_t* T3 = scratch;
     uint8_t* Th2 = scratch + TT::n3;
-    int any = 0;
     for (int q = threadIdx.x; q < TT::n3; q += blockDim.x) {
-        int a[3] = {o[0] - 3 + q % TT::E3x, o[1] - 3 + (q / TT::E3x) % TT::E3y, o[2] - 3 * dz + q / (TT::E3x * TT::E3y)};
         // a cell three layers outside a non-periodic boundary has no image
         // (the ghost frame is two layers deep) and feeds no theta below:
         // the theta of a ghost cell there is its image's
-        bool outside = false;
-#pragma unroll
-        for (int d = 0; d < D; d++)
-            outside |= G.bc[d] != kPeriodic && (a[d] < -2 || a[d] >= G.N[d] * n + 2);
-        bool fl[3];
-        const uint8_t tq = outside ? (uint8_t)0 : T[cell_image<D, P>(G, a, fl)];
-        T3[q] = tq;
-        any |= tq;
+        const int id = map.cell(q % TT::E3x, (q / TT::E3x) % TT::E3y, q / (TT::E3x * TT::E3y));
+        T3[q] = id >= 0 ? T[id] : (uint8_t)0;
     }
-    if (!__syncthreads_or(any)) {
-        // no trouble within three cells of the tile: theta is zero on it
-        for (int q = threadIdx.x; q < TT::n1; q += blockDim.x) {
-            th[q] = 0;
-            const int l0[3] = {q % TT::E1x, (q / TT::E1x) % TT::E1y, q / (TT::E1x * TT::E1y)};
-            const bool inner = l0[0] >= 1 && l0[0] <= TT::Bx && l0[1] >= 1 && l0[1] <= TT::By &&
-                               (D == 2 || (l0[2] >= 1 && l0[2] <= TT::Bz));
-            if (inner) {
-                int ga[3] = {o[0] + l0[0] - 1, o[1] + l0[1] - 1, o[2] + l0[2] - dz};
-                theta_out[cell_id<D, P>(G, ga)] = 0;
-            }
-        }
-        return 0;
-    }
+    __syncthreads();
     if (G.blending) {
         for (int q = threadIdx.x; q < TT::n2; q += blockDim.x) {
             const int x = q % TT::E2x + 1, y = (q / TT::E2x) % TT::E2y + 1, z = q / (TT::E2x * TT::E2y) + dz;
@@ -536,12 +613,17 @@ __device__ __forceinline__ int theta_on_tile(const DevGrid& G, const uint8_t* __
     for (int q = threadIdx.x; q < TT::n1; q += blockDim.x) {
         const int l0[3] = {q % TT::E1x, (q / TT::E1x) % TT::E1y, q / (TT::E1x * TT::E1y)};
         int l[3] = {l0[0], l0[1], l0[2]};
+        int ga[3] = {o[0] + l0[0] - 1, o[1] + l0[1] - 1, o[2] + l0[2] - dz};
+        if (!has_image<D, P>(G, ga, 1)) {
+            th[q] = 0;
+            continue;
+        }
 #pragma unroll
         for (int d = 0; d < D; d++) {
-            const int a = o[d] - 1 + l[d], na = G.N[d] * n;
-            if ((a < 0 || a >= na) && G.bc[d] != kPeriodic) {
+            const int na = G.N[d] * n;
+            if ((ga[d] < 0 || ga[d] >= na) && G.bc[d] != kPeriodic) {
                 bool f = false;
-                l[d] = fv_image(a, na, G.bc[d], &f) - o[d] + 1;
+                l[d] = fv_image(ga[d], na, G.bc[d], &f) - o[d] + 1;
             }
         }
         int t8;
@@ -562,22 +644,17 @@ __device__ __forceinline__ int theta_on_tile(const DevGrid& G, const uint8_t* __
         th[q] = (uint8_t)t8;
         const bool inner = l0[0] >= 1 && l0[0] <= TT::Bx && l0[1] >= 1 && l0[1] <= TT::By &&
                            (D == 2 || (l0[2] >= 1 && l0[2] <= TT::Bz));
-        if (inner) {
-            int ga[3] = {o[0] + l0[0] - 1, o[1] + l0[1] - 1, o[2] + l0[2] - dz};
-            theta_out[cell_id<D, P>(G, ga)] = (uint8_t)t8;
-        }
+        if (inner && in_domain<D, P>(G, ga)) theta_out[map.cell(l0[0] + 2, l0[1] + 2, l0[2] + 2 * dz)] = (uint8_t)t8;
     }
-    return 1;
 }
 
-// MUSCL-Hancock face states of cell X for a face of direction Dn
-// (src/hydro.cpp:622-681); returns the state on the cell's low face (wlo)
-// and high face (whi). Wc(offset) gives W_old of neighbouring cells.
+// Limited slopes of W_old along every direction and the Hancock time
+// derivative of cell fa (frame indices), from W_old around it
+// (src/hydro.cpp:622-681); Wc(oi, oj, ok) gives W_old of neighbouring cells
 template <int D, typename R, typename WF>
-__device__ __forceinline__ void muscl_cell(const DevGrid& G, const int fa[3], int Dn, R dtw, WF Wc,
-                                           R* wlo, R* whi) {
+__device__ __forceinline__ void muscl_slopes(const DevGrid& G, const int fa[3], WF Wc, R (*dW)[D + 2], R* dwt) {
     constexpr int V = D + 2;
-    R w[V], dW[D][V], dwt[V];
+    R w[V];
     const R* wc = Wc(0, 0, 0);
 #pragma unroll
     for (int v = 0; v < V; v++) w[v] = wc[v];
@@ -585,85 +662,88 @@ __device__ __forceinline__ void muscl_cell(const DevGrid& G, const int fa[3], in
     for (int d = 0; d < D; d++) {
         const R* wm = Wc(d == 0 ? -1 : 0, d == 1 ? -1 : 0, d == 2 ? -1 : 0);
         const R* wp = Wc(d == 0 ? 1 : 0, d == 1 ? 1 : 0, d == 2 ? 1 : 0);
-        const double* xc = G.fvc[d];
-        const double* xf = G.fvf[d];
-        const int i = fa[d];
+        const Width dp = G.fd[d][fa[d]], dm = G.fd[d][fa[d] - 1];
+        const R h = (R)G.fw[d][fa[d]].h;
 #pragma unroll
         for (int v = 0; v < V; v++)
-            dW[d][v] = minmod((wp[v] - w[v]) / (R)(xc[i + 1] - xc[i]), (w[v] - wm[v]) / (R)(xc[i] - xc[i - 1]),
-                              (R)xf[i], (R)xf[i + 1]);
+            dW[d][v] = minmod(div_width(G, wp[v] - w[v], dp), div_width(G, w[v] - wm[v], dm), h);
     }
     hancock<D>(w, dwt, dW, (R)G.gm);
-    const double* xf = G.fvf[Dn];
-    const int i = fa[Dn];
-    const R h = (R)(xf[i + 1] - xf[i]);
-#pragma unroll
-    for (int v = 0; v < V; v++) {
-        const R dw = dW[Dn][v];
-        whi[v] = w[v] + dw + dwt[v] * dtw / h;  // reference "WL": left state of the high face
-        wlo[v] = w[v] - dw + dwt[v] * dtw / h;  // reference "WR": right state of the low face
-    }
 }
 
-// resident blocks the update kernel is compiled for: 5 (48 registers) in 2D,
-// where the extra warps hide its gather latency (measured on B200 at 256^2,
-// p = 3: 62.6 against 72.0 us in FP32, 139 against 176 us in FP64). In 3D
-// (one element per block) the 140-register kernel ran one block per SM;
-// measured per step of 4 updates, FP64: 32^3 p=3 6.15 / 3.47 / 2.52 ms at
-// 2 / 3 / 4 blocks, 16^3 p=5 4.13 / 3.65 / 4.05 ms. The FP32 3D update
-// above p = 3 fits 4 blocks without spills (64 registers) and takes them:
-// KH 16^3 p=5 FP32 step 4.91 -> 4.68 ms together with the 3D detection's
-// 3 blocks.
+// ---------------------------------------------------------------------------
+// Blend kernel of slice t: fluxes of the faces with theta > 0
+// (src/hydro.cpp:683-788) written over the SD face fluxes, each element's own
+// copy of an interface.
+//
+// A tile without trouble within three cells returns after looking at the
+// flags of the elements around it. On the others W_old is formed once on the
+// tile + 2 halo, the slopes of a cell once for all its faces (they were formed
+// by every face for both of its cells: 4 times a cell in 2D, 6 in 3D, with
+// the divisions that dominate them in FP64), and each face takes one HLLC
+// solve. Bounded by the latency of its chain of phases: it is separate from
+// the update, whose blocks would otherwise all reserve the shared memory and
+// wait for the few that blend.
+// ---------------------------------------------------------------------------
+// elements of a blend block: 4 x 4 up to p = 3 and 2 x 2 above in 2D, 2 x 1 x 1
+// up to p = 3 and one above in 3D
 template <int D, int P>
-constexpr int kUpdateBlocksPerSM = D == 2 ? 5 : (P <= 3 ? 4 : 3);
+struct BlendTile {
+    static constexpr int X = D == 2 ? (P <= 3 ? 4 : 2) : (P <= 3 ? 2 : 1);
+    static constexpr int Y = D == 2 ? (P <= 3 ? 4 : 2) : 1;
+    static constexpr int Z = 1;
+};
 
 template <typename R, int D, int P, int TX, int TY, int TZ>
-struct UpdateSmem {
+struct BlendSmem {
     static constexpr int n = P + 1, V = D + 2;
-    static constexpr int NPT = Shape<D, P>::NPT;
-    static constexpr int NE = TX * TY * TZ;
     static constexpr int Bx = TX * n, By = TY * n, Bz = D == 3 ? TZ * n : 1;
-    static constexpr int NC = Bx * By * Bz;
     static constexpr int E1x = Bx + 2, E1y = By + 2, E1z = D == 3 ? Bz + 2 : 1;
     static constexpr int E2x = Bx + 4, E2y = By + 4, E2z = D == 3 ? Bz + 4 : 1;
+    static constexpr int n1 = E1x * E1y * E1z, n2 = E2x * E2y * E2z;
     static constexpr int NF0 = (Bx + 1) * By * Bz;
     static constexpr int NF1 = Bx * (By + 1) * Bz;
     static constexpr int NF2 = D == 3 ? Bx * By * (Bz + 1) : 0;
-    static constexpr size_t faces = (size_t)(NF0 + NF1 + NF2) * V;
-    static constexpr size_t wold = (size_t)E2x * E2y * E2z * V;
-    static constexpr size_t epi = 2 * (size_t)NE * V * NPT;
-    static constexpr size_t reals = faces + (wold > epi ? wold : epi);
-    static_assert(ThetaTile<D, P, TX, TY, TZ>::scratch <= (wold > epi ? wold : epi) * sizeof(R),
-                  "theta scratch fits the W_old area");
-    static_assert((size_t)NE * NPT * 16 + NE * 8 <= faces * sizeof(R), "indicator scratch fits the face area");
-    static constexpr size_t bytes = reals * sizeof(R) + ((size_t)E1x * E1y * E1z + 15) / 16 * 16;
+    // cells whose slopes some face of the tile needs: the tile's own, then the
+    // ones across its low and high x, y (and z) faces
+    static constexpr int NC = Bx * By * Bz, HX = By * Bz, HY = Bx * Bz, HZ = D == 3 ? Bx * By : 0;
+    static constexpr int ns = NC + 2 * (HX + HY + HZ);
+    __device__ static int slot(int x, int y, int z) {  // tile coordinates, at most one of them outside
+        if (x < 0 || x >= Bx) return NC + (x < 0 ? 0 : HX) + y + By * z;
+        if (y < 0 || y >= By) return NC + 2 * HX + (y < 0 ? 0 : HY) + x + Bx * z;
+        if (z < 0 || z >= Bz) return NC + 2 * (HX + HY) + (z < 0 ? 0 : HZ) + x + Bx * y;
+        return x + Bx * (y + By * z);
+    }
+    __device__ static void coords(int q, int l[3]) {
+        if (q < NC) { l[0] = q % Bx; l[1] = (q / Bx) % By; l[2] = q / (Bx * By); return; }
+        q -= NC;
+        if (q < 2 * HX) { l[0] = q < HX ? -1 : Bx; q %= HX; l[1] = q % By; l[2] = q / By; return; }
+        q -= 2 * HX;
+        if (q < 2 * HY) { l[1] = q < HY ? -1 : By; q %= HY; l[0] = q % Bx; l[2] = q / Bx; return; }
+        q -= 2 * HY;
+        l[2] = q < HZ ? -1 : Bz;
+        q %= HZ > 0 ? HZ : 1;
+        l[0] = q % Bx;
+        l[1] = q / Bx;
+    }
+    static constexpr size_t slopes = (size_t)ns * (D + 1) * V;  // [D slopes, dW/dt][V][cell]
+    static constexpr size_t wold = (size_t)n2 * V;
+    static_assert(ThetaTile<D, P, TX, TY, TZ>::scratch <= slopes * sizeof(R), "theta scratch fits the slopes' area");
+    static constexpr size_t bytes = (slopes + wold) * sizeof(R) + ((size_t)n1 + 15) / 16 * 16;
 };
 
-// ---------------------------------------------------------------------------
-// Blended fluxes and the corrected sub-cell update of slice t
-// (src/hydro.cpp:683-788, src/transforms.cpp:483-543 with update=1), then
-// either the next slice's candidate or, after the last slice,
-// U_sp = cv_to_sp(U_cv), the RK combination, W_cv and the next dt.
-// ---------------------------------------------------------------------------
 template <typename R, int D, int P, int TX, int TY, int TZ>
-__device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const DevMatsT<R>& M, const FallbackArgsT<R>& A, long long bidx) {
-    using SM = UpdateSmem<R, D, P, TX, TY, TZ>;
-    constexpr int n = P + 1, nf = P + 2, V = D + 2, NPT = SM::NPT, NFP = Shape<D, P>::NFP;
-    constexpr int Bx = SM::Bx, By = SM::By, Bz = SM::Bz, NC = SM::NC;
-    constexpr int E1x = SM::E1x, E1y = SM::E1y, E2x = SM::E2x, E2y = SM::E2y;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    R* smem = reinterpret_cast<R*>(smem_raw);
-    R* Fs = smem;                                   // faces of the tile, [face][V]
-    R* Wo = Fs + SM::faces;                         // W_old on the tile + 2 halo
-    uint8_t* th = (uint8_t*)(Wo + (SM::wold > SM::epi ? SM::wold : SM::epi));
-    __shared__ long long el_ge[SM::NE];
+__device__ __forceinline__ void fv_blend_kernel_body(const DevGrid& G, const DevMatsT<R>& M, const BlendArgsT<R>& A,
+                                                     long long bidx) {
+    using SM = BlendSmem<R, D, P, TX, TY, TZ>;
+    constexpr int n = P + 1, nf = P + 2, V = D + 2, NPT = Shape<D, P>::NPT, NFP = Shape<D, P>::NFP;
+    constexpr int Bx = SM::Bx, By = SM::By, Bz = SM::Bz;
+    constexpr int E1x = SM::E1x, E1y = SM::E1y, E2x = SM::E2x, E2y = SM::E2y, ns = SM::ns;
     const int dz = D == 3 ? 1 : 0;
-    R* const ffd[3] = {A.ff0, A.ff1, A.ff2};
-
     int o[3], oe[3];
     {
-        int b = bidx;
-        const int tx = G.N[0] / TX, ty = G.N[1] / TY;
+        int b = (int)bidx;
+        const int tx = (G.N[0] + TX - 1) / TX, ty = (G.N[1] + TY - 1) / TY;
         oe[0] = (b % tx) * TX;
         b /= tx;
         oe[1] = (b % ty) * TY;
@@ -673,134 +753,216 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
         o[1] = oe[1] * n;
         o[2] = oe[2] * n;
     }
-    for (int s = threadIdx.x; s < SM::NE; s += blockDim.x) {
-        const int lx = s % TX, ly = (s / TX) % TY, lz = s / (TX * TY);
-        el_ge[s] = ((long long)(oe[2] + lz) * G.N[1] + (oe[1] + ly)) * G.N[0] + (oe[0] + lx);
-    }
-    __syncthreads();  // el_ge is read by every thread below
-    const R dt = (R)(*A.dt);
-    const R wdt = M.wt[A.t] * dt;
-    const long long E = G.E;
-    // theta on the tile + 1 halo from the troubles (scratch: the W_old area,
-    // written only after the barrier that follows)
-    const int near = theta_on_tile<D, P, TX, TY, TZ>(G, A.trouble, o, reinterpret_cast<uint8_t*>(Wo), th, A.theta);
-    // SD face fluxes of the tile
-    const int nfaces[3] = {SM::NF0, SM::NF1, SM::NF2};
-    int fbase[3] = {0, SM::NF0, SM::NF0 + SM::NF1};
-    // direction loops unrolled: ffd, nfaces and fbase stay in registers
+    // any trouble within three cells: the elements they lie in
+    {
+        constexpr int K = (3 + n - 1) / n;
+        constexpr int Mx = TX + 2 * K, My = TY + 2 * K, Mz = D == 3 ? TZ + 2 * K : 1;
+        int any = 0;
+        for (int q = threadIdx.x; q < Mx * My * Mz; q += blockDim.x) {
+            int g[3] = {oe[0] - K + q % Mx, oe[1] - K + (q / Mx) % My, D == 3 ? oe[2] - K + q / (Mx * My) : 0};
+            bool in = true;
 #pragma unroll
-    for (int d = 0; d < D; d++) {
-        const int ex = Bx + (d == 0), ey = By + (d == 1);
-        for (int q = threadIdx.x; q < nfaces[d]; q += blockDim.x) {
-            int a[3] = {q % ex, (q / ex) % ey, q / (ex * ey)};  // tile-local: face a[d] is the low face of cell a
-            int cl[3] = {a[0], a[1], a[2]};
-            int llv;
-            if (a[d] == (d == 0 ? Bx : (d == 1 ? By : Bz))) { cl[d] = a[d] - 1; llv = n; }
-            else llv = -1;
-            const int el = (cl[0] / n) + TX * ((cl[1] / n) + TY * (cl[2] / n));
-            int c[3] = {cl[0] % n, cl[1] % n, cl[2] % n};
-            if (llv < 0) llv = c[d];
-            c[d] = llv;
-            const int fi = fp_index<n, nf>(d, c);
-            const R* src = ffd[d] + ((long long)A.t * E + el_ge[el]) * V * NFP;
-            R* dst = Fs + (size_t)(fbase[d] + q) * V;
-#pragma unroll
-            for (int v = 0; v < V; v++) dst[v] = src[v * NFP + fi];
+            for (int d = 0; d < D; d++) {
+                if (g[d] >= 0 && g[d] < G.N[d]) continue;
+                // ghosts of a non-periodic edge are images of the tile's own cells
+                if (G.bc[d] != kPeriodic) in = false;
+                else g[d] = (g[d] + K * G.N[d]) % G.N[d];
+            }
+            if (in) any |= A.elem_any[((long long)g[2] * G.N[1] + g[1]) * G.N[0] + g[0]];
         }
+        if (!__syncthreads_or(any)) return;
+    }
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    R* SL = reinterpret_cast<R*>(smem_raw);  // slopes and dW/dt on the tile + 1 halo
+    R* Wo = SL + SM::slopes;                 // W_old on the tile + 2 halo
+    uint8_t* th = (uint8_t*)(Wo + SM::wold);
+    __shared__ CellMap<D, P, TX, TY, TZ, 3> map;
+    map.fill(G, o, 3);
+    __syncthreads();
+    // W_old = prim(U_cv), reflective images flipped
+    for (int q = threadIdx.x; q < SM::n2; q += blockDim.x) {
+        const int x = q % E2x + 1, y = (q / E2x) % E2y + 1, z = q / (E2x * E2y) + dz;
+        const int cid = map.cell(x, y, z);
+        if (cid < 0) continue;
+        const bool fl[3] = {map.flip[x] != 0, map.flip[map.Lx + y] != 0, D == 3 && map.flip[map.Lx + map.Ly + z] != 0};
+        const long long ge = cid / NPT;
+        const int pt = cid % NPT;
+        R u[V], w[V];
+#pragma unroll
+        for (int v = 0; v < V; v++) u[v] = A.ucv[(ge * V + v) * NPT + pt];
+        primitives<D>(u, w, (R)G.gm);
+#pragma unroll
+        for (int d = 0; d < D; d++)
+            if (fl[d]) w[1 + d] = -w[1 + d];
+#pragma unroll
+        for (int v = 0; v < V; v++) Wo[(size_t)q * V + v] = w[v];
+    }
+    theta_on_tile<D, P, TX, TY, TZ>(G, map, A.trouble, o, reinterpret_cast<uint8_t*>(SL), th, A.theta);
+    __syncthreads();
+    // slopes of the tile's cells and of the cells across its faces, where
+    // one of the cell's faces blends
+    for (int q = threadIdx.x; q < ns; q += blockDim.x) {
+        int l[3];
+        SM::coords(q, l);
+        int a[3] = {o[0] + l[0], o[1] + l[1], o[2] + l[2]};
+        if (!has_image<D, P>(G, a, 1)) continue;
+        const bool ox = l[0] < 0 || l[0] == Bx, oy = l[1] < 0 || l[1] == By, oz = D == 3 && (l[2] < 0 || l[2] == Bz);
+        const int t0 = (l[0] + 1) + E1x * ((l[1] + 1) + E1y * (l[2] + dz));
+        int near = th[t0];
+        if (!oy && !oz) near |= (l[0] >= 0 ? th[t0 - 1] : 0) | (l[0] < Bx ? th[t0 + 1] : 0);
+        if (!ox && !oz) near |= (l[1] >= 0 ? th[t0 - E1x] : 0) | (l[1] < By ? th[t0 + E1x] : 0);
+        if (D == 3 && !ox && !oy)
+            near |= (l[2] >= 0 ? th[t0 - E1x * E1y] : 0) | (l[2] < Bz ? th[t0 + E1x * E1y] : 0);
+        if (!near) continue;
+        int fa[3] = {a[0] + 2, a[1] + 2, a[2] + 2};
+        auto Wc = [&](int oi, int oj, int ok) -> const R* {
+            return Wo + (size_t)((l[0] + 2 + oi) + E2x * ((l[1] + 2 + oj) + E2y * (l[2] + 2 * dz + ok))) * V;
+        };
+        R dW[D][V], dwt[V];
+        muscl_slopes<D, R>(G, fa, Wc, dW, dwt);
+#pragma unroll
+        for (int d = 0; d < D; d++)
+#pragma unroll
+            for (int v = 0; v < V; v++) SL[(d * V + v) * ns + q] = dW[d][v];
+#pragma unroll
+        for (int v = 0; v < V; v++) SL[(D * V + v) * ns + q] = dwt[v];
     }
     __syncthreads();
-    // faces that blend in the fallback flux (none when no trouble is near)
-    int need = 0;
+    const R wdt = M.wt[A.t] * (R)(*A.dt);
+    const long long E = G.E;
+    const int nfaces[3] = {SM::NF0, SM::NF1, SM::NF2};
 #pragma unroll
     for (int d = 0; d < D; d++) {
-        if (need || !near) break;
         const int ex = Bx + (d == 0), ey = By + (d == 1);
+        const int Bd = d == 0 ? Bx : (d == 1 ? By : Bz);
         for (int q = threadIdx.x; q < nfaces[d]; q += blockDim.x) {
-            int a[3] = {q % ex, (q / ex) % ey, q / (ex * ey)};
+            const int a[3] = {q % ex, (q / ex) % ey, q / (ex * ey)};  // the low face of cell a
             const int sR = (a[0] + 1) + E1x * ((a[1] + 1) + E1y * (a[2] + dz));
             const int sL = sR - (d == 0 ? 1 : (d == 1 ? E1x : E1x * E1y));
-            if (th[sR] | th[sL]) { need = 1; break; }
-        }
-    }
-    need = near ? __syncthreads_or(need) : 0;
-    if (need) {
-        // W_old = prim(U_cv) on the tile + 2 halo, reflective images flipped
-        for (int q = threadIdx.x; q < E2x * E2y * SM::E2z; q += blockDim.x) {
-            int a[3] = {o[0] - 2 + q % E2x, o[1] - 2 + (q / E2x) % E2y, o[2] - 2 * dz + q / (E2x * E2y)};
-            bool fl[3] = {false, false, false};
-            const long long cid = cell_image<D, P>(G, a, fl);
-            const long long ge = cid / NPT;
-            const int pt = (int)(cid - ge * NPT);
-            R u[V], w[V];
+            const R tR = (R)(th[sR] * 0.125), tL = (R)(th[sL] * 0.125);
+            const R tf = smax(tR, tL);
+            if (!(tf > 0)) continue;
+            bool in = true;
 #pragma unroll
-            for (int v = 0; v < V; v++) u[v] = A.ucv_in[(ge * V + v) * NPT + pt];
-            primitives<D>(u, w, (R)G.gm);
+            for (int e = 0; e < D; e++) in &= o[e] + a[e] < G.N[e] * n + (e == d);
+            if (!in) continue;
+            const int wR = (a[0] + 2) + E2x * ((a[1] + 2) + E2y * (a[2] + 2 * dz));
+            const int wL = wR - (d == 0 ? 1 : (d == 1 ? E2x : E2x * E2y));
+            const int cR = SM::slot(a[0], a[1], a[2]);
+            const int cL = SM::slot(a[0] - (d == 0), a[1] - (d == 1), a[2] - (d == 2));
+            const Width hR = G.fw[d][o[d] + a[d] + 2], hL = G.fw[d][o[d] + a[d] + 1];
+            R whi[V], wlo[V];
 #pragma unroll
-            for (int d = 0; d < D; d++)
-                if (fl[d]) w[1 + d] = -w[1 + d];
+            for (int v = 0; v < V; v++) {
+                whi[v] = Wo[(size_t)wL * V + v] + SL[(d * V + v) * ns + cL] +
+                         div_width(G, SL[(D * V + v) * ns + cL] * wdt, hL);
+                wlo[v] = Wo[(size_t)wR * V + v] - SL[(d * V + v) * ns + cR] +
+                         div_width(G, SL[(D * V + v) * ns + cR] * wdt, hR);
+            }
+            R uL[V], uR[V], fL[V];
+            conservatives<D>(whi, uL, (R)G.gm);
+            conservatives<D>(wlo, uR, (R)G.gm);
+            riemann_hllc<D>(fL, uL, uR, d, (R)G.gm);
+            // the copies of the face in the tile's elements: of the element
+            // on its high side (flux point 0 at an interface) and, at an
+            // interface, of the one on its low side
+            const bool iface = a[d] % n == 0;
 #pragma unroll
-            for (int v = 0; v < V; v++) Wo[(size_t)q * V + v] = w[v];
-        }
-        __syncthreads();
-        for (int d = 0; d < D; d++) {
-            const int ex = Bx + (d == 0), ey = By + (d == 1);
-            for (int q = threadIdx.x; q < nfaces[d]; q += blockDim.x) {
-                int a[3] = {q % ex, (q / ex) % ey, q / (ex * ey)};
-                const int sR = (a[0] + 1) + E1x * ((a[1] + 1) + E1y * (a[2] + dz));
-                const int sL = sR - (d == 0 ? 1 : (d == 1 ? E1x : E1x * E1y));
-                const R tR = (R)(th[sR] * 0.125), tL = (R)(th[sL] * 0.125);
-                const R tf = smax(tR, tL);
-                if (!(tf > 0)) continue;
-                // cells L (low) and R (high) of the face; W_old box index
-                R wlo_R[V], whi_R[V], wlo_L[V], whi_L[V];
-                for (int side = 0; side < 2; side++) {
-                    int cb[3] = {a[0] + 2, a[1] + 2, a[2] + 2 * dz};
-                    if (side == 0) cb[d] -= 1;
-                    int fa[3];  // frame indices of the cell
-                    fa[0] = o[0] + cb[0] - 2 + 2;
-                    fa[1] = o[1] + cb[1] - 2 + 2;
-                    fa[2] = o[2] + cb[2] - 2 * dz + 2;
-                    auto Wc = [&](int oi, int oj, int ok) -> const R* {
-                        return Wo + (size_t)((cb[0] + oi) + E2x * ((cb[1] + oj) + E2y * (cb[2] + ok))) * V;
-                    };
-                    if (side == 0) muscl_cell<D, R>(G, fa, d, wdt, Wc, wlo_L, whi_L);
-                    else muscl_cell<D, R>(G, fa, d, wdt, Wc, wlo_R, whi_R);
-                }
-                R uL[V], uR[V], fL[V];
-                conservatives<D>(whi_L, uL, (R)G.gm);
-                conservatives<D>(wlo_R, uR, (R)G.gm);
-                riemann_hllc<D>(fL, uL, uR, d, (R)G.gm);
-                R* F = Fs + (size_t)(fbase[d] + q) * V;
+            for (int side = 0; side < 2; side++) {
+                if (side == 0 ? a[d] == Bd || o[d] + a[d] >= G.N[d] * n : !iface || a[d] == 0) continue;
+                int c[3] = {a[0], a[1], a[2]};
+                c[d] -= side;
+                const long long ge = ((long long)(oe[2] + c[2] / n) * G.N[1] + (oe[1] + c[1] / n)) * G.N[0] + oe[0] + c[0] / n;
+                int p[3] = {c[0] % n, c[1] % n, c[2] % n};
+                p[d] += side;
+                R* F = A.ff[d] + ((long long)A.t * E + ge) * V * NFP + fp_index<n, nf>(d, p);
 #pragma unroll
                 for (int v = 0; v < V; v++) {
-                    R f = F[v];
-                    f = f + tf * (fL[v] - f);
-                    F[v] = f;
+                    const R f = F[v * NFP];
+                    F[v * NFP] = f + tf * (fL[v] - f);
                 }
             }
         }
-        __syncthreads();
     }
-    // corrected sub-cell update
-    R* Ub = Wo;                   // [NE][V][NPT] new U_cv of the tile
-    R* Tmp = Wo + SM::NE * V * NPT;
-    for (int q = threadIdx.x; q < NC; q += blockDim.x) {
-        int a[3] = {q % Bx, (q / Bx) % By, q / (Bx * By)};
-        const int el = (a[0] / n) + TX * ((a[1] / n) + TY * (a[2] / n));
-        int c[3] = {a[0] % n, a[1] % n, a[2] % n};
-        const int pt = pt_index<n>(c);
-        const long long ge = el_ge[el];
-        R hd[3];
-        int fl_[3], fr_[3];
+}
+
+// resident blocks the blend kernel's registers are sized for
+template <typename R, int D>
+constexpr int kBlendBlocksPerSM = sizeof(R) == 4 ? (D == 2 ? 4 : 3) : (D == 2 ? 3 : 2);
+
+template <typename R, int D, int P, int TX, int TY, int TZ>
+__global__ void __launch_bounds__(kThreads, kBlendBlocksPerSM<R, D>) fv_blend_kernel(DevGrid G, DevMatsT<R> M, BlendArgsT<R> A) {
+    pdl_wait();
+    if (gate_closed(G)) return;
+    fv_blend_kernel_body<R, D, P, TX, TY, TZ>(G, M, A, blockIdx.x);
+}
+
+// resident blocks the update kernel's registers are sized for
+template <typename R, int D>
+constexpr int kUpdateBlocksPerSM = sizeof(R) == 4 ? 5 : 4;
+
+// elements of an update block: consecutive ones (no neighbour is read), as
+// many as give every thread a sub-cell
+template <int D, int P>
+struct UpdateBlock {
+    static constexpr int NPT = Shape<D, P>::NPT;
+    static constexpr int NE = kThreads / NPT > 0 ? kThreads / NPT : 1;
+};
+
+template <typename R, int D, int P>
+struct UpdateSmem {
+    static constexpr int n = P + 1, V = D + 2;
+    static constexpr int NPT = Shape<D, P>::NPT;
+    static constexpr int NE = UpdateBlock<D, P>::NE;
+    static constexpr size_t epi = 2 * (size_t)NE * V * NPT;                    // U_cv and sweep scratch
+    static constexpr size_t ind = (size_t)NE * NPT * 16 + NE * 8;               // indicator scratch (bytes)
+    static constexpr size_t epi_bytes = (epi * sizeof(R) + 15) / 16 * 16;       // the indicator's pairs follow
+    static constexpr size_t bytes = epi_bytes + ind;
+};
+
+// ---------------------------------------------------------------------------
+// The corrected sub-cell update of slice t (src/transforms.cpp:483-543 with
+// update=1) from the blended face fluxes, then either the next slice's
+// candidate or, after the last slice, U_sp = cv_to_sp(U_cv), the RK
+// combination, W_cv and the next dt. Blocks of consecutive elements: a
+// sub-cell reads only its own element's state and face fluxes. Bounded by
+// HBM and by the latency of the flux loads.
+// ---------------------------------------------------------------------------
+template <typename R, int D, int P>
+__device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const DevMatsT<R>& M, const FallbackArgsT<R>& A, long long bidx) {
+    using SM = UpdateSmem<R, D, P>;
+    constexpr int n = P + 1, nf = P + 2, V = D + 2, NPT = SM::NPT, NFP = Shape<D, P>::NFP, NE = SM::NE;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    R* Ub = reinterpret_cast<R*>(smem_raw);   // [NE][V][NPT] new U_cv
+    R* Tmp = Ub + NE * V * NPT;
+    __shared__ R Mcs[n * n], Mcv[n * n];  // cv_to_sp, sp_to_cv (lane-dependent rows)
+    if (A.last)
+        for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
+            Mcs[i] = M.cv_to_sp[i];
+            Mcv[i] = M.sp_to_cv[i];
+        }
+    const R dt = (R)(*A.dt);
+    const R wdt = M.wt[A.t] * dt;
+    const long long E = G.E, e0 = bidx * NE;
+    const int ne = (int)(E - e0 < NE ? E - e0 : NE);  // elements of this block
+    for (int q = threadIdx.x; q < ne * NPT; q += blockDim.x) {
+        const int el = q / NPT, pt = q % NPT;
+        const long long ge = e0 + el;
+        int c[3];
+        pt_coords<n>(pt, c);
+        int eg[3];
+        eg[0] = (int)(ge % G.N[0]);
+        eg[1] = (int)((ge / G.N[0]) % G.N[1]);
+        eg[2] = (int)(ge / ((long long)G.N[0] * G.N[1]));
+        Width hd[D];
+        int fl_[D], fr_[D];
 #pragma unroll
         for (int d = 0; d < D; d++) {
-            const long long I = (long long)o[d] + a[d] + 2;
-            hd[d] = (R)(G.fvf[d][I + 1] - G.fvf[d][I]);
-            const int ex = Bx + (d == 0), ey = By + (d == 1);
-            int lo[3] = {a[0], a[1], a[2]}, hi[3] = {a[0], a[1], a[2]};
-            hi[d] += 1;
-            fl_[d] = fbase[d] + lo[0] + ex * (lo[1] + ey * lo[2]);
-            fr_[d] = fbase[d] + hi[0] + ex * (hi[1] + ey * hi[2]);
+            hd[d] = G.fw[d][eg[d] * n + c[d] + 2];
+            int cc[3] = {c[0], c[1], c[2]};
+            fl_[d] = fp_index<n, nf>(d, cc);
+            cc[d] = c[d] + 1;
+            fr_[d] = fp_index<n, nf>(d, cc);
         }
         R un[V];
 #pragma unroll
@@ -808,7 +970,10 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
             const R uold = A.ucv_in[(ge * V + v) * NPT + pt];
             R F = 0;
 #pragma unroll
-            for (int d = 0; d < D; d++) F += (Fs[(size_t)fr_[d] * V + v] - Fs[(size_t)fl_[d] * V + v]) / hd[d];
+            for (int d = 0; d < D; d++) {
+                const R* f = A.ff[d] + (((long long)A.t * E + ge) * V + v) * NFP;
+                F += div_width(G, f[fr_[d]] - f[fl_[d]], hd[d]);
+            }
             if (G.grav && v != 0) {
                 R s;
                 if (v <= D) s = un[0] * (R)G.g[v - 1];
@@ -820,15 +985,15 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
             }
             un[v] = uold - wdt * F;
         }
+        if (A.last) {
 #pragma unroll
-        for (int v = 0; v < V; v++) {
-            A.ucv_out[(ge * V + v) * NPT + pt] = un[v];
-            Ub[(el * V + v) * NPT + pt] = un[v];
-        }
-        if (!A.last) {
+            for (int v = 0; v < V; v++) Ub[(el * V + v) * NPT + pt] = un[v];
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; v++) A.ucv_out[(ge * V + v) * NPT + pt] = un[v];
             // candidate of slice t+1 from the new U_cv
             R uc[V];
-            fv_candidate<D, P, R>(G, ffd, A.t + 1, ge, pt, un, M.wt[A.t + 1] * dt, uc);
+            fv_candidate<D, P, R>(G, A.ff, A.t + 1, ge, pt, un, M.wt[A.t + 1] * dt, uc);
             A.rp_old_next[ge * NPT + pt] = rho_p_fp64<D>(un, G.gm);
             A.rp_new_next[ge * NPT + pt] = rho_p_fp64<D>(uc, G.gm);
         }
@@ -836,19 +1001,20 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
     if (!A.last) return;
     __syncthreads();
     // U_sp = cv_to_sp(U_cv) (src/hydro_ader.hpp:570)
+    double2* RPs = reinterpret_cast<double2*>(reinterpret_cast<unsigned char*>(Ub) + SM::epi_bytes);
     {
         R* bufs[2] = {Tmp, Ub};
         const R* src = Ub;
         for (int d = 0; d < D; d++) {
             R* dst = bufs[d % 2];
-            sweep_smem<D, P, R>(src, dst, M.cv_to_sp, d, SM::NE * V * NPT);
+            sweep_smem<D, P, R>(src, dst, Mcs, d, ne * V * NPT);
             __syncthreads();
             src = dst;
         }
         R* Wsp = (R*)(src == Ub ? Tmp : Ub);
-        for (int q = threadIdx.x; q < SM::NE * NPT; q += blockDim.x) {
+        for (int q = threadIdx.x; q < ne * NPT; q += blockDim.x) {
             const int el = q / NPT, pt = q % NPT;
-            const long long ge = el_ge[el];
+            const long long ge = e0 + el;
             R u[V];
 #pragma unroll
             for (int v = 0; v < V; v++) {
@@ -862,11 +1028,10 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
                 A.u[gi] = val;
             }
             if (A.final_stage && A.feat) {
-                // (rho, p) of the new state for the indicator's features;
-                // the face-flux area is free now
+                // (rho, p) of the new state for the indicator's features
                 double r, pr;
                 feature_rho_p(u, 1, V, G.gm, &r, &pr);
-                reinterpret_cast<double2*>(Fs)[q] = make_double2(r, pr);
+                RPs[q] = make_double2(r, pr);
             }
             if (A.final_stage) {
                 R w[V];
@@ -881,9 +1046,8 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
             // element means summed in point order, then the nodal features
             // rho / mean - 1 and p / mean - 1 as BF16 (the values of the
             // indicator's feature kernels)
-            const double2* RPs = reinterpret_cast<const double2*>(Fs);
-            float2* Mn = reinterpret_cast<float2*>(Fs) + 2 * SM::NE * NPT;
-            for (int el = threadIdx.x; el < SM::NE; el += blockDim.x) {
+            float2* Mn = reinterpret_cast<float2*>(RPs + NE * NPT);
+            for (int el = threadIdx.x; el < ne; el += blockDim.x) {
                 double sr = 0, sp = 0;
                 for (int pt = 0; pt < NPT; pt++) {
                     sr = __dadd_rn(sr, RPs[el * NPT + pt].x);
@@ -891,14 +1055,14 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
                 }
                 const float2 mn = make_float2((float)__ddiv_rn(sr, (double)NPT), (float)__ddiv_rn(sp, (double)NPT));
                 Mn[el] = mn;
-                A.means[el_ge[el]] = mn;
+                A.means[e0 + el] = mn;
             }
             __syncthreads();
-            for (int q = threadIdx.x; q < SM::NE * NPT; q += blockDim.x) {
+            for (int q = threadIdx.x; q < ne * NPT; q += blockDim.x) {
                 const int el = q / NPT, pt = q % NPT;
                 const double2 v = RPs[q];
                 const float2 mn = Mn[el];
-                uint16_t* row = A.feat + el_ge[el] * A.n_in;
+                uint16_t* row = A.feat + (e0 + el) * A.n_in;
                 row[pt] = bf16_bits(feature_ratio(v.x, mn.x));
                 row[NPT + pt] = bf16_bits(feature_ratio(v.y, mn.y));
             }
@@ -907,14 +1071,14 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
         const R* s2 = Wsp;
         for (int d = 0; d < D; d++) {
             R* dst = bufs2[d % 2];
-            sweep_smem<D, P, R>(s2, dst, M.sp_to_cv, d, SM::NE * V * NPT);
+            sweep_smem<D, P, R>(s2, dst, Mcv, d, ne * V * NPT);
             __syncthreads();
             s2 = dst;
         }
         double dtl = 1.7976931348623157e308;
-        for (int q = threadIdx.x; q < SM::NE * NPT; q += blockDim.x) {
+        for (int q = threadIdx.x; q < ne * NPT; q += blockDim.x) {
             const int el = q / NPT, pt = q % NPT;
-            const long long ge = el_ge[el];
+            const long long ge = e0 + el;
             R w[V];
 #pragma unroll
             for (int v = 0; v < V; v++) w[v] = s2[(el * V + v) * NPT + pt];
@@ -927,11 +1091,11 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
     }
 }
 
-template <typename R, int D, int P, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<D, P> + (sizeof(R) == 4 && D == 3 && P > 3 ? 1 : 0)) fv_update_kernel(DevGrid G, DevMatsT<R> M, FallbackArgsT<R> A) {
+template <typename R, int D, int P>
+__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D>) fv_update_kernel(DevGrid G, DevMatsT<R> M, FallbackArgsT<R> A) {
     pdl_wait();
     if (gate_closed(G)) return;
-    fv_update_kernel_body<R, D, P, TX, TY, TZ>(G, M, A, blockIdx.x);
+    fv_update_kernel_body<R, D, P>(G, M, A, blockIdx.x);
 }
 
 }  // namespace spdk

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "spdk.h"
@@ -57,6 +58,19 @@ int dalloc(spdk_hydro* h, void** p, size_t bytes) {
     return 0;
 }
 
+// the distances of consecutive axis positions with their reciprocals
+int upload_widths(spdk_hydro* h, const std::vector<double>& x, Width** out) {
+    std::vector<Width> w(x.size() - 1);
+    for (size_t i = 0; i + 1 < x.size(); i++) {
+        const double d = x[i + 1] - x[i], r = 1.0 / d;
+        w[i] = Width{d, r, std::fma(-d, r, 1.0) * r, 0.0};
+    }
+    if (int rc = dalloc(h, (void**)out, w.size() * sizeof(Width))) return rc;
+    if (cudaMemcpy(*out, w.data(), w.size() * sizeof(Width), cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(SPDK_E_CUDA, "upload widths");
+    return 0;
+}
+
 // open / close an event bracket around one launch when profiling
 void prof_begin(spdk_hydro* h) {
     if (!h->profiling) return;
@@ -99,6 +113,8 @@ template <typename R>
 int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm) {
     const unsigned pblocks = tile_blocks(h->D, h->G.N, k.picard_tile);
     const unsigned blocks = tile_blocks(h->D, h->G.N, k.tile);
+    const unsigned bblocks = tile_blocks(h->D, h->G.N, k.blend_tile);
+    const unsigned ublocks = (unsigned)((h->E + k.update_elems - 1) / k.update_elems);
     const dim3 pthreads(k.picard_threads);
     int launches = 0;
     // viscous face fluxes of a pass's input, written just before the pass
@@ -177,23 +193,27 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
                 SPDK_CUDA(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
                 h->join_pending = false;
             }
+            DetectArgs DA{h->rpo, h->rpn, h->trouble, h->theta, h->elem_any};
             for (int t = 0; t < h->nt; t++) {
                 prof_begin(h);
-                SPDK_CUDA(launch_pdl(k.detect, dim3(blocks), dim3(kThreads), 0, h->stream, h->G,
-                                     (const double2*)h->rpo, (const double2*)h->rpn, h->trouble, (int*)nullptr));
+                SPDK_CUDA(launch_pdl(k.detect, dim3(blocks), dim3(kThreads), 0, h->stream, h->G, DA));
                 prof_end(h, SPDK_KERNEL_DETECT);
+                BlendArgsT<R> B{};
                 FallbackArgsT<R> F{};
+                for (int d = 0; d < 3; d++) B.ff[d] = F.ff[d] = (R*)h->ff[d];
+                B.ucv = ucv[t % 2];
+                B.trouble = h->trouble;
+                B.elem_any = h->elem_any;
+                B.theta = h->theta;
+                B.t = t;
+                B.dt = h->dt;
+                prof_begin(h);
+                SPDK_CUDA(launch_pdl(k.blend, dim3(bblocks), dim3(kThreads), k.blend_smem, h->stream, h->G, dm, B));
+                prof_end(h, SPDK_KERNEL_THETA);
                 F.ucv_in = ucv[t % 2];
                 F.ucv_out = ucv[(t + 1) % 2];
-                F.ff0 = (R*)h->ff[0];
-                F.ff1 = (R*)h->ff[1];
-                F.ff2 = (R*)h->ff[2];
-                F.rp_old = h->rpo;
-                F.rp_new = h->rpn;
                 F.rp_old_next = h->rpo;
                 F.rp_new_next = h->rpn;
-                F.trouble = h->trouble;
-                F.theta = h->theta;
                 F.t = t;
                 F.last = t == h->nt - 1;
                 F.u = (R*)h->u;
@@ -209,9 +229,9 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
                     F.n_in = 2 * h->NPT + 4 * h->D;
                 }
                 prof_begin(h);
-                SPDK_CUDA(launch_pdl(k.update, dim3(blocks), dim3(kThreads), k.update_smem, h->stream, h->G, dm, F));
+                SPDK_CUDA(launch_pdl(k.update, dim3(ublocks), dim3(kThreads), k.update_smem, h->stream, h->G, dm, F));
                 prof_end(h, SPDK_KERNEL_UPDATE);
-                launches += 2;
+                launches += 3;
             }
         }
     }
@@ -315,10 +335,13 @@ int set_attributes(const KernelSetT<R>& ks) {
         // limited by shared memory, not by L1 (staging goes through TMA)
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
-    cudaFuncSetAttribute((const void*)ks.update, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (cudaFuncSetAttribute((const void*)ks.update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)ks.update_smem) != cudaSuccess)
-        return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(ks.update_smem) + " bytes");
+    const std::pair<const void*, size_t> fv[] = {{(const void*)ks.blend, ks.blend_smem},
+                                                 {(const void*)ks.update, ks.update_smem}};
+    for (const auto& f : fv) {
+        cudaFuncSetAttribute(f.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second) != cudaSuccess)
+            return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(f.second) + " bytes");
+    }
     return 0;
 }
 
@@ -328,6 +351,7 @@ void release(spdk_hydro* h) {
     if (h->graph_evolve) cudaGraphExecDestroy(h->graph_evolve);
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     void* ptrs[] = {h->u, h->ua[0], h->ua[1], h->u0, h->ucv[0], h->ucv[1], h->ff[0], h->ff[1], h->ff[2],
+                    h->elem_any, h->fw[0], h->fw[1], h->fw[2], h->fd[0], h->fd[1], h->fd[2],
                     h->wcv, h->dt, h->fvf[0], h->fvf[1], h->fvf[2], h->fvc[0], h->fvc[1], h->fvc[2],
                     h->rpo, h->rpn, h->trouble, h->theta, h->dtmin, h->status, h->elem_trouble, h->elem_pred,
                     h->feat, h->means, h->vg[0], h->vg[1], h->vg[2], h->gate, h->tb, h->stage};
@@ -485,6 +509,7 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
         if (!rc) rc = dalloc(h, (void**)&h->rpn, (size_t)h->E * h->NPT * sizeof(double2));
         if (!rc) rc = dalloc(h, (void**)&h->trouble, (size_t)h->E * h->NPT);
         if (!rc) rc = dalloc(h, (void**)&h->theta, (size_t)h->E * h->NPT);
+        if (!rc) rc = dalloc(h, (void**)&h->elem_any, (size_t)h->E);
         if (!rc) rc = dalloc(h, (void**)&h->elem_trouble, (size_t)h->E);
         if (!rc && cudaMemset(h->elem_trouble, 0, (size_t)h->E) != cudaSuccess) rc = fail(SPDK_E_CUDA, "memset");
         G.elem_trouble = h->elem_trouble;
@@ -499,6 +524,10 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
                 rc = fail(SPDK_E_CUDA, "upload fv_centers");
             G.fvf[d] = h->fvf[d];
             G.fvc[d] = h->fvc[d];
+            if (!rc) rc = upload_widths(h, h->ax[d].fv_faces, &h->fw[d]);
+            if (!rc) rc = upload_widths(h, h->ax[d].fv_centers, &h->fd[d]);
+            G.fw[d] = h->fw[d];
+            G.fd[d] = h->fd[d];
         }
         if (!rc && cudaMemset(h->trouble, 0, (size_t)h->E * h->NPT) != cudaSuccess)
             rc = fail(SPDK_E_CUDA, "memset");
@@ -567,7 +596,7 @@ int spdk_hydro_get_info(const spdk_hydro* h, spdk_hydro_info* info) {
     info->n_dof = h->E * h->NPT;
     info->n_time_slices = h->nt;
     int l = 0;
-    for (int s = 0; s < h->nstages; s++) l += (h->nt - 1) + (h->cfg.fallback ? 1 + 2 * h->nt : 1);
+    for (int s = 0; s < h->nstages; s++) l += (h->nt - 1) + (h->cfg.fallback ? 1 + 3 * h->nt : 1);
     if (h->vg[0]) l += h->nstages * h->nt;  // a viscous pre-pass before every Picard pass
     info->launches_per_step = l + 1 + (h->mlp ? 2 : 0) + (h->elem_trouble ? 1 : 0);
     info->device_bytes = h->bytes;

@@ -39,6 +39,12 @@ struct DevMatsT {
 };
 using DevMats = DevMatsT<double>;
 
+// a width of the sub-cell grid, its reciprocal rounded to nearest, and what
+// that lacks of 1/h (div_const)
+struct __align__(16) Width {
+    double h, ih, ihl, pad;
+};
+
 struct DevGrid {
     int N[3];
     int bc[3];
@@ -54,6 +60,8 @@ struct DevGrid {
     long long E;
     const double* fvf[3];  // FV faces in frame indexing (active cell a has faces a+2, a+3)
     const double* fvc[3];  // FV centres in frame indexing
+    const Width* fw[3];    // widths of the sub-cells (faces i, i+1), frame indexing
+    const Width* fd[3];    // distances of the centres i, i+1
     int* status;           // device-detected faults (kStatus* bits)
     // fallback settings
     double nad_tol;
@@ -262,6 +270,31 @@ __device__ __forceinline__ void sweep_smem(const R* in, R* out, const R* M, int 
     }
 }
 
+// x / h for a step-constant h from its correctly rounded reciprocal y and
+// y's own remainder: q is a faithful quotient, and the exact remainder
+// x - h q times y rounds it correctly (Markstein's theorem for a quotient
+// with a fused multiply-add), for x = 0 or x far from under- and overflow
+__device__ __forceinline__ double div_const(double x, double h, double y, double yl) {
+    const double q = __fma_rn(x, y, __dmul_rn(x, yl));
+    return __fma_rn(__fma_rn(-h, q, x), y, q);
+}
+// whether a flux value's products with the derivative coefficients lie in
+// that range: zero, or an exponent within 700 of 1's
+__device__ __forceinline__ bool div_range(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) & 0x7ff00000u;
+    return (e - ((1023u - 700u) << 20)) < (1400u << 20) || x == 0.0;
+}
+__device__ __forceinline__ bool div_range(float) { return true; }
+
+// x / h for a width of the sub-cell grid: the division's own bits in FP64, a
+// product with the reciprocal in FP32
+__device__ __forceinline__ double div_width(const DevGrid& G, double x, const Width& w) {
+    double q = div_const(x, w.h, w.ih, w.ihl);
+    if (!div_range(x) || !G.safe_div) q = x / w.h;
+    return q;
+}
+__device__ __forceinline__ float div_width(const DevGrid&, float x, const Width& w) { return x * (float)w.ih; }
+
 // Sub-cell candidate of the FV update (src/transforms.cpp:483-543 with
 // update=0): U_new = U_old - (w_t dt) sum_d (F_{+} - F_{-}) / h_d for the
 // cell at point pt of element ge; F from FF_d of slice t.
@@ -276,12 +309,11 @@ __device__ __forceinline__ void fv_candidate(const DevGrid& G, R* const* ff, int
     eg[0] = ge % G.N[0];
     eg[1] = (ge / G.N[0]) % G.N[1];
     eg[2] = ge / ((long long)G.N[0] * G.N[1]);
-    R hd[3];
+    Width hd[D];
     int fl[3], fr[3];
 #pragma unroll
     for (int d = 0; d < D; d++) {
-        const long long I = eg[d] * n + c[d] + 2;
-        hd[d] = (R)(G.fvf[d][I + 1] - G.fvf[d][I]);
+        hd[d] = G.fw[d][eg[d] * n + c[d] + 2];
         int cc[3] = {c[0], c[1], c[2]};
         fl[d] = fp_index<n, nf>(d, cc);
         cc[d] = c[d] + 1;
@@ -293,7 +325,7 @@ __device__ __forceinline__ void fv_candidate(const DevGrid& G, R* const* ff, int
 #pragma unroll
         for (int d = 0; d < D; d++) {
             const R* f = ff[d] + (((long long)t * G.E + ge) * V + v) * S::NFP;
-            F += (f[fr[d]] - f[fl[d]]) / hd[d];
+            F += div_width(G, f[fr[d]] - f[fl[d]], hd[d]);
         }
         if (G.grav) {
             R s = 0;

@@ -137,15 +137,18 @@ struct KernelSetT {
     void (*predict)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*correct)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*flux)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
-    void (*detect)(DevGrid, const double2*, const double2*, uint8_t*, int*) = nullptr;
+    void (*detect)(DevGrid, DetectArgs) = nullptr;
+    void (*blend)(DevGrid, DevMatsT<R>, BlendArgsT<R>) = nullptr;
     void (*update)(DevGrid, DevMatsT<R>, FallbackArgsT<R>) = nullptr;
     void (*init)(DevGrid, DevMatsT<R>, const R*, R*, unsigned long long*) = nullptr;
     void (*derive)(DevGrid, DevMatsT<R>, const R*, R*, unsigned long long*) = nullptr;
     void (*visc)(DevGrid, DevMatsT<R>, ViscArgsT<R>) = nullptr;
-    size_t picard_smem[3] = {0, 0, 0}, update_smem = 0;  // predict, correct, flux
+    size_t picard_smem[3] = {0, 0, 0}, blend_smem = 0, update_smem = 0;  // predict, correct, flux
     int picard_threads = kThreads;
     int picard_tile[3] = {1, 1, 1};  // elements of a Picard pass's block (2D: may hang over the domain's edge)
-    int tile[3] = {1, 1, 1};         // elements of a detect / update block
+    int tile[3] = {1, 1, 1};         // elements of a detect block
+    int blend_tile[3] = {1, 1, 1};   // elements of a blend block
+    int update_elems = 1;            // consecutive elements of an update block
     int visc_epb = 1;  // elements per block of the viscous face kernel
 };
 using KernelSet = KernelSetT<double>;
@@ -162,7 +165,14 @@ KernelSetT<R> make_set() {
     k.picard_tile[1] = PY;
     k.picard_tile[2] = TZ;
     k.detect = fv_detect_kernel<R, D, P, TX, TY, TZ>;
-    k.update = fv_update_kernel<R, D, P, TX, TY, TZ>;
+    using BT = BlendTile<D, P>;
+    k.blend = fv_blend_kernel<R, D, P, BT::X, BT::Y, BT::Z>;
+    k.blend_smem = BlendSmem<R, D, P, BT::X, BT::Y, BT::Z>::bytes;
+    k.blend_tile[0] = BT::X;
+    k.blend_tile[1] = BT::Y;
+    k.blend_tile[2] = BT::Z;
+    k.update = fv_update_kernel<R, D, P>;
+    k.update_elems = UpdateBlock<D, P>::NE;
     k.init = init_state_kernel<R, D, P>;
     k.derive = derive_kernel<R, D, P>;
     k.visc = visc_face_kernel<R, D, P>;
@@ -170,7 +180,7 @@ KernelSetT<R> make_set() {
     k.picard_smem[kPredict] = picard_smem_bytes<R, D, P, PX, PY, TZ, kPredict>();
     k.picard_smem[kCorrect] = picard_smem_bytes<R, D, P, PX, PY, TZ, kCorrect>();
     k.picard_smem[kFlux] = picard_smem_bytes<R, D, P, PX, PY, TZ, kFlux>();
-    k.update_smem = UpdateSmem<R, D, P, TX, TY, TZ>::bytes;
+    k.update_smem = UpdateSmem<R, D, P>::bytes;
     k.tile[0] = TX;
     k.tile[1] = TY;
     k.tile[2] = TZ;
@@ -207,20 +217,17 @@ inline void set_spacing(DevGrid& G, int D, const double h[3], const double* dfp_
     }
 }
 
-// Tile choice: the largest instantiated tile that divides the element counts.
-// Viscous runs (VISC) take the same tiles with the viscous Picard passes.
+// 2D: the detect tile (its blocks may hang over the domain) is 4 x 4 elements
+// up to p = 4 and 2 x 2 above, whatever the element counts
 template <typename R, int P, bool VISC>
-bool pick2_t(int Nx, int Ny, KernelSetT<R>* k) {
-    if constexpr (P <= 4) {
-        if (Nx % 4 == 0 && Ny % 4 == 0) { *k = make_set<R, 2, P, 4, 4, 1, VISC>(); return true; }
-    }
-    if (Nx % 2 == 0 && Ny % 2 == 0) { *k = make_set<R, 2, P, 2, 2, 1, VISC>(); return true; }
-    *k = make_set<R, 2, P, 1, 1, 1, VISC>();
+bool pick2_t(KernelSetT<R>* k) {
+    constexpr int T = P <= 4 ? 4 : 2;
+    *k = make_set<R, 2, P, T, T, 1, VISC>();
     return true;
 }
 template <typename R, int P>
-bool pick2(int Nx, int Ny, KernelSetT<R>* k, bool visc) {
-    return visc ? pick2_t<R, P, true>(Nx, Ny, k) : pick2_t<R, P, false>(Nx, Ny, k);
+bool pick2(KernelSetT<R>* k, bool visc) {
+    return visc ? pick2_t<R, P, true>(k) : pick2_t<R, P, false>(k);
 }
 // 3D: one element per tile, or 2x1x1 elements at p <= 3, where one
 // element's (p+1)^3 points would leave most of the block idle in the

@@ -142,13 +142,14 @@ __device__ __forceinline__ void riemann_hllc(R* F, const R* UL, const R* UR, int
     F[D + 1] = v * (e + pg);
 }
 
-// src/muscl.hpp:2-12
-template <typename R> __device__ __forceinline__ R minmod(R SL, R SR, R xL, R xR) {
+// src/muscl.hpp:2-12, h = xR - xL the cell's width
+template <typename R> __device__ __forceinline__ R minmod(R SL, R SR, R h) {
     R ratio = SR / SL;
     ratio = smax(R(0.0), smin(ratio, R(1.0)));
     R slope = ratio * SL;
-    return R(0.5) * slope * (xR - xL);
+    return R(0.5) * slope * h;
 }
+template <typename R> __device__ __forceinline__ R minmod(R SL, R SR, R xL, R xR) { return minmod(SL, SR, xR - xL); }
 
 // src/hydro.cpp:591-615: Hancock time derivative of the primitives from the
 // limited slopes dW[d][*] of every active direction (terms of inactive

@@ -222,22 +222,6 @@ __device__ __forceinline__ void interface2(const DevGrid& G, R (&uL)[4], R (&uR)
     }
 }
 
-// x / h for a step-constant h from its correctly rounded reciprocal y and
-// y's own remainder: q is a faithful quotient, and the exact remainder
-// x - h q times y rounds it correctly (Markstein's theorem for a quotient
-// with a fused multiply-add), for x = 0 or x far from under- and overflow
-__device__ __forceinline__ double div_const(double x, double h, double y, double yl) {
-    const double q = __fma_rn(x, y, __dmul_rn(x, yl));
-    return __fma_rn(__fma_rn(-h, q, x), y, q);
-}
-// whether a flux value's products with the derivative coefficients lie in
-// that range: zero, or an exponent within 700 of 1's
-__device__ __forceinline__ bool div_range(double x) {
-    const unsigned e = (unsigned)__double2hiint(x) & 0x7ff00000u;
-    return (e - ((1023u - 700u) << 20)) < (1400u << 20) || x == 0.0;
-}
-__device__ __forceinline__ bool div_range(float) { return true; }
-
 template <typename R, int P, int TX, int TY, int MODE, bool VISC>
 __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R>& M, const PicardArgsT<R>& A,
                                               long long bidx) {
