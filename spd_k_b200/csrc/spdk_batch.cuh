@@ -21,14 +21,14 @@ struct BatchItem {
     long long first;  // first block of this problem in the launch
 };
 
-// the item of this block, copied to shared memory (all threads return it)
+// the item of block `block`, copied to shared memory (all threads return it)
 template <typename Item>
-__device__ __forceinline__ const Item& batch_item(const Item* __restrict__ items, int n, long long* local) {
+__device__ __forceinline__ const Item& batch_item(const Item* __restrict__ items, int n, long long* local, long long block) {
     __shared__ __align__(16) unsigned char raw[sizeof(Item)];
     __shared__ int q;
     if (threadIdx.x == 0) {
         int lo = 0, hi = n - 1;
-        const long long b = blockIdx.x;
+        const long long b = block;
         while (lo < hi) {
             const int mid = (lo + hi + 1) / 2;
             if (items[mid].first <= b) lo = mid;
@@ -43,7 +43,7 @@ __device__ __forceinline__ const Item& batch_item(const Item* __restrict__ items
     for (int w = threadIdx.x; w < (int)(sizeof(Item) / 4); w += blockDim.x) dst[w] = src[w];
     __syncthreads();
     const Item& it = *reinterpret_cast<const Item*>(raw);
-    *local = (long long)blockIdx.x - it.first;
+    *local = block - it.first;
     return it;
 }
 
@@ -51,7 +51,7 @@ template <typename R, int D, int P, int TX, int TY, int TZ, int MODE>
 __global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_blocks<R, D, P, TX, TY, TZ, MODE>())
     picard_batched(const BatchItem<PicardArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
     long long b;
-    const BatchItem<PicardArgsT<R>>& it = batch_item(items, n, &b);
+    const BatchItem<PicardArgsT<R>>& it = batch_item(items, n, &b, blockIdx.x);
     if constexpr (D == 2) picard2d_body<R, P, TX, TY, MODE, false>(it.G, M, it.A, b);
     else picard_kernel_body<R, D, P, TX, TY, TZ, MODE>(it.G, M, it.A, b);
 }
@@ -65,23 +65,31 @@ constexpr int kDetectBlocksPerSMBatched = D == 2 ? 5 : kDetectBlocksPerSM<D>;
 template <typename R, int D, int P, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(kThreads, kDetectBlocksPerSMBatched<D>) detect_batched(const BatchItem<DetectArgs>* __restrict__ items, int n) {
     long long b;
-    const BatchItem<DetectArgs>& it = batch_item(items, n, &b);
+    const BatchItem<DetectArgs>& it = batch_item(items, n, &b, blockIdx.x);
     fv_detect_kernel_body<R, D, P, TX, TY, TZ>(it.G, it.A, b);
 }
 
+// the tiles of all members that the detection listed, shared out among the blocks
 template <typename R, int D, int P, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(kThreads, kBlendBlocksPerSM<R, D>)
     blend_batched(const BatchItem<BlendArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
-    long long b;
-    const BatchItem<BlendArgsT<R>>& it = batch_item(items, n, &b);
-    fv_blend_kernel_body<R, D, P, TX, TY, TZ>(it.G, M, it.A, b);
+    const BlendList list = items[0].A.list;
+    const int count = *list.count;
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        const int tile = list.tiles[i];
+        long long b;
+        const BatchItem<BlendArgsT<R>>& it = batch_item(items, n, &b, tile);
+        fv_blend_kernel_body<R, D, P, TX, TY, TZ>(it.G, M, it.A, b);
+        __syncthreads();  // the next tile reuses the shared memory
+        if (threadIdx.x == 0) list.mark[tile] = 0;
+    }
 }
 
 template <typename R, int D, int P>
 __global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D>)
     update_batched(const BatchItem<FallbackArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
     long long b;
-    const BatchItem<FallbackArgsT<R>>& it = batch_item(items, n, &b);
+    const BatchItem<FallbackArgsT<R>>& it = batch_item(items, n, &b, blockIdx.x);
     fv_update_kernel_body<R, D, P>(it.G, M, it.A, b);
 }
 

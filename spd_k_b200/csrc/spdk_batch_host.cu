@@ -50,6 +50,7 @@ struct Group {
     BatchSetT<double> k64;
     BatchSetT<float> k32;
     std::vector<Pass> passes;
+    int* blend = nullptr;  // the members' blend tiles: marks, list, count
     cudaStream_t st = nullptr;
     cudaEvent_t join = nullptr;
 };
@@ -80,6 +81,8 @@ namespace {
 void free_tables(Group& g) {
     for (Pass& p : g.passes) cudaFree(p.items);
     g.passes.clear();
+    if (g.blend) cudaFree(g.blend);
+    g.blend = nullptr;
 }
 
 template <typename Item>
@@ -179,6 +182,8 @@ int plan_group(spdk_batch* b, Group& g) {
         }
         if ((rc = upload_pass(g, kPassFlux, pblocks, items))) return rc;
     }
+    BCUDA(cudaMalloc((void**)&g.blend, (2 * btotal + 1) * sizeof(int)));
+    BCUDA(cudaMemset(g.blend, 0, (2 * btotal + 1) * sizeof(int)));
     for (int t = 0; t < nt && !rc; t++) {
         std::vector<BatchItem<DetectArgs>> det(n);
         std::vector<BatchItem<BlendArgsT<R>>> bl(n);
@@ -189,21 +194,24 @@ int plan_group(spdk_batch* b, Group& g) {
             det[q].G = bq.G;
             if (b->labels) det[q].G.elem_trouble = h->elem_trouble;
             det[q].first = first[q];
-            det[q].A = DetectArgs{h->rpo, h->rpn, h->trouble, h->theta, h->elem_any};
+            BlendList list{g.blend + bfirst[q], g.blend + btotal, g.blend + 2 * btotal, (int)bfirst[q]};
+            det[q].A = DetectArgs{h->rpo, h->rpn, h->trouble, h->theta, list};
             bl[q].G = bq.G;
             bl[q].first = bfirst[q];
             BlendArgsT<R>& B = bl[q].A;
             B = BlendArgsT<R>{};
+            FallbackArgsT<R>& F = up[q].A;
+            F = FallbackArgsT<R>{};
             B.ucv = (R*)h->ucv[t % 2];
             B.trouble = h->trouble;
-            B.elem_any = h->elem_any;
+            B.list = list;
+            if (q == 0) B.list.mark = g.blend;
+            F.blend_count = list.count;
             B.theta = h->theta;
             B.t = t;
             B.dt = h->dt;
             up[q].G = bq.G;
             up[q].first = ufirst[q];
-            FallbackArgsT<R>& F = up[q].A;
-            F = FallbackArgsT<R>{};
             F.ucv_in = (R*)h->ucv[t % 2];
             F.ucv_out = (R*)h->ucv[(t + 1) % 2];
             for (int d = 0; d < 3; d++) B.ff[d] = F.ff[d] = (R*)h->ff[d];
@@ -220,7 +228,7 @@ int plan_group(spdk_batch* b, Group& g) {
             F.dt = h->dt;
         }
         rc = upload_pass(g, kPassDetect, blocks, det);
-        if (!rc) rc = upload_pass(g, kPassBlend, (unsigned)btotal, bl);
+        if (!rc) rc = upload_pass(g, kPassBlend, (unsigned)std::min<long long>(btotal, kBlendGrid), bl);
         if (!rc) rc = upload_pass(g, kPassUpdate, (unsigned)utotal, up);
     }
     return rc;

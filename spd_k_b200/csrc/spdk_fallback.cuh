@@ -14,6 +14,15 @@
 
 namespace spdk {
 
+// The blend tiles that have trouble within three cells, collected by the
+// detection and emptied again by the blend (marks) and the update (count)
+struct BlendList {
+    int* mark;   // [tile] 1: listed
+    int* tiles;  // block numbers of the listed tiles
+    int* count;
+    int first;   // block number of tile 0 (a batch lists its members' tiles together)
+};
+
 // Blended fluxes of one slice (blend kernel): the SD face fluxes of the faces
 // that the troubles reach are replaced in place
 template <typename R>
@@ -21,8 +30,8 @@ struct BlendArgsT {
     const R* ucv;             // U_cv at the start of slice t [E][V][NPT]
     R* ff[3];                 // FV face fluxes of each direction, all slices
     const uint8_t* trouble;   // [E][NPT]
-    const uint8_t* elem_any;  // [E]: any troubled sub-cell in the element
     uint8_t* theta;           // [E][NPT], theta * 8 (zero on entry where no trouble is near)
+    BlendList list;           // tiles with trouble near
     int t;                    // slice
     const double* dt;
 };
@@ -43,6 +52,7 @@ struct FallbackArgsT {
     R* wcv;
     unsigned long long* dtmin;
     const double* dt;
+    int* blend_count;       // emptied for the next slice's detection
     // learned indicator (nullable): after the final stage, the element means
     // of (rho, p) and the nodal part of each feature row (row length n_in)
     // of the new state, for the next step's a-priori flags
@@ -57,7 +67,7 @@ struct DetectArgs {
     const double2* rpn;
     uint8_t* T;          // troubles
     uint8_t* theta;      // cleared for the blend kernel
-    uint8_t* elem_any;   // [E]: any troubled sub-cell
+    BlendList list;      // blend tiles the troubles reach
 };
 
 template <int D, int P>
@@ -147,6 +157,16 @@ __device__ __forceinline__ bool has_image(const DevGrid& G, const int a[3], int 
 }
 
 __device__ __forceinline__ double rp_var(const double2 v, int k) { return k == 0 ? v.x : v.y; }
+
+// elements of a blend block: 64 to 150 sub-cells, so that nearly every one of
+// the block's phases takes its 256 threads one round: a tile's time is a
+// chain of their latencies (4 x 4 elements at p = 3 took twice as long)
+template <int D, int P>
+struct BlendTile {
+    static constexpr int X = D == 2 ? (P <= 3 ? 4 : 2) : (P <= 3 ? 2 : 1);
+    static constexpr int Y = D == 2 ? (P <= 2 ? 4 : (P <= 5 ? 2 : 1)) : 1;
+    static constexpr int Z = 1;
+};
 
 // ---------------------------------------------------------------------------
 // Trouble detection of every active sub-cell (src/trouble_detection.cpp:35-290
@@ -534,10 +554,28 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const De
         if (tr) el_any[q / NPT] = 1;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < NE; e += blockDim.x) {
-        const int g0 = o[0] / n + e % TX, g1 = o[1] / n + (e / TX) % TY, g2 = o[2] / n + e / (TX * TY);
-        if (g0 < G.N[0] && g1 < G.N[1] && (D == 2 || g2 < G.N[2]))
-            A.elem_any[((long long)g2 * G.N[1] + g1) * G.N[0] + g0] = (uint8_t)el_any[e];
+    // list the blend tiles within three cells (K elements) of a troubled element
+    using BT = BlendTile<D, P>;
+    constexpr int K = (3 + n - 1) / n;
+    constexpr int Rx = 2 * K + 1, Ry = Rx, Rz = D == 3 ? Rx : 1;
+    const int nbx = (G.N[0] + BT::X - 1) / BT::X, nby = (G.N[1] + BT::Y - 1) / BT::Y;
+    for (int w = threadIdx.x; w < NE * Rx * Ry * Rz; w += blockDim.x) {
+        const int e = w / (Rx * Ry * Rz), r = w % (Rx * Ry * Rz);
+        if (!el_any[e]) continue;
+        int g[3] = {o[0] / n + e % TX + r % Rx - K, o[1] / n + (e / TX) % TY + (r / Rx) % Ry - K,
+                    D == 3 ? o[2] / n + e / (TX * TY) + r / (Rx * Ry) - K : 0};
+        bool in = true;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            if (g[d] >= 0 && g[d] < G.N[d]) continue;
+            // ghosts of a non-periodic edge are images of the edge's own cells
+            if (G.bc[d] != kPeriodic) in = false;
+            else g[d] = (g[d] + K * G.N[d]) % G.N[d];
+        }
+        if (!in) continue;
+        const int tile = g[0] / BT::X + nbx * (g[1] / BT::Y + nby * (g[2] / BT::Z));
+        if (!*(volatile int*)&A.list.mark[tile] && atomicExch(&A.list.mark[tile], 1) == 0)
+            A.list.tiles[atomicAdd(A.list.count, 1)] = A.list.first + tile;
     }
 }
 
@@ -676,24 +714,14 @@ __device__ __forceinline__ void muscl_slopes(const DevGrid& G, const int fa[3], 
 // (src/hydro.cpp:683-788) written over the SD face fluxes, each element's own
 // copy of an interface.
 //
-// A tile without trouble within three cells returns after looking at the
-// flags of the elements around it. On the others W_old is formed once on the
-// tile + 2 halo, the slopes of a cell once for all its faces (they were formed
+// The launch's blocks share out the tiles that the detection listed (those
+// with trouble within three cells). W_old is formed once on the tile + 2 halo, the slopes of a cell once for all its faces (they were formed
 // by every face for both of its cells: 4 times a cell in 2D, 6 in 3D, with
 // the divisions that dominate them in FP64), and each face takes one HLLC
 // solve. Bounded by the latency of its chain of phases: it is separate from
 // the update, whose blocks would otherwise all reserve the shared memory and
 // wait for the few that blend.
 // ---------------------------------------------------------------------------
-// elements of a blend block: 4 x 4 up to p = 3 and 2 x 2 above in 2D, 2 x 1 x 1
-// up to p = 3 and one above in 3D
-template <int D, int P>
-struct BlendTile {
-    static constexpr int X = D == 2 ? (P <= 3 ? 4 : 2) : (P <= 3 ? 2 : 1);
-    static constexpr int Y = D == 2 ? (P <= 3 ? 4 : 2) : 1;
-    static constexpr int Z = 1;
-};
-
 template <typename R, int D, int P, int TX, int TY, int TZ>
 struct BlendSmem {
     static constexpr int n = P + 1, V = D + 2;
@@ -752,25 +780,6 @@ __device__ __forceinline__ void fv_blend_kernel_body(const DevGrid& G, const Dev
         o[0] = oe[0] * n;
         o[1] = oe[1] * n;
         o[2] = oe[2] * n;
-    }
-    // any trouble within three cells: the elements they lie in
-    {
-        constexpr int K = (3 + n - 1) / n;
-        constexpr int Mx = TX + 2 * K, My = TY + 2 * K, Mz = D == 3 ? TZ + 2 * K : 1;
-        int any = 0;
-        for (int q = threadIdx.x; q < Mx * My * Mz; q += blockDim.x) {
-            int g[3] = {oe[0] - K + q % Mx, oe[1] - K + (q / Mx) % My, D == 3 ? oe[2] - K + q / (Mx * My) : 0};
-            bool in = true;
-#pragma unroll
-            for (int d = 0; d < D; d++) {
-                if (g[d] >= 0 && g[d] < G.N[d]) continue;
-                // ghosts of a non-periodic edge are images of the tile's own cells
-                if (G.bc[d] != kPeriodic) in = false;
-                else g[d] = (g[d] + K * G.N[d]) % G.N[d];
-            }
-            if (in) any |= A.elem_any[((long long)g[2] * G.N[1] + g[1]) * G.N[0] + g[0]];
-        }
-        if (!__syncthreads_or(any)) return;
     }
     extern __shared__ __align__(128) unsigned char smem_raw[];
     R* SL = reinterpret_cast<R*>(smem_raw);  // slopes and dW/dt on the tile + 1 halo
@@ -894,7 +903,13 @@ template <typename R, int D, int P, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(kThreads, kBlendBlocksPerSM<R, D>) fv_blend_kernel(DevGrid G, DevMatsT<R> M, BlendArgsT<R> A) {
     pdl_wait();
     if (gate_closed(G)) return;
-    fv_blend_kernel_body<R, D, P, TX, TY, TZ>(G, M, A, blockIdx.x);
+    const int count = *A.list.count;
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        const int tile = A.list.tiles[i];
+        fv_blend_kernel_body<R, D, P, TX, TY, TZ>(G, M, A, tile);
+        __syncthreads();  // the next tile reuses the shared memory
+        if (threadIdx.x == 0) A.list.mark[tile] = 0;
+    }
 }
 
 // resident blocks the update kernel's registers are sized for
@@ -914,10 +929,19 @@ struct UpdateSmem {
     static constexpr int n = P + 1, V = D + 2;
     static constexpr int NPT = Shape<D, P>::NPT;
     static constexpr int NE = UpdateBlock<D, P>::NE;
-    static constexpr size_t epi = 2 * (size_t)NE * V * NPT;                    // U_cv and sweep scratch
+    static constexpr int NFP = Shape<D, P>::NFP;
+    // the block's inputs arrive as bulk copies (its elements are consecutive
+    // in every array) where an element's blocks are whole 16-byte units
+    static constexpr bool bulk = (V * NFP * sizeof(R)) % 16 == 0 && (V * NPT * sizeof(R)) % 16 == 0;
+    static constexpr size_t faces = (size_t)D * NE * V * NFP;                  // face fluxes of one slice
+    static constexpr size_t ucv = (size_t)NE * V * NPT;
+    static constexpr size_t epi = 2 * ucv;                                     // U_cv and sweep scratch
     static constexpr size_t ind = (size_t)NE * NPT * 16 + NE * 8;               // indicator scratch (bytes)
+    static constexpr size_t in0 = bulk ? (ucv + faces) * sizeof(R) : 0;         // slice t
+    static constexpr size_t in1 = bulk ? faces * sizeof(R) : 0;                 // slice t + 1, else the epilogue's
     static constexpr size_t epi_bytes = (epi * sizeof(R) + 15) / 16 * 16;       // the indicator's pairs follow
-    static constexpr size_t bytes = epi_bytes + ind;
+    static constexpr size_t out = epi_bytes + ind;
+    static constexpr size_t bytes = in0 + (in1 > out ? in1 : out);
 };
 
 // ---------------------------------------------------------------------------
@@ -926,16 +950,40 @@ struct UpdateSmem {
 // candidate or, after the last slice, U_sp = cv_to_sp(U_cv), the RK
 // combination, W_cv and the next dt. Blocks of consecutive elements: a
 // sub-cell reads only its own element's state and face fluxes. Bounded by
-// HBM and by the latency of the flux loads.
+// HBM: the inputs of a block (its U_cv, and the face fluxes of slices t and
+// t + 1) are contiguous, so one thread fetches them as a handful of bulk
+// copies instead of every thread waiting for its own 36 gathers.
 // ---------------------------------------------------------------------------
 template <typename R, int D, int P>
 __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const DevMatsT<R>& M, const FallbackArgsT<R>& A, long long bidx) {
     using SM = UpdateSmem<R, D, P>;
     constexpr int n = P + 1, nf = P + 2, V = D + 2, NPT = SM::NPT, NFP = Shape<D, P>::NFP, NE = SM::NE;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    R* Ub = reinterpret_cast<R*>(smem_raw);   // [NE][V][NPT] new U_cv
-    R* Tmp = Ub + NE * V * NPT;
+    R* Uin = reinterpret_cast<R*>(smem_raw);                   // [NE][V][NPT] U_cv of slice t
+    R* F0 = Uin + SM::ucv;                                      // [D][NE][V][NFP] face fluxes of slice t
+    R* F1 = reinterpret_cast<R*>(smem_raw + SM::in0);           // ... of slice t + 1
+    R* Ub = F1;                                                 // last slice: [NE][V][NPT] new U_cv
+    R* Tmp = Ub + SM::ucv;
     __shared__ R Mcs[n * n], Mcv[n * n];  // cv_to_sp, sp_to_cv (lane-dependent rows)
+    __shared__ uint64_t bar;
+    if (bidx == 0 && threadIdx.x == 0) *A.blend_count = 0;
+    const long long E = G.E, e0 = bidx * NE;
+    const int ne = (int)(E - e0 < NE ? E - e0 : NE);  // elements of this block
+    if constexpr (SM::bulk) {
+        if (threadIdx.x == 0) {
+            mbar_init(&bar, 1);
+            mbar_fence_init();
+            const uint32_t ub = (uint32_t)(ne * V * NPT * sizeof(R)), fb = (uint32_t)(ne * V * NFP * sizeof(R));
+            mbar_expect_tx(&bar, ub + D * fb * (A.last ? 1 : 2));
+            bulk_g2s(Uin, A.ucv_in + e0 * V * NPT, ub, &bar);
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+                const R* src = A.ff[d] + ((long long)A.t * E + e0) * V * NFP;
+                bulk_g2s(F0 + d * NE * V * NFP, src, fb, &bar);
+                if (!A.last) bulk_g2s(F1 + d * NE * V * NFP, src + E * V * NFP, fb, &bar);
+            }
+        }
+    }
     if (A.last)
         for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
             Mcs[i] = M.cv_to_sp[i];
@@ -943,19 +991,33 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
         }
     const R dt = (R)(*A.dt);
     const R wdt = M.wt[A.t] * dt;
-    const long long E = G.E, e0 = bidx * NE;
-    const int ne = (int)(E - e0 < NE ? E - e0 : NE);  // elements of this block
+    if constexpr (SM::bulk) {
+        __syncthreads();  // the barrier is initialised
+        mbar_wait_bounded(&bar, 0, G.status);
+    }
     for (int q = threadIdx.x; q < ne * NPT; q += blockDim.x) {
         const int el = q / NPT, pt = q % NPT;
         const long long ge = e0 + el;
-        int c[3];
+        int c[3], eg[3];
         pt_coords<n>(pt, c);
-        int eg[3];
-        eg[0] = (int)(ge % G.N[0]);
-        eg[1] = (int)((ge / G.N[0]) % G.N[1]);
-        eg[2] = (int)(ge / ((long long)G.N[0] * G.N[1]));
+        elem_pos(G, (int)ge, eg);
         Width hd[D];
         int fl_[D], fr_[D];
+        const R* f0[D];
+        const R* f1[D];
+        const R* u0;
+        if constexpr (SM::bulk) {
+            u0 = Uin + el * V * NPT + pt;
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+                f0[d] = F0 + (d * NE + el) * V * NFP;
+                f1[d] = F1 + (d * NE + el) * V * NFP;
+            }
+        } else {
+            u0 = A.ucv_in + ge * V * NPT + pt;
+            face_blocks<D, P, R>(G, A.ff, A.t, (int)ge, f0);
+            face_blocks<D, P, R>(G, A.ff, A.last ? A.t : A.t + 1, (int)ge, f1);
+        }
 #pragma unroll
         for (int d = 0; d < D; d++) {
             hd[d] = G.fw[d][eg[d] * n + c[d] + 2];
@@ -967,13 +1029,9 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
         R un[V];
 #pragma unroll
         for (int v = 0; v < V; v++) {
-            const R uold = A.ucv_in[(ge * V + v) * NPT + pt];
             R F = 0;
 #pragma unroll
-            for (int d = 0; d < D; d++) {
-                const R* f = A.ff[d] + (((long long)A.t * E + ge) * V + v) * NFP;
-                F += div_width(G, f[fr_[d]] - f[fl_[d]], hd[d]);
-            }
+            for (int d = 0; d < D; d++) F += div_width(G, f0[d][v * NFP + fr_[d]] - f0[d][v * NFP + fl_[d]], hd[d]);
             if (G.grav && v != 0) {
                 R s;
                 if (v <= D) s = un[0] * (R)G.g[v - 1];
@@ -983,7 +1041,7 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
                 }
                 F -= s;
             }
-            un[v] = uold - wdt * F;
+            un[v] = u0[v * NPT] - wdt * F;
         }
         if (A.last) {
 #pragma unroll
@@ -993,7 +1051,7 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
             for (int v = 0; v < V; v++) A.ucv_out[(ge * V + v) * NPT + pt] = un[v];
             // candidate of slice t+1 from the new U_cv
             R uc[V];
-            fv_candidate<D, P, R>(G, A.ff, A.t + 1, ge, pt, un, M.wt[A.t + 1] * dt, uc);
+            fv_candidate<D, P, R>(G, f1, eg, pt, un, M.wt[A.t + 1] * dt, uc);
             A.rp_old_next[ge * NPT + pt] = rho_p_fp64<D>(un, G.gm);
             A.rp_new_next[ge * NPT + pt] = rho_p_fp64<D>(uc, G.gm);
         }

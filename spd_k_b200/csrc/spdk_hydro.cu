@@ -113,7 +113,8 @@ template <typename R>
 int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm) {
     const unsigned pblocks = tile_blocks(h->D, h->G.N, k.picard_tile);
     const unsigned blocks = tile_blocks(h->D, h->G.N, k.tile);
-    const unsigned bblocks = tile_blocks(h->D, h->G.N, k.blend_tile);
+    // the blend's blocks share out the listed tiles
+    const unsigned bblocks = std::min(tile_blocks(h->D, h->G.N, k.blend_tile), kBlendGrid);
     const unsigned ublocks = (unsigned)((h->E + k.update_elems - 1) / k.update_elems);
     const dim3 pthreads(k.picard_threads);
     int launches = 0;
@@ -193,7 +194,8 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
                 SPDK_CUDA(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
                 h->join_pending = false;
             }
-            DetectArgs DA{h->rpo, h->rpn, h->trouble, h->theta, h->elem_any};
+            const BlendList list{h->blend_mark, h->blend_tiles, h->blend_count, 0};
+            DetectArgs DA{h->rpo, h->rpn, h->trouble, h->theta, list};
             for (int t = 0; t < h->nt; t++) {
                 prof_begin(h);
                 SPDK_CUDA(launch_pdl(k.detect, dim3(blocks), dim3(kThreads), 0, h->stream, h->G, DA));
@@ -203,7 +205,8 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
                 for (int d = 0; d < 3; d++) B.ff[d] = F.ff[d] = (R*)h->ff[d];
                 B.ucv = ucv[t % 2];
                 B.trouble = h->trouble;
-                B.elem_any = h->elem_any;
+                B.list = list;
+                F.blend_count = h->blend_count;
                 B.theta = h->theta;
                 B.t = t;
                 B.dt = h->dt;
@@ -351,7 +354,7 @@ void release(spdk_hydro* h) {
     if (h->graph_evolve) cudaGraphExecDestroy(h->graph_evolve);
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     void* ptrs[] = {h->u, h->ua[0], h->ua[1], h->u0, h->ucv[0], h->ucv[1], h->ff[0], h->ff[1], h->ff[2],
-                    h->elem_any, h->fw[0], h->fw[1], h->fw[2], h->fd[0], h->fd[1], h->fd[2],
+                    h->blend_mark, h->blend_tiles, h->blend_count, h->fw[0], h->fw[1], h->fw[2], h->fd[0], h->fd[1], h->fd[2],
                     h->wcv, h->dt, h->fvf[0], h->fvf[1], h->fvf[2], h->fvc[0], h->fvc[1], h->fvc[2],
                     h->rpo, h->rpn, h->trouble, h->theta, h->dtmin, h->status, h->elem_trouble, h->elem_pred,
                     h->feat, h->means, h->vg[0], h->vg[1], h->vg[2], h->gate, h->tb, h->stage};
@@ -509,7 +512,13 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
         if (!rc) rc = dalloc(h, (void**)&h->rpn, (size_t)h->E * h->NPT * sizeof(double2));
         if (!rc) rc = dalloc(h, (void**)&h->trouble, (size_t)h->E * h->NPT);
         if (!rc) rc = dalloc(h, (void**)&h->theta, (size_t)h->E * h->NPT);
-        if (!rc) rc = dalloc(h, (void**)&h->elem_any, (size_t)h->E);
+        const size_t tiles = tile_blocks(D, G.N, h->prec == SPDK_PRECISION_FP32 ? h->ks32.blend_tile : h->ks64.blend_tile);
+        if (!rc) rc = dalloc(h, (void**)&h->blend_mark, tiles * sizeof(int));
+        if (!rc) rc = dalloc(h, (void**)&h->blend_tiles, tiles * sizeof(int));
+        if (!rc) rc = dalloc(h, (void**)&h->blend_count, sizeof(int));
+        if (!rc && (cudaMemset(h->blend_mark, 0, tiles * sizeof(int)) != cudaSuccess ||
+                    cudaMemset(h->blend_count, 0, sizeof(int)) != cudaSuccess))
+            rc = fail(SPDK_E_CUDA, "memset");
         if (!rc) rc = dalloc(h, (void**)&h->elem_trouble, (size_t)h->E);
         if (!rc && cudaMemset(h->elem_trouble, 0, (size_t)h->E) != cudaSuccess) rc = fail(SPDK_E_CUDA, "memset");
         G.elem_trouble = h->elem_trouble;

@@ -38,7 +38,7 @@ struct spdk_hydro {
     double *fvf[3] = {nullptr, nullptr, nullptr}, *fvc[3] = {nullptr, nullptr, nullptr};
     Width *fw[3] = {nullptr, nullptr, nullptr}, *fd[3] = {nullptr, nullptr, nullptr};
     double2 *rpo = nullptr, *rpn = nullptr;
-    uint8_t* elem_any = nullptr;  // per element: a troubled sub-cell in this slice
+    int *blend_mark = nullptr, *blend_tiles = nullptr, *blend_count = nullptr;  // tiles the troubles reach
     uint8_t *trouble = nullptr, *theta = nullptr;
     unsigned long long* dtmin = nullptr;
     // viscous runs: face viscous fluxes of the pass being evaluated, per

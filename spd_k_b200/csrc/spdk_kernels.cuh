@@ -297,18 +297,15 @@ __device__ __forceinline__ float div_width(const DevGrid&, float x, const Width&
 
 // Sub-cell candidate of the FV update (src/transforms.cpp:483-543 with
 // update=0): U_new = U_old - (w_t dt) sum_d (F_{+} - F_{-}) / h_d for the
-// cell at point pt of element ge; F from FF_d of slice t.
+// cell at point pt of the element at eg; f[d]: the element's face fluxes of
+// direction d and slice t.
 template <int D, int P, typename R>
-__device__ __forceinline__ void fv_candidate(const DevGrid& G, R* const* ff, int t, long long ge, int pt,
+__device__ __forceinline__ void fv_candidate(const DevGrid& G, const R* const (&f)[D], const int eg[3], int pt,
                                              const R* uold, R wdt, R* unew) {
     using S = Shape<D, P>;
     constexpr int n = S::n, nf = S::nf, V = S::V;
     int c[3];
     pt_coords<n>(pt, c);
-    long long eg[3];
-    eg[0] = ge % G.N[0];
-    eg[1] = (ge / G.N[0]) % G.N[1];
-    eg[2] = ge / ((long long)G.N[0] * G.N[1]);
     Width hd[D];
     int fl[3], fr[3];
 #pragma unroll
@@ -323,10 +320,8 @@ __device__ __forceinline__ void fv_candidate(const DevGrid& G, R* const* ff, int
     for (int v = 0; v < V; v++) {
         R F = 0;
 #pragma unroll
-        for (int d = 0; d < D; d++) {
-            const R* f = ff[d] + (((long long)t * G.E + ge) * V + v) * S::NFP;
-            F += div_width(G, f[fr[d]] - f[fl[d]], hd[d]);
-        }
+        for (int d = 0; d < D; d++)
+            F += div_width(G, f[d][v * S::NFP + fr[d]] - f[d][v * S::NFP + fl[d]], hd[d]);
         if (G.grav) {
             R s = 0;
             if (v >= 1 && v <= D) s = uold[0] * (R)G.g[v - 1];
@@ -338,6 +333,18 @@ __device__ __forceinline__ void fv_candidate(const DevGrid& G, R* const* ff, int
         }
         unew[v] = uold[v] - wdt * F;
     }
+}
+// its element's position
+__device__ __forceinline__ void elem_pos(const DevGrid& G, int ge, int eg[3]) {
+    eg[0] = ge % G.N[0];
+    eg[1] = (ge / G.N[0]) % G.N[1];
+    eg[2] = ge / (G.N[0] * G.N[1]);
+}
+// the face-flux blocks of element ge and slice t
+template <int D, int P, typename R>
+__device__ __forceinline__ void face_blocks(const DevGrid& G, const R* const* ff, int t, int ge, const R* (&f)[D]) {
+#pragma unroll
+    for (int d = 0; d < D; d++) f[d] = ff[d] + ((long long)t * G.E + ge) * (D + 2) * Shape<D, P>::NFP;
 }
 
 // (rho, p) of a conserved state with the pressure recovered in FP64
@@ -1022,7 +1029,11 @@ __device__ __forceinline__ void picard_kernel_body(const DevGrid& G, const DevMa
             R uo[V], un[V];
 #pragma unroll
             for (int v = 0; v < V; v++) uo[v] = src[(el * V + v) * NPT + pt];
-            fv_candidate<D, P, R>(G, A.ff, 0, ge, pt, uo, M.wt[0] * dt, un);
+            int eg[3];
+            const R* fb[D];
+            elem_pos(G, (int)ge, eg);
+            face_blocks<D, P, R>(G, A.ff, 0, (int)ge, fb);
+            fv_candidate<D, P, R>(G, fb, eg, pt, uo, M.wt[0] * dt, un);
             A.rp_old[ge * NPT + pt] = rho_p_fp64<D>(uo, G.gm);
             A.rp_new[ge * NPT + pt] = rho_p_fp64<D>(un, G.gm);
         }

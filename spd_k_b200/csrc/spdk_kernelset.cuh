@@ -187,6 +187,9 @@ KernelSetT<R> make_set() {
     return k;
 }
 
+// blocks of a blend launch at most: eight per SM share out the listed tiles
+constexpr unsigned kBlendGrid = 8 * 148;
+
 // blocks of tiles that cover the domain
 inline unsigned tile_blocks(int D, const int N[3], const int tile[3]) {
     long long b = 1;

@@ -747,7 +747,11 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             R uo[V], un[V];
 #pragma unroll
             for (int v = 0; v < V; v++) uo[v] = src[(el * V + v) * NPT + pt];
-            fv_candidate<D, P, R>(G, A.ff, 0, ge, pt, uo, M.wt[0] * dt, un);
+            int eg[3];
+            const R* fb[D];
+            elem_pos(G, (int)ge, eg);
+            face_blocks<D, P, R>(G, A.ff, 0, (int)ge, fb);
+            fv_candidate<D, P, R>(G, fb, eg, pt, uo, M.wt[0] * dt, un);
             A.rp_old[ge * NPT + pt] = rho_p_fp64<D>(uo, G.gm);
             A.rp_new[ge * NPT + pt] = rho_p_fp64<D>(un, G.gm);
         }
