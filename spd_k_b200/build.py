@@ -23,7 +23,7 @@ SOURCES = ["spdk_hydro.cu", "spdk_select_2d_low.cu", "spdk_select_2d_high.cu", "
            "spdk_host_api.cpp"]
 FP32_SOURCES = {"spdk_select_f32_2d.cu", "spdk_select_f32_3d.cu", "spdk_batch_f32.cu", "spdk_tc_study.cu"}
 HEADERS = ["spdk_physics.cuh", "spdk_kernels.cuh", "spdk_fallback.cuh", "spdk_kernelset.cuh", "spdk_setup.h",
-           "spdk_reflayout.cuh", "spdk_learned_impl.h", "spdk_batch.cuh", "spdk_hydro_impl.h", "spdk_viscous.cuh", "spdk_picard2d.cuh"]
+           "spdk_reflayout.cuh", "spdk_learned_impl.h", "spdk_batch.cuh", "spdk_hydro_impl.h", "spdk_viscous.cuh", "spdk_picard2d.cuh", "spdk_picard3d.cuh"]
 
 
 def nvcc_path():

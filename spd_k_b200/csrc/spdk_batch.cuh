@@ -47,13 +47,12 @@ __device__ __forceinline__ const Item& batch_item(const Item* __restrict__ items
     return it;
 }
 
-template <typename R, int D, int P, int TX, int TY, int TZ, int MODE>
-__global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_blocks<R, D, P, TX, TY, TZ, MODE>())
+template <typename R, int P, int TX, int TY, int MODE>
+__global__ void __launch_bounds__(picard_threads<R, 2, P, TX, TY>(), picard_blocks<R, 2, P, MODE>())
     picard_batched(const BatchItem<PicardArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
     long long b;
     const BatchItem<PicardArgsT<R>>& it = batch_item(items, n, &b, blockIdx.x);
-    if constexpr (D == 2) picard2d_body<R, P, TX, TY, MODE, false>(it.G, M, it.A, b);
-    else picard_kernel_body<R, D, P, TX, TY, TZ, MODE>(it.G, M, it.A, b);
+    picard2d_body<R, P, TX, TY, MODE, false>(it.G, M, it.A, b);
 }
 
 // the batched detect takes one block per SM more than the single-problem
@@ -116,9 +115,9 @@ template <typename R, int P, int TX, int TY>
 BatchSetT<R> make_batch_set() {
     BatchSetT<R> k;
     constexpr int PX = kLineTX<P>, PY = kLineTY<P>;
-    k.predict = picard_batched<R, 2, P, PX, PY, 1, kPredict>;
-    k.correct = picard_batched<R, 2, P, PX, PY, 1, kCorrect>;
-    k.flux = picard_batched<R, 2, P, PX, PY, 1, kFlux>;
+    k.predict = picard_batched<R, P, PX, PY, kPredict>;
+    k.correct = picard_batched<R, P, PX, PY, kCorrect>;
+    k.flux = picard_batched<R, P, PX, PY, kFlux>;
     k.picard_threads = picard_threads<R, 2, P, PX, PY>();
     k.picard_tile[0] = PX;
     k.picard_tile[1] = PY;
@@ -130,9 +129,9 @@ BatchSetT<R> make_batch_set() {
     k.blend_tile[1] = BT::Y;
     k.update = update_batched<R, 2, P>;
     k.update_elems = UpdateBlock<2, P>::NE;
-    k.picard_smem[kPredict] = picard_smem_bytes<R, 2, P, PX, PY, 1, kPredict>();
-    k.picard_smem[kCorrect] = picard_smem_bytes<R, 2, P, PX, PY, 1, kCorrect>();
-    k.picard_smem[kFlux] = picard_smem_bytes<R, 2, P, PX, PY, 1, kFlux>();
+    k.picard_smem[kPredict] = picard_smem_bytes<R, 2, P, PX, PY, kPredict>();
+    k.picard_smem[kCorrect] = picard_smem_bytes<R, 2, P, PX, PY, kCorrect>();
+    k.picard_smem[kFlux] = picard_smem_bytes<R, 2, P, PX, PY, kFlux>();
     k.update_smem = UpdateSmem<R, 2, P>::bytes;
     k.tile[0] = TX;
     k.tile[1] = TY;

@@ -111,7 +111,7 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
 // launches of one step, recorded on h->stream (also used for capture)
 template <typename R>
 int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm) {
-    const unsigned pblocks = tile_blocks(h->D, h->G.N, k.picard_tile);
+    const unsigned pblocks = picard_grid(k, h->D, h->G.N);
     const unsigned blocks = tile_blocks(h->D, h->G.N, k.tile);
     // the blend's blocks share out the listed tiles
     const unsigned bblocks = std::min(tile_blocks(h->D, h->G.N, k.blend_tile), kBlendGrid);

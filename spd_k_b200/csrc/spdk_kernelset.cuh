@@ -145,7 +145,9 @@ struct KernelSetT {
     void (*visc)(DevGrid, DevMatsT<R>, ViscArgsT<R>) = nullptr;
     size_t picard_smem[3] = {0, 0, 0}, blend_smem = 0, update_smem = 0;  // predict, correct, flux
     int picard_threads = kThreads;
-    int picard_tile[3] = {1, 1, 1};  // elements of a Picard pass's block (2D: may hang over the domain's edge)
+    // elements of a Picard pass's block: a tile (2D, may hang over the
+    // domain's edge) or consecutive ones (3D)
+    int picard_tile[3] = {1, 1, 1}, picard_elems = 0;
     int tile[3] = {1, 1, 1};         // elements of a detect block
     int blend_tile[3] = {1, 1, 1};   // elements of a blend block
     int update_elems = 1;            // consecutive elements of an update block
@@ -156,14 +158,14 @@ using KernelSet = KernelSetT<double>;
 template <typename R, int D, int P, int TX, int TY, int TZ, bool VISC = false>
 KernelSetT<R> make_set() {
     KernelSetT<R> k;
-    constexpr int PX = D == 2 ? kLineTX<P> : TX, PY = D == 2 ? kLineTY<P> : TY;
-    k.predict = picard_kernel<R, D, P, PX, PY, TZ, kPredict, VISC>;
-    k.correct = picard_kernel<R, D, P, PX, PY, TZ, kCorrect, VISC>;
-    k.flux = picard_kernel<R, D, P, PX, PY, TZ, kFlux, VISC>;
+    constexpr int PX = D == 2 ? kLineTX<P> : 1, PY = D == 2 ? kLineTY<P> : 1;
+    k.predict = picard_kernel<R, D, P, PX, PY, kPredict, VISC>;
+    k.correct = picard_kernel<R, D, P, PX, PY, kCorrect, VISC>;
+    k.flux = picard_kernel<R, D, P, PX, PY, kFlux, VISC>;
     k.picard_threads = picard_threads<R, D, P, PX, PY>();
     k.picard_tile[0] = PX;
     k.picard_tile[1] = PY;
-    k.picard_tile[2] = TZ;
+    if constexpr (D == 3) k.picard_elems = Line3<R, P, kFlux>::EB;
     k.detect = fv_detect_kernel<R, D, P, TX, TY, TZ>;
     using BT = BlendTile<D, P>;
     k.blend = fv_blend_kernel<R, D, P, BT::X, BT::Y, BT::Z>;
@@ -177,9 +179,9 @@ KernelSetT<R> make_set() {
     k.derive = derive_kernel<R, D, P>;
     k.visc = visc_face_kernel<R, D, P>;
     k.visc_epb = ViscShape<R, D, P>::EPB;
-    k.picard_smem[kPredict] = picard_smem_bytes<R, D, P, PX, PY, TZ, kPredict>();
-    k.picard_smem[kCorrect] = picard_smem_bytes<R, D, P, PX, PY, TZ, kCorrect>();
-    k.picard_smem[kFlux] = picard_smem_bytes<R, D, P, PX, PY, TZ, kFlux>();
+    k.picard_smem[kPredict] = picard_smem_bytes<R, D, P, PX, PY, kPredict>();
+    k.picard_smem[kCorrect] = picard_smem_bytes<R, D, P, PX, PY, kCorrect>();
+    k.picard_smem[kFlux] = picard_smem_bytes<R, D, P, PX, PY, kFlux>();
     k.update_smem = UpdateSmem<R, D, P>::bytes;
     k.tile[0] = TX;
     k.tile[1] = TY;
@@ -195,6 +197,14 @@ inline unsigned tile_blocks(int D, const int N[3], const int tile[3]) {
     long long b = 1;
     for (int d = 0; d < D; d++) b *= (N[d] + tile[d] - 1) / tile[d];
     return (unsigned)b;
+}
+
+// blocks of a Picard pass
+template <typename K>
+unsigned picard_grid(const K& k, int D, const int N[3]) {
+    if (!k.picard_elems) return tile_blocks(D, N, k.picard_tile);
+    const long long E = (long long)N[0] * N[1] * N[2];
+    return (unsigned)((E + k.picard_elems - 1) / k.picard_elems);
 }
 
 // element widths, their reciprocals and powers of two (G.N, D and the box
@@ -232,29 +242,12 @@ template <typename R, int P>
 bool pick2(KernelSetT<R>* k, bool visc) {
     return visc ? pick2_t<R, P, true>(k) : pick2_t<R, P, false>(k);
 }
-// 3D: one element per tile, or 2x1x1 elements at p <= 3, where one
-// element's (p+1)^3 points would leave most of the block idle in the
-// per-point phases; the FP64 form takes 2x2x1 elements at p = 2, 3 when
-// nx1 and nx2 are even
+// 3D: 2x2x1 elements up to p = 3 (one element's (p+1)^3 points would leave
+// most of the block idle), one above
 template <typename R, int P>
-bool pick3(int Nx, int Ny, int, KernelSetT<R>* k, bool visc) {
-    if (visc) {
-        *k = make_set<R, 3, P, 1, 1, 1, true>();
-        return true;
-    }
-    if constexpr (sizeof(R) == 8 && (P == 2 || P == 3)) {
-        if (Nx % 2 == 0 && Ny % 2 == 0) {
-            *k = make_set<R, 3, P, 2, 2, 1>();
-            return true;
-        }
-    }
-    if constexpr (P <= 3) {
-        if (Nx % 2 == 0) {
-            *k = make_set<R, 3, P, 2, 1, 1>();
-            return true;
-        }
-    }
-    *k = make_set<R, 3, P, 1, 1, 1>();
+bool pick3(KernelSetT<R>* k, bool visc) {
+    constexpr int T = P <= 3 ? 2 : 1;
+    *k = visc ? make_set<R, 3, P, T, T, 1, true>() : make_set<R, 3, P, T, T, 1>();
     return true;
 }
 

@@ -170,7 +170,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
     G.status = status;
 
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned blocks = tile_blocks(D, N, ks.picard_tile);
+    const unsigned blocks = picard_grid(ks, D, N);
     noalloc_arm<<<1, 1, 0, s>>>(dtmin, status);
     double rk_a[3] = {0, 0, 0};
     if (c.rk_order == 2) rk_a[1] = 0.5;

@@ -1,5 +1,6 @@
 """Element counts that no tile divides: the 2D Picard pass runs 4 x 4 (above
-p = 3: 4 x 2) element tiles that hang over the domain's high edges, and
+p = 3: 4 x 2) element tiles that hang over the domain's high edges, the 3D pass
+blocks of 8, 4, 2 or 1 consecutive elements, the fallback its own tiles, and
 spacings that are no power of two take the division by h from its reciprocal.
 The plain form against the oracle, bit for bit; the precision form against
 the plain form."""
@@ -51,6 +52,19 @@ def test_ragged_counts_match_the_oracle(p, size):
     if integrator == "ader" and k % 5 == 0:
         ov.append("hydro/g2=-0.3")
     against_oracle(ov, *random_state(gpu_config(ov), seed=k))
+
+
+@pytest.mark.parametrize("p", range(1, 6))
+@pytest.mark.parametrize("size", [(2, 2, 2), (3, 2, 5), (5, 3, 2)])
+def test_ragged_counts_match_the_oracle_3d(p, size):
+    k = zlib.crc32(repr((p, size)).encode())
+    ov = overrides(p, size[0], size[1], (EDGES[k % 3], EDGES[(k // 3) % 3]), fallback=k % 2 == 0,
+                   integrator=["ader", "ader", "rk2"][(k // 9) % 3])
+    ov[3] = f"mesh/nx3={size[2]}"
+    ov.append(f"mesh/x3_bc={EDGES[(k // 27) % 3]}")
+    if k % 5 < 2:
+        ov.append("hydro/g3=-0.3")
+    against_oracle(ov, *random_state(gpu_config(ov), seed=k), steps=1 if p == 5 else 2)
 
 
 @pytest.mark.parametrize("scale", [1e-160, 1e-300, 1e80])
