@@ -102,12 +102,13 @@ constexpr int flux_stride() {
 // Phase B: rows of points x H groups of variables.
 // A thread has registers for either the predictor's sums or the flux
 // evaluation at the occupancy that hides its latency, so the predictor keeps
-// the sums in shared memory (one private column per thread) and pays for it
-// with single staging and flux-point buffers: the next slice's copy starts
-// when phase A is over and runs under phase B. Measured per predictor pass at
-// 256^2, p = 3 (the average of a step's three): FP64 260 us with the sums in
-// registers (3 blocks, 356 bytes of spills), 198 us in shared memory (3
-// blocks); FP32 87 us in registers (4 blocks), 84 us in shared memory (6).
+// the sums in shared memory (one private column per thread). A pass has one
+// staging and one flux-point buffer: the next slice's copy starts when phase
+// A is over and runs under phase B, and the shared memory saved is more
+// resident blocks. Measured per predictor pass at 256^2, p = 3 (the average of
+// a step's three): FP64 260 us with the sums in registers (3 blocks, 356
+// bytes of spills), 198 us in shared memory (3 blocks); FP32 87 us in
+// registers (4 blocks), 84 us in shared memory (6).
 template <typename R, int P, int TX, int TY, int MODE>
 struct Line2 {
     static constexpr int n = P + 1, nf = P + 2, V = 4, NPT = n * n, NFP = n * nf, NE = TX * TY;
@@ -122,12 +123,10 @@ struct Line2 {
     static constexpr int A = 2 * LW + warps(EDGE0 + EDGE1);
     static constexpr int threads = A > warps(ROWS) ? A : warps(ROWS);
     static constexpr bool shared_sums = MODE == kPredict;
-    static constexpr int fbufs = (sizeof(R) == 8 || MODE == kPredict) ? 1 : 2;  // staging and flux-point buffers
-    static constexpr int stages = fbufs;
     static constexpr int SS = PicardPad<2, P, R>::SS;          // staged element
     static constexpr int FE = flux_stride<R, n>();             // flux points of an element, one direction
-    static constexpr size_t stage = (size_t)stages * NS * SS;
-    static constexpr size_t fx = (size_t)fbufs * 2 * NE * FE;
+    static constexpr size_t stage = (size_t)NS * SS;
+    static constexpr size_t fx = (size_t)2 * NE * FE;
     static constexpr size_t sums = shared_sums ? (size_t)VB * n * n * ROWS : 0;
     static constexpr size_t grav = MODE == kPredict ? (size_t)n * 3 * NE * NPT : 0;  // predictor slices of rho, m (gravity)
     static constexpr size_t epi = 2 * (size_t)NE * V * NPT;         // W_sp / U_sp and sweep scratch
@@ -144,11 +143,12 @@ template <int P> constexpr int kLineTY = P <= 3 ? 4 : 2;
 // resident blocks per SM the 2D pass's registers are sized for
 // (threads x blocks leave 64 registers a thread at p = 3 in FP32 and 96 to 128
 // in FP64, where spills stay below 40 bytes; FP64 flux pass at p = 3: 347 us
-// at 3 blocks, 304 us at 4; FP32 predictor at p = 5: 98 us with the sums in
+// at 3 blocks, 304 us at 4; FP32 with double buffers at 5 blocks 138 us,
+// single at 5 and 6 134 and 125 us; FP32 predictor at p = 5: 98 us with the sums in
 // registers, 91 / 88 us in shared memory at 5 / 4 blocks)
 template <typename R, int P, int MODE>
 constexpr int kLineBlocksPerSM =
-    sizeof(R) == 4 ? (P == 1 ? 8 : P <= 3 ? (MODE == kPredict ? 6 : 5) : P == 4 ? 5 : P == 5 ? 4 : 2)
+    sizeof(R) == 4 ? (P == 1 ? 8 : P <= 3 ? 6 : P == 4 ? 5 : P == 5 ? 4 : 2)
                    : (P == 1 ? 5 : P <= 4 ? (MODE == kPredict ? 3 : 4) : P == 5 ? (MODE == kPredict ? 2 : 3) : 2);
 
 // the values of one line of one variable's point block: x lines are
@@ -233,8 +233,7 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
     constexpr int NE = TL::NE, NS = TL::NS, NTH = LN::threads;
     constexpr int NT = MODE == kFlux ? 1 : (P + 1);
     constexpr int ND = MODE == kPredict ? NT : 1;  // divergence values kept per point
-    constexpr int SS = LN::SS, FE = LN::FE, VB = LN::VB, ST = LN::stages;
-    constexpr int NFX = LN::fbufs;
+    constexpr int SS = LN::SS, FE = LN::FE, VB = LN::VB;
     constexpr int Q = 16 / (int)sizeof(R);
     using VT = typename Vec16<R>::T;
     static_assert((V * NPT * sizeof(R)) % 16 == 0, "2D element chunks are whole 16-byte units");
@@ -242,11 +241,11 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     R* smem = reinterpret_cast<R*>(smem_raw);
-    R* Sbuf = smem;                       // [stages][NS][SS]
-    R* FX0 = Sbuf + LN::stage;            // [NFX][2][NE][FE]
+    R* Sbuf = smem;                       // [NS][SS]
+    R* FX = Sbuf + LN::stage;             // [2][NE][FE]
     __shared__ int sl_elem[NS];           // staged element (a periodic image outside the domain), -1: none
     __shared__ int el_own[NE];            // element of the tile, -1 outside the domain
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar;
 
     const int tid = threadIdx.x;
     int o[2];
@@ -275,8 +274,7 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         }
     }
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        mbar_init(&bar, 1);
         mbar_fence_init();
     }
     const R dt = (R)(*A.dt);
@@ -320,34 +318,30 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         }
     }
     __syncthreads();
-    // the last warp issues the bulk copies of slice t into buffer b, one
+    // the last warp issues the bulk copies of slice t, one
     // staged element per lane
-    auto issue = [&](int t, int b) {
+    auto issue = [&](int t) {
         if (tid < NTH - 32) return;
         const int lane = tid & 31;
         const R* src = A.in_slices > 1 ? A.ua_in + (long long)t * E * V * NPT : A.ua_in;
-        R* dst = Sbuf + b * NS * SS;
         int cnt = 0;
         for (int s = lane; s < NS; s += 32) cnt += sl_elem[s] >= 0;
         cnt = __reduce_add_sync(0xffffffffu, cnt);
         if (lane == 0) {
             fence_proxy_async_smem();
-            mbar_expect_tx(&bar[b], (uint32_t)(cnt * V * NPT * sizeof(R)));
+            mbar_expect_tx(&bar, (uint32_t)(cnt * V * NPT * sizeof(R)));
         }
         __syncwarp();
         for (int s = lane; s < NS; s += 32)
             if (sl_elem[s] >= 0)
-                bulk_g2s(dst + s * SS, src + (long long)sl_elem[s] * V * NPT, V * NPT * sizeof(R), &bar[b]);
+                bulk_g2s(Sbuf + s * SS, src + (long long)sl_elem[s] * V * NPT, V * NPT * sizeof(R), &bar);
     };
     const bool multi = A.in_slices > 1;
     const int nt_eval = (MODE == kPredict && !multi) ? 1 : nt;
-    issue(0, 0);
+    issue(0);
     for (int t = 0; t < nt_eval; t++) {
-        const int b = ST == 2 && multi ? (t & 1) : 0;
-        const R* Ss = Sbuf + b * NS * SS;
-        R* FX = FX0 + (NFX == 1 ? 0 : (t & 1)) * (2 * NE * FE);
-        if (ST == 2 && multi && t + 1 < nt) issue(t + 1, b ^ 1);
-        if (t == 0 || multi) mbar_wait_bounded(&bar[b], multi ? (ST == 2 ? (t >> 1) & 1 : t & 1) : 0, G.status);
+        const R* Ss = Sbuf;
+        if (t == 0 || multi) mbar_wait_bounded(&bar, t & 1, G.status);
         // ---- phase A: fluxes at every flux point of the slice ----
         bool bad = false;  // a flux value outside div_range
         const bool check = MODE != kFlux && sizeof(R) == 8 && !G.uniform_pow2;
@@ -464,7 +458,7 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         // one staging buffer: the next slice's copy may start, unless phase B
         // still reads this slice's state
         const bool reads = MODE == kCorrect && G.grav;
-        if (ST == 1 && multi && t + 1 < nt && !reads) issue(t + 1, 0);
+        if (multi && t + 1 < nt && !reads) issue(t + 1);
         if constexpr (MODE != kFlux) {
             // ---- phase B: divergence of the thread's rows ----
             if (brow) {
@@ -585,13 +579,9 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
                         reinterpret_cast<const VT*>(FX + d * NE * FE + el * FE)[c];
             }
         }
-        // with one flux buffer the next slice's phase A overwrites this
-        // slice's fluxes; the corrector's gravity source reads this slice's
-        // staging buffer, which the next slice's prefetch overwrites
-        if (NFX == 1 || reads) __syncthreads();
-        if (ST == 1 && multi && t + 1 < nt && reads) issue(t + 1, 0);
+        __syncthreads();  // the next slice's phase A overwrites this slice's fluxes
+        if (multi && t + 1 < nt && reads) issue(t + 1);
     }
-    __syncthreads();
     const int bge = brow ? el_own[bel] : -1;
 
     if constexpr (MODE == kPredict) {
@@ -716,30 +706,46 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             block_min_dt(dtl, A.dtmin);
         }
     } else {
-        // ---- U_cv = sp_to_cv(U) and the slice-0 FV candidate ----
-        __shared__ R Mcv[S::n * S::n];
-        constexpr int CH = V * NPT / Q;  // vectors per element
-        R* Ut = Sbuf;
-        R* Tmp = Sbuf + NE * V * NPT;
-        for (int i = tid; i < S::n * S::n; i += NTH) Mcv[i] = M.sp_to_cv[i];
-        for (int q = tid; q < NE * CH; q += NTH) {
-            const int el = q / CH, c = q % CH;
-            if (el_own[el] >= 0)
-                reinterpret_cast<VT*>(Ut + el * V * NPT)[c] =
-                    reinterpret_cast<const VT*>(A.u + (long long)el_own[el] * V * NPT)[c];
+        // ---- U_cv = sp_to_cv(U) and the slice-0 FV candidate: a thread
+        // averages its rows in x, then, from the rows' x averages, in y ----
+        R* Tx = smem;                      // [NE][V][NPT]
+        R* src = smem + NE * V * NPT;
+        if (brow && bge >= 0) {
+#pragma unroll
+            for (int k = 0; k < VB; k++) {
+                R u[n], a[n];
+                row_load<R, n>(A.u + ((long long)bge * V + bv + k) * NPT + br * n, u);
+#pragma unroll
+                for (int c = 0; c < n; c++) {
+                    a[c] = 0;
+#pragma unroll
+                    for (int l = 0; l < n; l++) a[c] += u[l] * M.sp_to_cv[c * n + l];
+                }
+                row_store<R, n>(Tx + (bel * V + bv + k) * NPT + br * n, a);
+            }
         }
         __syncthreads();
-        sweep_smem<D, P, R>(Ut, Tmp, Mcv, 0, NE * V * NPT);
-        __syncthreads();
-        sweep_smem<D, P, R>(Tmp, Ut, Mcv, 1, NE * V * NPT);
-        __syncthreads();
-        const R* src = Ut;
-        for (int q = tid; q < NE * CH; q += NTH) {
-            const int el = q / CH, c = q % CH;
-            if (el_own[el] >= 0)
-                reinterpret_cast<VT*>(A.ucv + (long long)el_own[el] * V * NPT)[c] =
-                    reinterpret_cast<const VT*>(src + el * V * NPT)[c];
+        if (brow && bge >= 0) {
+            R m[n];
+#pragma unroll
+            for (int l = 0; l < n; l++) m[l] = M.sp_to_cv[br * n + l];
+#pragma unroll
+            for (int k = 0; k < VB; k++) {
+                R a[n];
+#pragma unroll
+                for (int c = 0; c < n; c++) a[c] = 0;
+#pragma unroll
+                for (int l = 0; l < n; l++) {
+                    R u[n];
+                    row_load<R, n>(Tx + (bel * V + bv + k) * NPT + l * n, u);
+#pragma unroll
+                    for (int c = 0; c < n; c++) a[c] += u[c] * m[l];
+                }
+                row_store<R, n>(src + (bel * V + bv + k) * NPT + br * n, a);
+                row_store<R, n>(A.ucv + ((long long)bge * V + bv + k) * NPT + br * n, a);
+            }
         }
+        __syncthreads();
         for (int q = tid; q < NE * NPT; q += NTH) {
             const int el = q / NPT, pt = q % NPT;
             const long long ge = el_own[el];
