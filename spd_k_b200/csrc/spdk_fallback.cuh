@@ -305,7 +305,9 @@ static __device__ __noinline__ void sed_al_tile_2d(const SedGeom S, const double
 // instantiation per form keeps each form's compile flags on its own copy.
 //
 // Each thread loads its cells' candidates before it stages the tile's W_old,
-// so a block waits for one memory round trip, not two. In 2D the kernel is
+// so a block waits for one memory round trip, not two. Cell numbers come from
+// per-direction tables (CellMap), and a thread's cells are in memory order, so
+// the flags leave in whole sectors. In 2D the kernel is
 // compiled for 4 resident blocks (64 registers, the NAD pass unspilled;
 // measured on B200: 38.6 us against 43.2 us at 6 blocks with spills); in
 // 3D for 3 (80 registers, 20-50 bytes of spills; 90 registers and 2

@@ -178,7 +178,8 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.wcv = (R*)h->wcv;
             A.dtmin = h->dtmin;
             prof_begin(h);
-            SPDK_CUDA(launch_pdl(k.correct, dim3(pblocks), pthreads, k.picard_smem[kCorrect], h->stream, h->G, dm, A));
+            const auto correct = k.correct_few && pblocks <= kFewBlocks ? k.correct_few : k.correct;
+            SPDK_CUDA(launch_pdl(correct, dim3(pblocks), pthreads, k.picard_smem[kCorrect], h->stream, h->G, dm, A));
             prof_end(h, SPDK_KERNEL_CORRECT);
             launches++;
         } else {
@@ -339,8 +340,10 @@ int set_attributes(const KernelSetT<R>& ks) {
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
     const std::pair<const void*, size_t> fv[] = {{(const void*)ks.blend, ks.blend_smem},
-                                                 {(const void*)ks.update, ks.update_smem}};
+                                                 {(const void*)ks.update, ks.update_smem},
+                                                 {(const void*)ks.correct_few, ks.picard_smem[kCorrect]}};
     for (const auto& f : fv) {
+        if (!f.first) continue;
         cudaFuncSetAttribute(f.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         if (cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second) != cudaSuccess)
             return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(f.second) + " bytes");

@@ -123,19 +123,16 @@ struct Shape {
     static constexpr int NFP = NTP * nf;   // flux points per direction
 };
 
-// padded shared-memory strides of the Picard pass (bank spreading); an
-// element block (SS) starts on a 16-byte boundary whenever its data is a
-// whole number of 16-byte units, so it can be a bulk-copy destination
+// stride of a staged element of the 2D Picard pass: whole 16-byte units (it is
+// a bulk copy's destination), not a multiple of 32 banks
 template <int D, int P, typename R = double>
 struct PicardPad {
     static constexpr int V = D + 2;
     static constexpr int NPT = D == 2 ? (P + 1) * (P + 1) : (P + 1) * (P + 1) * (P + 1);
-    static constexpr int NFP = NPT / (P + 1) * (P + 2);
     static constexpr int Q = 16 / (int)sizeof(R);                   // elements per 16 bytes
     static constexpr int WORDS = (int)sizeof(R) / 4;                 // 4-byte banks per element
     static constexpr int SS0 = (V * NPT + Q - 1) / Q * Q;
     static constexpr int SS = SS0 + ((SS0 * WORDS) % 32 == 0 ? Q : 0);
-    static constexpr int FXS = NFP + ((NFP * V) % 16 == 0 ? 1 : 0);
 };
 
 // coordinates of a point index
@@ -171,7 +168,6 @@ struct Tile {
     static constexpr int NE = TX * TY * TZ;
     static constexpr int HX = TY * TZ, HY = TX * TZ, HZ = TX * TY;
     static constexpr int NS = NE + 2 * HX + 2 * HY + (D == 3 ? 2 * HZ : 0);
-    __device__ static int T(int d) { return d == 0 ? TX : (d == 1 ? TY : TZ); }
     // slot of tile-local element coordinates (at most one outside the tile)
     __device__ static int slot(int lx, int ly, int lz) {
         if (lx < 0 || lx >= TX) return NE + (lx < 0 ? 0 : HX) + ly + TY * lz;
@@ -202,22 +198,6 @@ struct Tile {
         l[2] = side ? TZ : -1; l[0] = q % TX; l[1] = q / TX;
     }
 };
-
-// global element index of tile-local coordinates, or -1 when the element
-// lies beyond a non-periodic domain edge
-template <int D>
-__device__ __forceinline__ long long elem_of(const DevGrid& G, const int o[3], const int l[3]) {
-    int g[3];
-    for (int d = 0; d < 3; d++) {
-        g[d] = o[d] + l[d];
-        if (d >= D) { g[d] = 0; continue; }
-        if (g[d] < 0 || g[d] >= G.N[d]) {
-            if (G.bc[d] != kPeriodic) return -1;
-            g[d] = g[d] < 0 ? g[d] + G.N[d] : g[d] - G.N[d];
-        }
-    }
-    return ((long long)g[2] * G.N[1] + g[1]) * G.N[0] + g[0];
-}
 
 // dt candidate of one W_cv point (src/hydro.cpp:222-254, inviscid), always
 // evaluated in FP64
@@ -445,6 +425,18 @@ __global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_bloc
     if (gate_closed(G)) return;
     if constexpr (D == 2) picard2d_body<R, P, TX, TY, MODE, VISC>(G, M, A, blockIdx.x);
     else picard3d_body<R, P, MODE, VISC>(G, M, A, blockIdx.x);
+}
+
+// The corrector for launches of few blocks: compiled for two blocks per SM
+// (no spills, more independent work per warp), because such a launch is one
+// chain of latencies. 32^2 p=3 FP64, 8 steps: 272 -> 262 us; at 256^2 the four
+// blocks of the other one are faster (3.19 against 3.53 ms for 4 steps).
+template <typename R, int P, int TX, int TY>
+__global__ void __launch_bounds__(picard_threads<R, 2, P, TX, TY>(), 2)
+    correct_few_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
+    pdl_wait();
+    if (gate_closed(G)) return;
+    picard2d_body<R, P, TX, TY, kCorrect, false>(G, M, A, blockIdx.x);
 }
 
 template <typename R, int D, int P, int TX, int TY, int MODE>

@@ -137,6 +137,8 @@ struct KernelSetT {
     void (*predict)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*correct)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*flux)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
+    // the corrector of a launch of at most kFewBlocks blocks (null: `correct`)
+    void (*correct_few)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*detect)(DevGrid, DetectArgs) = nullptr;
     void (*blend)(DevGrid, DevMatsT<R>, BlendArgsT<R>) = nullptr;
     void (*update)(DevGrid, DevMatsT<R>, FallbackArgsT<R>) = nullptr;
@@ -162,6 +164,7 @@ KernelSetT<R> make_set() {
     k.predict = picard_kernel<R, D, P, PX, PY, kPredict, VISC>;
     k.correct = picard_kernel<R, D, P, PX, PY, kCorrect, VISC>;
     k.flux = picard_kernel<R, D, P, PX, PY, kFlux, VISC>;
+    if constexpr (D == 2 && sizeof(R) == 8 && P <= 4 && !VISC) k.correct_few = correct_few_kernel<R, P, PX, PY>;
     k.picard_threads = picard_threads<R, D, P, PX, PY>();
     k.picard_tile[0] = PX;
     k.picard_tile[1] = PY;
@@ -188,6 +191,9 @@ KernelSetT<R> make_set() {
     k.tile[2] = TZ;
     return k;
 }
+
+// two blocks per SM at once
+constexpr unsigned kFewBlocks = 2 * 148;
 
 // blocks of a blend launch at most: eight per SM share out the listed tiles
 constexpr unsigned kBlendGrid = 8 * 148;
