@@ -126,14 +126,12 @@ __global__ void __launch_bounds__(256, 3) ind2_pass(Ind2Geo G, Ind2Mats<R> M, In
         Msf[i] = M.sp_to_fp[i];
         Mdf[i] = M.dfp_to_sp[i];
     }
-    const int tiles_x = G.N[0] / TX;
+    // tiles at the high edges may hang over the domain: their outside elements
+    // are periodic images, evaluated and not stored
+    const int tiles_x = (G.N[0] + TX - 1) / TX;
     const int i0 = (int)(blockIdx.x % tiles_x) * TX, j0 = (int)(blockIdx.x / tiles_x) * TY;
     for (int s = tid; s < NS; s += 256) {
-        int i = i0 + s % SX - 1, j = j0 + s / SX - 1;
-        if (i < 0) i += G.N[0];
-        if (i >= G.N[0]) i -= G.N[0];
-        if (j < 0) j += G.N[1];
-        if (j >= G.N[1]) j -= G.N[1];
+        const int i = (i0 + s % SX - 1 + G.N[0]) % G.N[0], j = (j0 + s / SX - 1 + G.N[1]) % G.N[1];
         sl_el[s] = j * G.N[0] + i;
     }
     const R vx = (R)G.v[0], vy = (R)G.v[1];
@@ -263,6 +261,7 @@ __global__ void __launch_bounds__(256, 3) ind2_pass(Ind2Geo G, Ind2Mats<R> M, In
         if (it >= T::ITEMS) continue;
         const int el = it / (2 * FB), r = it % (2 * FB);
         const bool isx = r < FB;
+        if (i0 + el % TX >= G.N[0] || j0 + el / TX >= G.N[1]) continue;
         const long long q = (long long)sl_el[(el / TX + 1) * SX + el % TX + 1] * FB + (isx ? r : r - FB);
         const R b_old = isx ? ((const R*)A.bx_old)[q] : ((const R*)A.by_old)[q];
         R* out = (R*)(isx ? A.bx_out : A.by_out);
@@ -385,7 +384,8 @@ int enqueue_t(spdk_induction2d* s) {
     if (cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return fail(SPDK_E_CUDA, "induction2d: shared memory request of " + std::to_string(smem) + " bytes");
-    const unsigned blocks = (unsigned)(E / (TX * TY));
+    const unsigned blocks =
+        (unsigned)((long long)((s->cfg.N[0] + TX - 1) / TX) * ((s->cfg.N[1] + TY - 1) / TY));
     int launches = 0;
     R* bx = (R*)s->bx;
     R* by = (R*)s->by;
@@ -437,16 +437,12 @@ int enqueue_t(spdk_induction2d* s) {
     return 0;
 }
 
-// tiles of 4 x 4 elements up to p = 4, 2 x 2 above (their per-thread
-// predictor slices stay in registers), whichever divides the element counts
+// tiles of 4 x 4 elements up to p = 4, 2 x 2 above, whatever the element
+// counts (one-element tiles for odd counts took 7 times as long per element)
 template <typename R, int P>
 int enqueue2(spdk_induction2d* s) {
-    const int Nx = s->cfg.N[0], Ny = s->cfg.N[1];
-    if constexpr (P <= 4) {
-        if (Nx % 4 == 0 && Ny % 4 == 0) return enqueue_t<R, P, 4, 4>(s);
-    }
-    if (Nx % 2 == 0 && Ny % 2 == 0) return enqueue_t<R, P, 2, 2>(s);
-    return enqueue_t<R, P, 1, 1>(s);
+    constexpr int T = P <= 4 ? 4 : 2;
+    return enqueue_t<R, P, T, T>(s);
 }
 
 template <typename R>

@@ -94,3 +94,15 @@ def test_field_loop_512_to_t1():
     for a, b in zip(e64, e32):
         assert a < 0.01
         assert abs(b - a) <= 0.01 * a
+
+
+@pytest.mark.parametrize("N,p,integrator", [(2, 2, "ader"), (5, 4, "ader"), (7, 3, "rk2"), (9, 5, "ader"), (11, 1, "rk3")])
+def test_counts_that_no_tile_divides(N, p, integrator):
+    """4 x 4 (2 x 2 above p = 4) element tiles hang over the domain's high
+    edges: a few steps against the same scheme in plain FP64 torch"""
+    from perf import cases
+    case = {"kind": "loop", "n": N, "p": p, "precision": "fp64", "integrator": integrator, "steps": 4}
+    got, want = cases.run(cases.prepare(case, 3)), cases.exact(case, 3)
+    for a, b in zip(got, want):
+        # each step re-evaluates the derivative sums: round-off times their condition (p^2)
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
