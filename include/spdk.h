@@ -259,6 +259,9 @@ int spdk_fv_faces(int N, int p, double L, int active, double* out, size_t count)
  * current, resolves the array's device address and sets kernel attributes:
  * make it before any stream capture. Calls share the array, so calls that
  * overlap on the GPU race; order them on one stream. No call allocates.
+ * Buffers are aligned to their 8-byte values; u_in and u_out start on 16-byte
+ * boundaries in 2D at odd p, and u_in in every ADER step in 2D or at odd p
+ * (otherwise SPDK_E_ARG). In 3D the step is fastest when both do.
  * Slab configurations (slab_lo, slab_n != 0) are rejected with SPDK_E_ARG.
  * Device-detected faults: every call clears the array's status word when it
  * starts; if a bounded shared-memory staging wait runs out during the call,

@@ -439,6 +439,15 @@ __global__ void __launch_bounds__(picard_threads<R, 2, P, TX, TY>(), 2)
     picard2d_body<R, P, TX, TY, kCorrect, false>(G, M, A, blockIdx.x);
 }
 
+// The 3D corrector on a caller's buffers that start on no 16-byte boundary
+template <typename R, int P>
+__global__ void __launch_bounds__(picard_threads<R, 3, P, 1, 1>(), picard_blocks<R, 3, P, kCorrect>())
+    correct_any_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
+    pdl_wait();
+    if (gate_closed(G)) return;
+    picard3d_body<R, P, kCorrect, false, true>(G, M, A, blockIdx.x);
+}
+
 template <typename R, int D, int P, int TX, int TY, int MODE>
 constexpr size_t picard_smem_bytes() {
     if constexpr (D == 2) return Line2<R, P, TX, TY, MODE>::bytes;

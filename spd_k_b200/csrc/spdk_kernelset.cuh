@@ -139,6 +139,9 @@ struct KernelSetT {
     void (*flux)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     // the corrector of a launch of at most kFewBlocks blocks (null: `correct`)
     void (*correct_few)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
+    // the corrector on state buffers that start on no 16-byte boundary (null:
+    // `correct` takes them if n is odd, and nothing does if n is even)
+    void (*correct_any)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*detect)(DevGrid, DetectArgs) = nullptr;
     void (*blend)(DevGrid, DevMatsT<R>, BlendArgsT<R>) = nullptr;
     void (*update)(DevGrid, DevMatsT<R>, FallbackArgsT<R>) = nullptr;
@@ -165,6 +168,7 @@ KernelSetT<R> make_set() {
     k.correct = picard_kernel<R, D, P, PX, PY, kCorrect, VISC>;
     k.flux = picard_kernel<R, D, P, PX, PY, kFlux, VISC>;
     if constexpr (D == 2 && sizeof(R) == 8 && P <= 4 && !VISC) k.correct_few = correct_few_kernel<R, P, PX, PY>;
+    if constexpr (D == 3 && sizeof(R) == 8 && P % 2 == 1 && !VISC) k.correct_any = correct_any_kernel<R, P>;
     k.picard_threads = picard_threads<R, D, P, PX, PY>();
     k.picard_tile[0] = PX;
     k.picard_tile[1] = PY;

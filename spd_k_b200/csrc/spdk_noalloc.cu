@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -82,10 +83,13 @@ int setup_device(int dev, const KernelSet& ks, void** base) {
         g_scratch_ptr[dev] = p;
     }
     // per-kernel attributes (idempotent, not an allocation)
-    const void* fns[] = {(const void*)ks.predict, (const void*)ks.correct};
-    for (int m = 0; m < 2; m++) {
-        const void* f = fns[m];
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem[m]);
+    const struct { const void* f; int mode; } fns[] = {{(const void*)ks.predict, kPredict},
+                                                       {(const void*)ks.correct, kCorrect},
+                                                       {(const void*)ks.correct_any, kCorrect}};
+    for (const auto& k : fns) {
+        const void* f = k.f;
+        if (!f) continue;
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem[k.mode]);
         if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
@@ -125,6 +129,17 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
     if (need > kScratchBytes - kHeaderBytes)
         return fail(SPDK_E_ARG, "problem needs " + std::to_string(need) + " bytes of working storage; the "
                                 "allocation-free step has " + std::to_string(kScratchBytes - kHeaderBytes));
+
+    // An even n moves rows as 16-byte vectors, and an ADER step copies u_in in
+    // bulk wherever an element is whole 16-byte units; only the 3D corrector
+    // (correct_any) has a form for buffers that start on an 8-byte boundary
+    auto off = [](const void* p, size_t to) { return (uintptr_t)p % to != 0; };
+    if (off(u_in, 8) || off(u_out, 8) || off(wcv_out, 8) || off(dt_inout, 8))
+        return fail(SPDK_E_ARG, "a buffer is not aligned to its 8-byte values");
+    if (ader && (D == 2 || n % 2 == 0) && off(u_in, 16))
+        return fail(SPDK_E_ARG, "an ADER step in 2D, or in 3D at odd p, needs u_in aligned to 16 bytes");
+    if (D == 2 && n % 2 == 0 && (off(u_in, 16) || off(u_out, 16)))
+        return fail(SPDK_E_ARG, "a 2D step at odd p needs u_in and u_out aligned to 16 bytes");
 
     KernelSet ks;
     if (!select_kernels(D, c.p, N, &ks)) return fail(SPDK_E_ARG, "no kernel instantiation for this ndim/p");
@@ -171,6 +186,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
 
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned blocks = picard_grid(ks, D, N);
+    const auto correct = ks.correct_any && (off(u_in, 16) || off(u_out, 16)) ? ks.correct_any : ks.correct;
     noalloc_arm<<<1, 1, 0, s>>>(dtmin, status);
     double rk_a[3] = {0, 0, 0};
     if (c.rk_order == 2) rk_a[1] = 0.5;
@@ -196,7 +212,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
         A.final_stage = 1;
         A.wcv = wcv_out;
         A.dtmin = dtmin;
-        ks.correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
+        correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
     } else {
         double* stage_in = work;
         double* u0 = work + (size_t)E * V * NPT;
@@ -218,7 +234,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
             A.wcv = wcv_out;
             A.dtmin = dtmin;
             A.dt = dt_inout;
-            ks.correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
+            correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
             cur = u_out;
         }
     }

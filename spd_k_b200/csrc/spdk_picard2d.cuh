@@ -41,10 +41,9 @@ template <> struct Vec16<double> { using T = double2; };
 template <typename R, int n>
 constexpr int kRowVec = sizeof(R) == 4 ? (n % 4 == 0 ? 4 : (n % 2 == 0 ? 2 : 1)) : (n % 2 == 0 ? 2 : 1);
 
-// n consecutive values between memory and registers
-template <typename R, int n>
+// n consecutive values between memory and registers, W at a time
+template <typename R, int n, int W = kRowVec<R, n>>
 __device__ __forceinline__ void row_load(const R* p, R* out) {
-    constexpr int W = kRowVec<R, n>;
     if constexpr (W == 1) {
 #pragma unroll
         for (int i = 0; i < n; i++) out[i] = p[i];
@@ -59,9 +58,8 @@ __device__ __forceinline__ void row_load(const R* p, R* out) {
         }
     }
 }
-template <typename R, int n>
+template <typename R, int n, int W = kRowVec<R, n>>
 __device__ __forceinline__ void row_store(R* p, const R* in) {
-    constexpr int W = kRowVec<R, n>;
     if constexpr (W == 1) {
 #pragma unroll
         for (int i = 0; i < n; i++) p[i] = in[i];

@@ -81,7 +81,9 @@ __device__ __forceinline__ void ghost3(const DevGrid& G, const R* in, R* out, in
     for (int v = 0; v < 5; v++) out[v] = (flip && v == 1 + d) ? -in[v] : in[v];
 }
 
-template <typename R, int P, int MODE, bool VISC>
+// ANY: the corrector's u, u0 and u_out are a caller's buffers that start on no
+// 16-byte boundary; their rows move value by value
+template <typename R, int P, int MODE, bool VISC, bool ANY = false>
 __device__ __forceinline__ void picard3d_body(const DevGrid& G, const DevMatsT<R>& M, const PicardArgsT<R>& A,
                                               long long bidx) {
     constexpr int D = 3;
@@ -465,20 +467,21 @@ __device__ __forceinline__ void picard3d_body(const DevGrid& G, const DevMatsT<R
         };
         if constexpr (MODE == kCorrect) {
             // ---- corrector / RK stage (src/transforms.cpp:327-374, 252-261) ----
+            constexpr int W = ANY ? 1 : kRowVec<R, n>;
             if (brow) {
                 const long long g = (bge * V + bv) * NPT + br * n;
                 R val[n];
-                row_load<R, n>(A.u + g, val);
+                row_load<R, n, W>(A.u + g, val);
 #pragma unroll
                 for (int i = 0; i < n; i++) val[i] -= acc(i, 0);
                 if (A.rk_a > 0) {
                     const R ra = (R)A.rk_a;
                     R u0[n];
-                    row_load<R, n>(A.u0 + g, u0);
+                    row_load<R, n, W>(A.u0 + g, u0);
 #pragma unroll
                     for (int i = 0; i < n; i++) val[i] = ra * u0[i] + ((R)1.0 - ra) * val[i];
                 }
-                row_store<R, n>(A.u_out + g, val);
+                row_store<R, n, W>(A.u_out + g, val);
 #pragma unroll
                 for (int i = 0; i < n; i++) B0[(bel * V + bv) * NPT + br * n + i] = val[i];
             }

@@ -174,3 +174,22 @@ def test_fv_faces_match_oracle(lib):
                                  ctypes.c_size_t(n)) == 0
         if act:
             assert np.array_equal(out, want)
+
+
+@pytest.mark.parametrize("ov,u_in,u_out,dt", [
+    (["mesh/nx3=1"], 0x1008, 0x2000, 0x3000),                                            # ADER: bulk copy of u_in
+    (["mesh/nx3=1", "mesh/p=2"], 0x1008, 0x2000, 0x3000),
+    (["mesh/nx3=1"], 0x1000, 0x2008, 0x3000),                                            # rows of u_out as vectors
+    (["mesh/nx3=1", "time/integrator=rk2"], 0x1008, 0x2000, 0x3000),                      # rows of u_in as vectors
+    (["mesh/nx1=3", "mesh/nx2=3", "mesh/nx3=3"], 0x1008, 0x2000, 0x3000),
+    (["mesh/nx1=3", "mesh/nx2=3", "mesh/nx3=3", "mesh/p=2"], 0x1000, 0x2004, 0x3000),     # not even whole doubles
+    (["mesh/nx3=1"], 0x1000, 0x2000, 0x3004),
+])
+def test_noalloc_refuses_buffers_its_kernels_cannot_take(lib, ov, u_in, u_out, dt):
+    """refused before any device call (the addresses are never touched)"""
+    from spd_k_b200.api import make_config
+    cfg = make_config(gpu_config(["job/fallback=false", *ov]))
+    f = lib.spdk_hydro_step_noalloc
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_void_p] * 6
+    assert f(ctypes.addressof(cfg), u_in, u_out, None, dt, None) == -1
+    assert b"aligned" in lib.spdk_last_error()

@@ -115,3 +115,43 @@ def test_noalloc_rejects_oversized_and_fallback_configs():
     slab.slab_lo = 2
     rc = step(ctypes.addressof(slab), 16, 16, None, 16, None)
     assert rc == -1 and b"slab" in lib.spdk_last_error()
+
+
+# (overrides, offset of u_in, offset of u_out) in doubles past a 16-byte boundary
+OFFSETS = {
+    "ader_3d_p3": (["mesh/p=3", "mesh/nx1=3", "mesh/nx2=2", "mesh/nx3=4"], 0, 1),
+    "ader_3d_p1": (["mesh/p=1", "mesh/nx1=5", "mesh/nx2=3", "mesh/nx3=3"], 0, 1),
+    "rk3_3d_p1": (["mesh/p=1", "mesh/nx1=5", "mesh/nx2=3", "mesh/nx3=3", "time/integrator=rk3"], 1, 1),
+    "rk2_3d_p5": (["mesh/p=5", "mesh/nx1=2", "mesh/nx2=2", "mesh/nx3=3", "time/integrator=rk2"], 1, 0),
+    "ader_3d_p2": (["mesh/p=2", "mesh/nx1=3", "mesh/nx2=3", "mesh/nx3=3"], 1, 1),
+    "rk2_2d_p2": (["mesh/p=2", "mesh/nx1=5", "mesh/nx2=6", "mesh/nx3=1", "time/integrator=rk2"], 1, 1),
+}
+
+
+@pytest.mark.parametrize("case", sorted(OFFSETS))
+def test_buffers_that_start_on_an_8_byte_boundary(case):
+    """sub-ranges of a caller's pool: the same bits as the allocating solver"""
+    import torch
+
+    import spd_k_b200 as S
+    from spd_k_b200.api import apply_overrides, config_from_params, make_config
+
+    ov, oi, oo = OFFSETS[case]
+    prob = "spherical_blast" if "3d" in case else "kelvin_helmholtz"
+    c = config_from_params(apply_overrides({}, ["job/fallback=false", f"problem/problem={prob}", *ov]))
+    ref, lib, cfg = S.HydroSolver(c), S.load_library(), make_config(c)
+    start = torch.from_numpy(ref.read(S.FIELD_U_SP)).cuda()
+    pool = [torch.zeros(start.numel() + 2, dtype=torch.float64, device="cuda") for _ in range(2)]
+    u, out = pool[0][oi:oi + start.numel()], pool[1][oo:oo + start.numel()]
+    assert u.data_ptr() % 16 == 8 * oi and out.data_ptr() % 16 == 8 * oo
+    u.copy_(start)
+    dt = torch.tensor([ref.dt()], dtype=torch.float64, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    rc = bind(lib)(ctypes.addressof(cfg), u.data_ptr(), out.data_ptr(), None, dt.data_ptr(), stream)
+    assert rc == 0, lib.spdk_last_error().decode()
+    ref.step()
+    assert status(lib, stream) == 0
+    assert np.array_equal(out.cpu().numpy(), ref.read(S.FIELD_U_SP)) and float(dt.item()) == ref.dt()
+    assert torch.equal(u, start)
+    assert pool[1][:oo].count_nonzero() == 0 and pool[1][oo + start.numel():].count_nonzero() == 0
+    ref.close()
