@@ -98,11 +98,19 @@ __device__ __forceinline__ long long cell_image(const DevGrid& G, const int a[3]
 
 // Cell numbers of a tile and its halo: the number of cell (x, y, z) of the
 // frame that begins H cells outside the tile is x0[x] + x1[y] + x2[z], each
-// part from the cell's image in that direction; a part is negative (kNoCell)
-// where there is none (outside the domain and its `layers` ghost layers), and
-// flip[d] marks reflective images. Formed once per block, so that a staged
-// cell costs two or three shared loads instead of the image arithmetic.
-constexpr int kNoCell = -(1 << 29);  // below minus any cell number (fewer than 2^29 cells fit the memory)
+// part from the cell's image in that direction; a part is kNoCell where there
+// is none (outside the domain and its `layers` ghost layers), and flip[d]
+// marks reflective images. Formed once per block, so that a staged cell costs
+// two or three shared loads instead of the image arithmetic. Cell numbers fit
+// 32 bits: the smallest state with the fallback (2D, FP32, SSP-RK1) takes 146
+// bytes a cell, 313 GB for 2^31 of them.
+constexpr int kNoCell = -1;
+__host__ __device__ constexpr int cell_number(int x, int y, int z) {
+    return (x | y | z) < 0 ? kNoCell : x + y + z;  // a part that is missing outweighs any sum of the others
+}
+static_assert(cell_number(kNoCell, 1 << 30, 0) < 0 && cell_number(1 << 30, kNoCell, 0) < 0 &&
+              cell_number(1 << 29, 1 << 29, kNoCell) < 0, "no image whatever the other parts");
+static_assert(cell_number(5, 1 << 29, 1 << 30) == 5 + (1 << 29) + (1 << 30), "large cell numbers");
 template <int D, int P, int TX, int TY, int TZ, int H>
 struct CellMap {
     static constexpr int n = P + 1;
@@ -131,7 +139,7 @@ struct CellMap {
     }
     // cell number, negative where the cell has no image
     __device__ __forceinline__ int cell(int x, int y, int z) const {
-        return x0[x] + x1[y] + (D == 3 ? x2[z] : 0);
+        return cell_number(x0[x], x1[y], D == 3 ? x2[z] : 0);
     }
 };
 
