@@ -438,13 +438,29 @@ int enqueue_t(spdk_induction2d* s) {
     return 0;
 }
 
-// tiles of 4 x 4 elements up to p = 4, 2 x 2 above, whatever the element
-// counts (255^2 p=4 FP64 steps: 12.9 ms on the one-element tiles that odd counts
-// took before, 4.2 ms)
+// Tiles of 4 x 4 elements up to p = 4 and 2 x 2 above re-read the least ring
+// per element, so they are the fastest where every SM has several blocks (256^2
+// p=4 FP64: 2 x 2 takes 1.31 of the time, one element 3.5), whatever the element
+// counts. A small grid is a chain of latencies that grows with a block's work:
+// it takes a smaller tile while that one's blocks per SM are few.
+// One element: up to 3 blocks per SM, which are resident at once (FP32 above p = 5: 4).
+//   20^2 against 2 x 2: p=5 FP64 110 / 167 us, p=7 FP64 275 / 417 us, p=6 FP32 (24^2) 119 / 155 us;
+//   24^2: p=5 FP64 198 / 167 us, p=7 FP64 488 / 417 us.
+// 2 x 2 (p = 2 to 4): up to 4 blocks per SM at p = 2, 6 above, 9 in FP32 at p = 4.
+//   48^2 against 4 x 4: p=2 FP64 0.73 / 1.02, p=4 FP64 0.77 / 1.01 of the time on 4 x 4 tiles;
+//   64^2: p=2 1.13 / 1.07, p=3 1.27 / 1.01, p=4 1.08 / 1.02, p=4 FP32 0.85 / 1.01 (80^2: 1.06 / 1.00).
+// p = 1 is launch latency on any tile.
 template <typename R, int P>
 int enqueue2(spdk_induction2d* s) {
-    constexpr int T = P <= 4 ? 4 : 2;
-    return enqueue_t<R, P, T, T>(s);
+    constexpr bool f32 = sizeof(R) == 4;
+    constexpr int kSMs = 148;
+    const int* N = s->cfg.N;
+    auto blocks = [&](int T) { return (long long)((N[0] + T - 1) / T) * ((N[1] + T - 1) / T); };
+    if constexpr (P > 1) {
+        if (blocks(1) <= kSMs * (f32 && P > 5 ? 4 : 3)) return enqueue_t<R, P, 1, 1>(s);
+        if (P > 4 || blocks(2) <= kSMs * (P == 2 ? 4 : (f32 && P == 4 ? 9 : 6))) return enqueue_t<R, P, 2, 2>(s);
+    }
+    if constexpr (P <= 4) return enqueue_t<R, P, 4, 4>(s);
 }
 
 template <typename R>

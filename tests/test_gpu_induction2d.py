@@ -16,7 +16,7 @@ import os
 import numpy as np
 import pytest
 
-from helpers import GOLDEN, same_bits
+from helpers import GOLDEN, field_loop_steps, same_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -96,13 +96,41 @@ def test_field_loop_512_to_t1():
         assert abs(b - a) <= 0.01 * a
 
 
+def against_plain_scheme(Nx, Ny, p, integrator, precision, steps=4):
+    from spd_k_b200.induction import FIELD2_BX, FIELD2_BY, Induction2D, field_loop_config
+    c = field_loop_config(N=Nx, p=p, precision=precision, integrator=integrator)
+    c["N"], c["L"], c["velocity"], c["cfl"] = [Nx, Ny], [2.0, 2.0 * Ny / Nx], (1.3, -0.7), 0.4
+    s = Induction2D(c)
+
+    def fields():
+        return (s.read(FIELD2_BX).reshape(Ny, Nx, p + 1, p + 2), s.read(FIELD2_BY).reshape(Ny, Nx, p + 2, p + 1))
+    start, dt = fields(), s.dt()
+    for _ in range(steps):
+        s.step()
+    got = fields()
+    s.close()
+    h = [c["L"][0] / Nx, c["L"][1] / Ny]
+    want = field_loop_steps(*start, h, c["velocity"], p, integrator, dt, steps)
+    # each step re-evaluates derivative sums of 2 (p + 2) terms: the round-off
+    # of a value times their condition, at most 8 (p + 1)^2
+    eps = 1.2e-7 if precision == "fp32" else 2.3e-16
+    for a, b in zip(got, want):
+        assert np.abs(a - b).max() <= steps * 8 * (p + 1) ** 2 * eps * np.abs(b).max()
+
+
 @pytest.mark.parametrize("N,p,integrator", [(2, 2, "ader"), (5, 4, "ader"), (7, 3, "rk2"), (9, 5, "ader"), (11, 1, "rk3")])
 def test_counts_that_no_tile_divides(N, p, integrator):
-    """4 x 4 (2 x 2 above p = 4) element tiles hang over the domain's high
-    edges: a few steps against the same scheme in plain FP64 torch"""
-    from perf import cases
-    case = {"kind": "loop", "n": N, "p": p, "precision": "fp64", "integrator": integrator, "steps": 4}
-    got, want = cases.run(cases.prepare(case, 3)), cases.exact(case, 3)
-    for a, b in zip(got, want):
-        # each step re-evaluates the derivative sums: round-off times their condition (p^2)
-        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+    """tiles hang over the domain's high edges: a few steps against the same
+    scheme in plain FP64 numpy"""
+    against_plain_scheme(N, N, p, integrator, "fp64")
+
+
+# both sides of every switch between one-element, 2 x 2 and 4 x 4 tiles
+SWITCHES = [(2, "fp64", [(21, 21), (22, 21), (47, 48), (50, 47)]), (3, "fp64", [(21, 21), (23, 20), (58, 59), (59, 60)]),
+            (4, "fp64", [(21, 21), (22, 21), (59, 58), (59, 60)]), (4, "fp32", [(21, 21), (22, 21), (73, 72), (74, 73)]),
+            (6, "fp64", [(21, 21), (22, 21)]), (7, "fp32", [(24, 24), (25, 24)]), (1, "fp32", [(3, 2), (33, 34)])]
+
+
+@pytest.mark.parametrize("p,precision,size", [(p, f, n) for p, f, ns in SWITCHES for n in ns])
+def test_tile_switches(p, precision, size):
+    against_plain_scheme(*size, p, "ader" if size[0] % 2 else "rk3", precision, steps=3)
