@@ -104,7 +104,10 @@ struct Ind2Pass {
     double rk_a;
 };
 
-template <typename R, int P, int TX, int TY, int MODE>
+// HANG: tiles at the high edges hang over the domain; their outside elements
+// are periodic images, evaluated and not stored. Counts that the tile divides
+// run without that code (100^2 p=3 FP32 step 113 -> 97 us, 256^2 p=2 FP64 5 %).
+template <typename R, int P, int TX, int TY, int MODE, bool HANG>
 __global__ void __launch_bounds__(256, 3) ind2_pass(Ind2Geo G, Ind2Mats<R> M, Ind2Pass A) {
     using T = Ind2Tile<R, P, TX, TY>;
     constexpr int n = T::n, nf = T::nf, FB = T::FB, NS = T::NS, SX = T::SX, NE = T::NE, IPT = T::IPT;
@@ -126,15 +129,22 @@ __global__ void __launch_bounds__(256, 3) ind2_pass(Ind2Geo G, Ind2Mats<R> M, In
         Msf[i] = M.sp_to_fp[i];
         Mdf[i] = M.dfp_to_sp[i];
     }
-    // tiles at the high edges may hang over the domain: their outside elements
-    // are periodic images, evaluated and not stored
-    const int tiles_x = (G.N[0] + TX - 1) / TX;
+    const int tiles_x = HANG ? (G.N[0] + TX - 1) / TX : G.N[0] / TX;
     const int i0 = (int)(blockIdx.x % tiles_x) * TX, j0 = (int)(blockIdx.x / tiles_x) * TY;
     for (int s = tid; s < NS; s += 256) {
-        const int i = (i0 + s % SX - 1 + G.N[0]) % G.N[0], j = (j0 + s / SX - 1 + G.N[1]) % G.N[1];
+        int i = i0 + s % SX - 1, j = j0 + s / SX - 1;
+        if (HANG) {
+            i = (i + G.N[0]) % G.N[0];
+            j = (j + G.N[1]) % G.N[1];
+        } else {
+            if (i < 0) i += G.N[0];
+            if (i >= G.N[0]) i -= G.N[0];
+            if (j < 0) j += G.N[1];
+            if (j >= G.N[1]) j -= G.N[1];
+        }
         sl_el[s] = j * G.N[0] + i;
     }
-    const bool whole = i0 + TX <= G.N[0] && j0 + TY <= G.N[1];
+    const bool whole = !HANG || (i0 + TX <= G.N[0] && j0 + TY <= G.N[1]);
     const R vx = (R)G.v[0], vy = (R)G.v[1];
     const int nt = G.nt;
     const int nt_eval = A.in_slices > 1 ? nt : 1;
@@ -370,7 +380,7 @@ void fill_mats(const Matrices& m, int nt, Ind2Mats<R>* M) {
 // one step's launches (src/induction_ader.hpp:351-385): per stage, the
 // Picard passes (ADER: nt - 1 predictor passes, then the corrector; SSP-RK:
 // the corrector of a single slice) on tiles of TX x TY elements
-template <typename R, int P, int TX, int TY>
+template <typename R, int P, int TX, int TY, bool HANG>
 int enqueue_t(spdk_induction2d* s) {
     using T = Ind2Tile<R, P, TX, TY>;
     Ind2Mats<R> M;
@@ -380,8 +390,8 @@ int enqueue_t(spdk_induction2d* s) {
     const size_t state = (size_t)E * T::FB;
     const size_t smem = (size_t)T::TOTAL * sizeof(R);
     cudaStream_t st = s->stream;
-    auto kp = ind2_pass<R, P, TX, TY, kInd2Predict>;
-    auto kc = ind2_pass<R, P, TX, TY, kInd2Correct>;
+    auto kp = ind2_pass<R, P, TX, TY, kInd2Predict, HANG>;
+    auto kc = ind2_pass<R, P, TX, TY, kInd2Correct, HANG>;
     if (cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return fail(SPDK_E_CUDA, "induction2d: shared memory request of " + std::to_string(smem) + " bytes");
@@ -449,18 +459,19 @@ int enqueue_t(spdk_induction2d* s) {
 // 2 x 2 (p = 2 to 4): up to 4 blocks per SM at p = 2, 6 above, 9 in FP32 at p = 4.
 //   48^2 against 4 x 4: p=2 FP64 0.73 / 1.02, p=4 FP64 0.77 / 1.01 of the time on 4 x 4 tiles;
 //   64^2: p=2 1.13 / 1.07, p=3 1.27 / 1.01, p=4 1.08 / 1.02, p=4 FP32 0.85 / 1.01 (80^2: 1.06 / 1.00).
-// p = 1 is launch latency on any tile.
+// p = 1: launch latency on any tile up to 24^2, 4 x 4 beyond (64^2 FP64: 18.5 / 12 us).
 template <typename R, int P>
 int enqueue2(spdk_induction2d* s) {
     constexpr bool f32 = sizeof(R) == 4;
     constexpr int kSMs = 148;
     const int* N = s->cfg.N;
     auto blocks = [&](int T) { return (long long)((N[0] + T - 1) / T) * ((N[1] + T - 1) / T); };
+    if (blocks(1) <= kSMs * (f32 && P > 5 ? 4 : 3)) return enqueue_t<R, P, 1, 1, false>(s);
     if constexpr (P > 1) {
-        if (blocks(1) <= kSMs * (f32 && P > 5 ? 4 : 3)) return enqueue_t<R, P, 1, 1>(s);
-        if (P > 4 || blocks(2) <= kSMs * (P == 2 ? 4 : (f32 && P == 4 ? 9 : 6))) return enqueue_t<R, P, 2, 2>(s);
+        if (P > 4 || blocks(2) <= kSMs * (P == 2 ? 4 : (f32 && P == 4 ? 9 : 6)))
+            return N[0] % 2 || N[1] % 2 ? enqueue_t<R, P, 2, 2, true>(s) : enqueue_t<R, P, 2, 2, false>(s);
     }
-    if constexpr (P <= 4) return enqueue_t<R, P, 4, 4>(s);
+    if constexpr (P <= 4) return N[0] % 4 || N[1] % 4 ? enqueue_t<R, P, 4, 4, true>(s) : enqueue_t<R, P, 4, 4, false>(s);
 }
 
 template <typename R>

@@ -128,7 +128,7 @@ def test_counts_that_no_tile_divides(N, p, integrator):
 # both sides of every switch between one-element, 2 x 2 and 4 x 4 tiles
 SWITCHES = [(2, "fp64", [(21, 21), (22, 21), (47, 48), (50, 47)]), (3, "fp64", [(21, 21), (23, 20), (58, 59), (59, 60)]),
             (4, "fp64", [(21, 21), (22, 21), (59, 58), (59, 60)]), (4, "fp32", [(21, 21), (22, 21), (73, 72), (74, 73)]),
-            (6, "fp64", [(21, 21), (22, 21)]), (7, "fp32", [(24, 24), (25, 24)]), (1, "fp32", [(3, 2), (33, 34)])]
+            (6, "fp64", [(21, 21), (22, 22)]), (7, "fp32", [(24, 24), (25, 24)]), (1, "fp32", [(3, 2), (33, 36), (36, 32)])]
 
 
 @pytest.mark.parametrize("p,precision,size", [(p, f, n) for p, f, ns in SWITCHES for n in ns])
