@@ -98,15 +98,16 @@ constexpr int flux_stride() {
 // Phase A: the x lines, then the y lines (each padded to whole warps, so that
 // a warp runs one direction), then the interfaces on the tile's high edges.
 // Phase B: rows of points x H groups of variables.
-// A thread has registers for either the predictor's sums or the flux
-// evaluation at the occupancy that hides its latency, so the predictor keeps
-// the sums in shared memory (one private column per thread). A pass has one
-// staging and one flux-point buffer: the next slice's copy starts when phase
-// A is over and runs under phase B, and the shared memory saved is more
-// resident blocks. Measured per predictor pass at 256^2, p = 3 (the average of
-// a step's three): FP64 260 us with the sums in registers (3 blocks, 356
-// bytes of spills), 198 us in shared memory (3 blocks); FP32 87 us in
-// registers (4 blocks), 84 us in shared memory (6).
+// A thread has registers for either the predictor's divergences of every slice
+// or the flux evaluation at the occupancy that hides its latency, so the
+// predictor keeps the divergences in shared memory (one private column per
+// thread) and forms the sums over slices once, at the end: 4 nt accesses a
+// point. (Summing as the slices pass rewrites every sum in every slice, 2 nt^2
+// accesses, which outweigh the FP64 arithmetic from p = 4 on: 128^2 steps without
+// the fallback, p=5 FP64 1744 -> 1498 us, p=5 FP32 678 -> 550 us, p=7 FP32 2052 ->
+// 1615 us, 64^2 p=4 FP64 298 -> 248 us.) A pass has one staging and one flux-point
+// buffer: the next slice's copy starts when phase A is over and runs under
+// phase B, and the shared memory saved is more resident blocks.
 template <typename R, int P, int TX, int TY, int MODE>
 struct Line2 {
     static constexpr int n = P + 1, nf = P + 2, V = 4, NPT = n * n, NFP = n * nf, NE = TX * TY;
@@ -140,14 +141,16 @@ template <int P> constexpr int kLineTY = P <= 3 ? 4 : 2;
 
 // resident blocks per SM the 2D pass's registers are sized for
 // (threads x blocks leave 64 registers a thread at p = 3 in FP32 and 96 to 128
-// in FP64, where spills stay below 40 bytes; FP64 flux pass at p = 3: 347 us
-// at 3 blocks, 304 us at 4; FP32 with double buffers at 5 blocks 138 us,
-// single at 5 and 6 134 and 125 us; FP32 predictor at p = 5: 98 us with the sums in
-// registers, 91 / 88 us in shared memory at 5 / 4 blocks)
+// in FP64, where the inviscid predictor spills 24 bytes at most and the corrector
+// 52 to 204; FP64 flux pass at p = 3: 347 us at 3 blocks, 304 us at 4; FP32 with
+// double buffers at 5 blocks 138 us, single at 5 and 6 134 and 125 us; the FP64
+// predictor's shared memory admits one block above p = 5: 128^2 p=7 steps 7100
+// us at the registers of two, 5830 us at those of one)
 template <typename R, int P, int MODE>
 constexpr int kLineBlocksPerSM =
     sizeof(R) == 4 ? (P == 1 ? 8 : P <= 3 ? 6 : P == 4 ? 5 : P == 5 ? 4 : 2)
-                   : (P == 1 ? 5 : P <= 4 ? (MODE == kPredict ? 3 : 4) : P == 5 ? (MODE == kPredict ? 2 : 3) : 2);
+                   : (P == 1 ? 5 : P <= 4 ? (MODE == kPredict ? 3 : 4) : P == 5 ? (MODE == kPredict ? 2 : 3)
+                                                                               : (MODE == kPredict ? 1 : 2));
 
 // the values of one line of one variable's point block: x lines are
 // contiguous, y lines strided by n
@@ -282,9 +285,8 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
     // phase B: row br of variables bv .. bv + VB - 1 of element bel
     const int bh = tid / (NE * n), bel = (tid / n) % NE, br = tid % n, bv = bh * VB;
     const bool brow = tid < LN::ROWS;
-    // kPredict: du of every slice, summed as the slices pass (with gravity
-    // dudt per slice, which the source of the updated state still joins);
-    // kCorrect: du
+    // kPredict: dudt of every slice (of one where all are equal), replaced by
+    // the du of every slice at the end; kCorrect: du
     R dreg[VB][n][LN::shared_sums ? 1 : ND];
     R* sums = smem + LN::m1 + tid;
     auto acc = [&](int k, int i, int tt) -> R& {
@@ -299,13 +301,12 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
     };
     R cy[nf];           // derivative coefficients of the row
     if (MODE != kFlux) {
+        if (MODE == kCorrect) {
 #pragma unroll
-        for (int k = 0; k < VB; k++)
+            for (int k = 0; k < VB; k++)
 #pragma unroll
-            for (int i = 0; i < n; i++)
-#pragma unroll
-                for (int t = 0; t < ND; t++)
-                    if (!LN::shared_sums || brow) acc(k, i, t) = 0;
+                for (int i = 0; i < n; i++) acc(k, i, 0) = 0;
+        }
 #pragma unroll
         for (int ll = 0; ll < nf; ll++) cy[ll] = M.dfp_to_sp[br * nf + ll];
         if constexpr (sizeof(R) == 4) {
@@ -518,19 +519,7 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
 #pragma unroll
                     for (int i = 0; i < n; i++) {
                         if constexpr (MODE == kPredict) {
-                            if (G.grav) {
-#pragma unroll
-                                for (int tt = 0; tt < ND; tt++)
-                                    if (tt == t || !multi) acc(k, i, tt) = dd[i];
-                            } else if (multi) {
-#pragma unroll
-                                for (int tt = 0; tt < ND; tt++) add_term(acc(k, i, tt), dd[i], tt, t);
-                            } else {
-#pragma unroll
-                                for (int tt = 0; tt < ND; tt++)
-#pragma unroll
-                                    for (int ll = 0; ll < ND; ll++) add_term(acc(k, i, tt), dd[i], tt, ll);
-                            }
+                            acc(k, i, t) = dd[i];
                         } else {
                             R dudt = dd[i];
                             if (G.grav && v != 0) {
@@ -603,29 +592,38 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
                         for (int i = 0; i < n; i++) uo[i] = 0;
                     }
                     if (G.grav && v != 0) {
+                        // (from the last slice down: where all are equal, slice 0 holds dudt)
 #pragma unroll
-                        for (int tt = 0; tt < NT; tt++)
+                        for (int tt = NT - 1; tt >= 0; tt--)
 #pragma unroll
                             for (int i = 0; i < n; i++) {
                                 const R* nw = O + ((tt * 3) * NE + bel) * NPT + br * n + i;
                                 R s;
                                 if (v <= D) s = nw[0] * (R)G.g[v - 1];
                                 else s = nw[NE * NPT] * (R)G.g[0] + nw[2 * NE * NPT] * (R)G.g[1];
-                                acc(k, i, tt) -= s;
+                                acc(k, i, tt) = acc(k, i, multi ? tt : 0) - s;
                             }
+                    }
+                    // the sums over slices, in place
+#pragma unroll (n > 4 ? 1 : n)
+                    for (int i = 0; i < n; i++) {
+                        R q[NT];
+#pragma unroll
+                        for (int ll = 0; ll < NT; ll++) q[ll] = acc(k, i, multi || (G.grav && v != 0) ? ll : 0);
+#pragma unroll
+                        for (int tt = 0; tt < NT; tt++) {
+                            R du = 0;
+#pragma unroll
+                            for (int ll = 0; ll < NT; ll++) add_term(du, q[ll], tt, ll);
+                            acc(k, i, tt) = du;
+                        }
                     }
 #pragma unroll
                     for (int tt = 0; tt < NT; tt++) {
                         R val[n];
 #pragma unroll
                         for (int i = 0; i < n; i++) {
-                            R du = 0;
-                            if (G.grav) {
-#pragma unroll
-                                for (int ll = 0; ll < NT; ll++) add_term(du, acc(k, i, ll), tt, ll);
-                            } else {
-                                du = acc(k, i, tt);
-                            }
+                            R du = acc(k, i, tt);
                             if constexpr (sizeof(R) == 4) du *= G.grav ? dt : dt * (R)G.ih[0];
                             val[i] = uo[i] - du;
                         }

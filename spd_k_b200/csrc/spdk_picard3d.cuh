@@ -152,11 +152,9 @@ __device__ __forceinline__ void picard3d_body(const DevGrid& G, const DevMatsT<R
     };
     R cy[nf], cz[nf];
     if (MODE != kFlux) {
-        if (brow) {
+        if (MODE == kCorrect) {
 #pragma unroll
-            for (int i = 0; i < n; i++)
-#pragma unroll
-                for (int t = 0; t < ND; t++) acc(i, t) = 0;
+            for (int i = 0; i < n; i++) acc(i, 0) = 0;
         }
         R ry = 1, rz = 1;  // the precision form scales the sum by 1/h_x alone
         if constexpr (sizeof(R) == 4) {
@@ -335,19 +333,7 @@ __device__ __forceinline__ void picard3d_body(const DevGrid& G, const DevMatsT<R
 #pragma unroll
                 for (int i = 0; i < n; i++) {
                     if constexpr (MODE == kPredict) {
-                        if (G.grav) {
-#pragma unroll
-                            for (int tt = 0; tt < ND; tt++)
-                                if (tt == t || !multi) acc(i, tt) = dd[i];
-                        } else if (multi) {
-#pragma unroll
-                            for (int tt = 0; tt < ND; tt++) add_term(acc(i, tt), dd[i], tt, t);
-                        } else {
-#pragma unroll
-                            for (int tt = 0; tt < ND; tt++)
-#pragma unroll
-                                for (int ll = 0; ll < ND; ll++) add_term(acc(i, tt), dd[i], tt, ll);
-                        }
+                        acc(i, t) = dd[i];
                     } else {
                         R dudt = dd[i];
                         if (G.grav && bv != 0) {
@@ -416,29 +402,38 @@ __device__ __forceinline__ void picard3d_body(const DevGrid& G, const DevMatsT<R
                 R uo[n];
                 row_load<R, n>(A.u + (bge * V + bv) * NPT + br * n, uo);
                 if (G.grav && bv != 0) {
+                    // (from the last slice down: where all are equal, slice 0 holds dudt)
 #pragma unroll
-                    for (int tt = 0; tt < NT; tt++)
+                    for (int tt = NT - 1; tt >= 0; tt--)
 #pragma unroll
                         for (int i = 0; i < n; i++) {
                             const R* nw = O + ((tt * 4) * EB + bel) * NPT + br * n + i;
                             R s;
                             if (bv <= D) s = nw[0] * (R)G.g[bv - 1];
                             else s = nw[EB * NPT] * (R)G.g[0] + nw[2 * EB * NPT] * (R)G.g[1] + nw[3 * EB * NPT] * (R)G.g[2];
-                            acc(i, tt) -= s;
+                            acc(i, tt) = acc(i, multi ? tt : 0) - s;
                         }
+                }
+                // the sums over slices, in place
+#pragma unroll (n > 4 ? 1 : n)
+                for (int i = 0; i < n; i++) {
+                    R q[NT];
+#pragma unroll
+                    for (int ll = 0; ll < NT; ll++) q[ll] = acc(i, multi || (G.grav && bv != 0) ? ll : 0);
+#pragma unroll
+                    for (int tt = 0; tt < NT; tt++) {
+                        R du = 0;
+#pragma unroll
+                        for (int ll = 0; ll < NT; ll++) add_term(du, q[ll], tt, ll);
+                        acc(i, tt) = du;
+                    }
                 }
 #pragma unroll
                 for (int tt = 0; tt < NT; tt++) {
                     R val[n];
 #pragma unroll
                     for (int i = 0; i < n; i++) {
-                        R du = 0;
-                        if (G.grav) {
-#pragma unroll
-                            for (int ll = 0; ll < NT; ll++) add_term(du, acc(i, ll), tt, ll);
-                        } else {
-                            du = acc(i, tt);
-                        }
+                        R du = acc(i, tt);
                         if constexpr (sizeof(R) == 4) du *= G.grav ? dt : dt * (R)G.ih[0];
                         val[i] = uo[i] - du;
                     }

@@ -54,6 +54,23 @@ def test_ragged_counts_match_the_oracle(p, size):
     against_oracle(ov, *random_state(gpu_config(ov), seed=k))
 
 
+# what the draws above leave out: gravity where a thread finishes two variables
+# (p <= 3) and where one does (above), the fallback's RK stages at every kind
+# of tile, and the viscous pass on odd counts
+EXPLICIT = ([(p, size, fb, "ader", "hydro/g2=-0.3") for p in (2, 3) for size in ((5, 3), (9, 7)) for fb in (False, True)] +
+            [(p, (5, 6), fb, "ader", "hydro/g2=-0.3") for p in (1, 5, 6, 7) for fb in (False, True)] +
+            [(p, (7, 5), True, "rk2", "hydro/g1=0.2") for p in (1, 2, 3, 5)] +
+            [(p, size, fb, "ader", "hydro/nu=0.01") for p, fb in ((1, True), (2, False), (3, True), (5, False), (7, True))
+             for size in ((5, 3), (3, 7))] +
+            [(3, (7, 9), True, "rk3", "hydro/nu=0.01")])
+
+
+@pytest.mark.parametrize("p,size,fallback,integrator,extra", EXPLICIT)
+def test_gravity_viscosity_and_stages_on_ragged_counts(p, size, fallback, integrator, extra):
+    ov = overrides(p, *size, ("gradfree", "reflective"), fallback=fallback, integrator=integrator) + [extra]
+    against_oracle(ov, *random_state(gpu_config(ov), seed=zlib.crc32(repr((p, size, extra)).encode())))
+
+
 @pytest.mark.parametrize("p", range(1, 6))
 @pytest.mark.parametrize("size", [(2, 2, 2), (3, 2, 5), (5, 3, 2)])
 def test_ragged_counts_match_the_oracle_3d(p, size):
