@@ -111,13 +111,15 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
 // launches of one step, recorded on h->stream (also used for capture)
 template <typename R>
 int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm) {
-    const unsigned pblocks = picard_grid(k, h->D, h->G.N);
     const unsigned blocks = tile_blocks(h->D, h->G.N, k.tile);
     // the blend's blocks share out the listed tiles
     const unsigned bblocks = std::min(tile_blocks(h->D, h->G.N, k.blend_tile), kBlendGrid);
     const unsigned ublocks = (unsigned)((h->E + k.update_elems - 1) / k.update_elems);
-    const dim3 pthreads(k.picard_threads);
     int launches = 0;
+    auto picard = [&](int mode, const PicardArgsT<R>& A) -> cudaError_t {
+        const PicardLaunch<R> L = picard_launch(k, mode, h->D, h->G.N, h->nt);
+        return launch_pdl(L.kernel, dim3(L.blocks), dim3(L.threads), L.smem, h->stream, h->G, dm, A);
+    };
     // viscous face fluxes of a pass's input, written just before the pass
     auto viscous = [&](PicardArgsT<R>& A) -> int {
         if (!h->vg[0]) return 0;
@@ -161,7 +163,7 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.ua_out = ua[it % 2];
             if (int rc = viscous(A)) return rc;
             prof_begin(h);
-            SPDK_CUDA(launch_pdl(k.predict, dim3(pblocks), pthreads, k.picard_smem[kPredict], h->stream, h->G, dm, A));
+            SPDK_CUDA(picard(kPredict, A));
             prof_end(h, SPDK_KERNEL_PREDICT);
             launches++;
             in = ua[it % 2];
@@ -178,8 +180,7 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.wcv = (R*)h->wcv;
             A.dtmin = h->dtmin;
             prof_begin(h);
-            const auto correct = k.correct_few && pblocks <= kFewBlocks ? k.correct_few : k.correct;
-            SPDK_CUDA(launch_pdl(correct, dim3(pblocks), pthreads, k.picard_smem[kCorrect], h->stream, h->G, dm, A));
+            SPDK_CUDA(picard(kCorrect, A));
             prof_end(h, SPDK_KERNEL_CORRECT);
             launches++;
         } else {
@@ -187,8 +188,9 @@ int enqueue_step_t(spdk_hydro* h, const KernelSetT<R>& k, const DevMatsT<R>& dm)
             A.ucv = ucv[0];
             A.rp_old = h->rpo;
             A.rp_new = h->rpn;
+            A.labels = s == 0 ? h->elem_trouble : nullptr;
             prof_begin(h);
-            SPDK_CUDA(launch_pdl(k.flux, dim3(pblocks), pthreads, k.picard_smem[kFlux], h->stream, h->G, dm, A));
+            SPDK_CUDA(picard(kFlux, A));
             prof_end(h, SPDK_KERNEL_FLUX);
             launches++;
             if (h->join_pending) {
@@ -264,11 +266,6 @@ int refresh_features(spdk_hydro* h) {
 }
 
 int enqueue_step(spdk_hydro* h) {
-    if (h->elem_trouble) {
-        clear_labels_kernel<<<(unsigned)std::min<long long>((h->E + 255) / 256, 1024), 256, 0, h->stream>>>(
-            h->G, h->elem_trouble, h->E);
-        SPDK_CUDA(cudaGetLastError());
-    }
     if (h->mlp) {
         if (int rc = refresh_features(h)) return rc;
         // a-priori flags of the state at the start of the step, on the side
@@ -330,20 +327,18 @@ __global__ void narrow_kernel(const double* __restrict__ a, float* __restrict__ 
 // per-kernel attributes: dynamic shared memory and the full carveout
 template <typename R>
 int set_attributes(const KernelSetT<R>& ks) {
-    const void* fns[] = {(const void*)ks.predict, (const void*)ks.correct, (const void*)ks.flux};
-    for (int m = 0; m < 3; m++) {
-        const void* f = fns[m];
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem[m]) != cudaSuccess)
-            return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(ks.picard_smem[m]) + " bytes");
+    const int rc = each_picard_kernel(ks, [](const void* f, size_t smem) {
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(smem) + " bytes");
         // the whole unified L1/shared array as shared memory: residency is
         // limited by shared memory, not by L1 (staging goes through TMA)
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    }
+        return 0;
+    });
+    if (rc) return rc;
     const std::pair<const void*, size_t> fv[] = {{(const void*)ks.blend, ks.blend_smem},
-                                                 {(const void*)ks.update, ks.update_smem},
-                                                 {(const void*)ks.correct_few, ks.picard_smem[kCorrect]}};
+                                                 {(const void*)ks.update, ks.update_smem}};
     for (const auto& f : fv) {
-        if (!f.first) continue;
         cudaFuncSetAttribute(f.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         if (cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second) != cudaSuccess)
             return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(f.second) + " bytes");
@@ -610,7 +605,7 @@ int spdk_hydro_get_info(const spdk_hydro* h, spdk_hydro_info* info) {
     int l = 0;
     for (int s = 0; s < h->nstages; s++) l += (h->nt - 1) + (h->cfg.fallback ? 1 + 3 * h->nt : 1);
     if (h->vg[0]) l += h->nstages * h->nt;  // a viscous pre-pass before every Picard pass
-    info->launches_per_step = l + 1 + (h->mlp ? 2 : 0) + (h->elem_trouble ? 1 : 0);
+    info->launches_per_step = l + 1 + (h->mlp ? 2 : 0);
     info->device_bytes = h->bytes;
     return 0;
 }

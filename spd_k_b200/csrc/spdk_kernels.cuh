@@ -105,6 +105,7 @@ struct PicardArgsT {
     R* ucv;                // kFlux: U_cv = sp_to_cv(U)
     double2* rp_old;       // kFlux: slice-0 candidate (rho, p) of U_old, FP64
     double2* rp_new;       // kFlux: slice-0 candidate (rho, p) of U_new, FP64
+    uint8_t* labels;       // kFlux: per-element trouble labels, cleared for the detections (nullable)
     R* wcv;                // kCorrect: W_cv output (nullable)
     unsigned long long* dtmin;  // kCorrect: next-dt reduction
     int final_stage;       // kCorrect: compute W_cv and dt
@@ -410,16 +411,16 @@ constexpr int picard_threads() {
     if constexpr (D == 2) return Line2<R, P, TX, TY, kFlux>::threads;
     else return Line3<R, P, kFlux>::threads;
 }
-template <typename R, int D, int P, int MODE>
+template <typename R, int D, int P, int MODE, bool VISC = false>
 constexpr int picard_blocks() {
-    if constexpr (D == 2) return kLineBlocksPerSM<R, P, MODE>;
+    if constexpr (D == 2) return VISC ? kLineBlocksPerSMVisc<R, P, MODE> : kLineBlocksPerSM<R, P, MODE>;
     else return kLine3BlocksPerSM<R, P, MODE>;
 }
 
 // VISC: instantiation that adds the viscous interface fluxes (hydro/nu > 0);
 // the inviscid kernels carry none of that code. (TX, TY: tile of the 2D pass)
 template <typename R, int D, int P, int TX, int TY, int MODE, bool VISC = false>
-__global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_blocks<R, D, P, MODE>())
+__global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_blocks<R, D, P, MODE, VISC>())
     picard_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
     pdl_wait();
     if (gate_closed(G)) return;
@@ -427,16 +428,13 @@ __global__ void __launch_bounds__(picard_threads<R, D, P, TX, TY>(), picard_bloc
     else picard3d_body<R, P, MODE, VISC>(G, M, A, blockIdx.x);
 }
 
-// The corrector for launches of few blocks: compiled for two blocks per SM
-// (no spills, more independent work per warp), because such a launch is one
-// chain of latencies. 32^2 p=3 FP64, 8 steps: 272 -> 262 us; at 256^2 the four
-// blocks of the other one are faster (3.19 against 3.53 ms for 4 steps).
-template <typename R, int P, int TX, int TY>
-__global__ void __launch_bounds__(picard_threads<R, 2, P, TX, TY>(), 2)
-    correct_few_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
+// The 2D pass with a tile, a direction form (RT) and registers of its own
+template <typename R, int P, int TX, int TY, int MODE, bool VISC, bool RT, int BLOCKS>
+__global__ void __launch_bounds__(Line2<R, P, TX, TY, MODE>::threads, BLOCKS)
+    picard2d_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
     pdl_wait();
     if (gate_closed(G)) return;
-    picard2d_body<R, P, TX, TY, kCorrect, false>(G, M, A, blockIdx.x);
+    picard2d_body<R, P, TX, TY, MODE, VISC, RT>(G, M, A, blockIdx.x);
 }
 
 // The 3D corrector on a caller's buffers that start on no 16-byte boundary

@@ -121,13 +121,9 @@ static __global__ void evolve_advance_kernel(double* dt, unsigned long long* dtm
     if (!(t < tb[3])) *gate = 1;
 }
 
-// per-element trouble labels of a step <- 0 (skipped once the gate is closed)
-static __global__ void clear_labels_kernel(DevGrid G, uint8_t* labels, long long n) {
-    pdl_wait();
-    if (gate_closed(G)) return;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        labels[i] = 0;
-}
+constexpr unsigned kSMs = 148;
+// blocks of small tiles at most (picard_launch)
+constexpr unsigned kSmallBlocks = 64;
 
 // ---------------------------------------------------------------------------
 // kernel table of one (R, D, P, tile) instantiation
@@ -137,8 +133,17 @@ struct KernelSetT {
     void (*predict)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*correct)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*flux)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
-    // the corrector of a launch of at most kFewBlocks blocks (null: `correct`)
+    // correctors of the same tile (null: `correct`): of an ADER step and of an
+    // SSP-RK stage on at most few_blocks blocks, and of an SSP-RK stage on more
     void (*correct_few)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
+    void (*correct_rk_few)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
+    void (*correct_rk)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
+    unsigned few_blocks = 0;
+    // passes on small tiles, for at most kSmallBlocks of them (null: none);
+    // [predict, corrector of an ADER step, of an SSP-RK stage]
+    void (*small[3])(DevGrid, DevMatsT<R>, PicardArgsT<R>) = {nullptr, nullptr, nullptr};
+    size_t small_smem[3] = {0, 0, 0};
+    int small_threads = 0, small_tile[3] = {1, 1, 1};
     // the corrector on state buffers that start on no 16-byte boundary (null:
     // `correct` takes them if n is odd, and nothing does if n is even)
     void (*correct_any)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
@@ -167,7 +172,25 @@ KernelSetT<R> make_set() {
     k.predict = picard_kernel<R, D, P, PX, PY, kPredict, VISC>;
     k.correct = picard_kernel<R, D, P, PX, PY, kCorrect, VISC>;
     k.flux = picard_kernel<R, D, P, PX, PY, kFlux, VISC>;
-    if constexpr (D == 2 && sizeof(R) == 8 && P <= 4 && !VISC) k.correct_few = correct_few_kernel<R, P, PX, PY>;
+    if constexpr (D == 2) {
+        constexpr bool f64 = sizeof(R) == 8;
+        if constexpr (f64 && !VISC) {
+            constexpr int few = P <= 4 ? 2 : 1;
+            k.correct_few = picard2d_kernel<R, P, PX, PY, kCorrect, false, false, few>;
+            k.correct_rk_few = picard2d_kernel<R, P, PX, PY, kCorrect, false, true, few>;
+            k.few_blocks = P <= 4 ? 2 * kSMs : 128;
+        }
+        if constexpr (f64) k.correct_rk = picard2d_kernel<R, P, PX, PY, kCorrect, VISC, true, picard_blocks<R, 2, P, kCorrect, VISC>()>;
+        if constexpr (P > 4) {
+            k.small[0] = picard2d_kernel<R, P, 2, 2, kPredict, VISC, false, 1>;
+            k.small[1] = picard2d_kernel<R, P, 2, 2, kCorrect, VISC, false, 1>;
+            k.small[2] = picard2d_kernel<R, P, 2, 2, kCorrect, VISC, f64, 1>;
+            k.small_smem[0] = Line2<R, P, 2, 2, kPredict>::bytes;
+            k.small_smem[1] = k.small_smem[2] = Line2<R, P, 2, 2, kCorrect>::bytes;
+            k.small_threads = Line2<R, P, 2, 2, kPredict>::threads;
+            k.small_tile[0] = k.small_tile[1] = 2;
+        }
+    }
     if constexpr (D == 3 && sizeof(R) == 8 && P % 2 == 1 && !VISC) k.correct_any = correct_any_kernel<R, P>;
     k.picard_threads = picard_threads<R, D, P, PX, PY>();
     k.picard_tile[0] = PX;
@@ -196,11 +219,9 @@ KernelSetT<R> make_set() {
     return k;
 }
 
-// two blocks per SM at once
-constexpr unsigned kFewBlocks = 2 * 148;
-
-// blocks of a blend launch at most: eight per SM share out the listed tiles
-constexpr unsigned kBlendGrid = 8 * 148;
+// blocks of a blend launch at most (two to four per SM are resident and
+// share out the listed tiles, the others find the list done)
+constexpr unsigned kBlendGrid = 8 * kSMs;
 
 // blocks of tiles that cover the domain
 inline unsigned tile_blocks(int D, const int N[3], const int tile[3]) {
@@ -209,12 +230,53 @@ inline unsigned tile_blocks(int D, const int N[3], const int tile[3]) {
     return (unsigned)b;
 }
 
-// blocks of a Picard pass
-template <typename K>
-unsigned picard_grid(const K& k, int D, const int N[3]) {
-    if (!k.picard_elems) return tile_blocks(D, N, k.picard_tile);
+// the launch of a Picard pass of nt slices
+template <typename R>
+struct PicardLaunch {
+    void (*kernel)(DevGrid, DevMatsT<R>, PicardArgsT<R>);
+    unsigned blocks, threads;
+    size_t smem;
+};
+// Which kernel a pass takes. Small tiles (2 x 2 elements above p = 4): a grid of
+// few blocks is a chain of latencies that grows with the elements of a block;
+// 16^2 steps without the fallback on 4 x 2 / 2 x 2 tiles: p=5 FP64 154 / 137 us,
+// p=7 FP64 362 / 317 us, p=5 FP32 97 / 74 us; beyond 64 blocks the device no longer
+// gives each an SM of its own (24^2, 144 blocks: p=5 FP64 186 / 214 us).
+// Few blocks: a corrector compiled for two blocks per SM (above p = 4: one), without
+// spills (32^2 p=3 FP64, 8 steps: 272 -> 262 us; 32^2 p=5 RK3 42.5 -> 41 us), up to
+// what is resident at once; from there the other one's occupancy counts (64 x 72
+// and 80^2, p=3 RK3: 48 / 58 us and 47 / 65 us).
+template <typename R>
+PicardLaunch<R> picard_launch(const KernelSetT<R>& k, int mode, int D, const int N[3], int nt) {
+    if (k.small[0] && mode != kFlux) {
+        const unsigned b = tile_blocks(D, N, k.small_tile);
+        const int i = mode == kPredict ? 0 : (nt > 1 ? 1 : 2);
+        if (b <= kSmallBlocks) return {k.small[i], b, (unsigned)k.small_threads, k.small_smem[i]};
+    }
     const long long E = (long long)N[0] * N[1] * N[2];
-    return (unsigned)((E + k.picard_elems - 1) / k.picard_elems);
+    const unsigned b = k.picard_elems ? (unsigned)((E + k.picard_elems - 1) / k.picard_elems)
+                                      : tile_blocks(D, N, k.picard_tile);
+    auto kernel = mode == kPredict ? k.predict : (mode == kFlux ? k.flux : k.correct);
+    if (mode == kCorrect) {
+        if (b <= k.few_blocks) kernel = nt > 1 ? k.correct_few : k.correct_rk_few;
+        else if (nt == 1 && k.correct_rk) kernel = k.correct_rk;
+    }
+    return {kernel, b, (unsigned)k.picard_threads, k.picard_smem[mode]};
+}
+
+// calls f(kernel, dynamic shared memory) for every Picard kernel of a set
+template <typename R, typename F>
+int each_picard_kernel(const KernelSetT<R>& k, F f) {
+    const struct { void (*kernel)(DevGrid, DevMatsT<R>, PicardArgsT<R>); size_t smem; } all[] = {
+        {k.predict, k.picard_smem[kPredict]}, {k.flux, k.picard_smem[kFlux]},
+        {k.correct, k.picard_smem[kCorrect]}, {k.correct_few, k.picard_smem[kCorrect]},
+        {k.correct_rk, k.picard_smem[kCorrect]}, {k.correct_rk_few, k.picard_smem[kCorrect]},
+        {k.correct_any, k.picard_smem[kCorrect]}, {k.small[0], k.small_smem[0]},
+        {k.small[1], k.small_smem[1]}, {k.small[2], k.small_smem[2]}};
+    for (const auto& a : all)
+        if (a.kernel)
+            if (int rc = f((const void*)a.kernel, a.smem)) return rc;
+    return 0;
 }
 
 // element widths, their reciprocals and powers of two (G.N, D and the box

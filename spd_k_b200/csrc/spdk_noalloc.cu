@@ -83,16 +83,13 @@ int setup_device(int dev, const KernelSet& ks, void** base) {
         g_scratch_ptr[dev] = p;
     }
     // per-kernel attributes (idempotent, not an allocation)
-    const struct { const void* f; int mode; } fns[] = {{(const void*)ks.predict, kPredict},
-                                                       {(const void*)ks.correct, kCorrect},
-                                                       {(const void*)ks.correct_any, kCorrect}};
-    for (const auto& k : fns) {
-        const void* f = k.f;
-        if (!f) continue;
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ks.picard_smem[k.mode]);
+    const int rc = each_picard_kernel(ks, [](const void* f, size_t smem) {
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    }
+        return 0;
+    });
+    if (rc) return rc;
     *base = g_scratch_ptr[dev];
     return 0;
 }
@@ -185,8 +182,9 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
     G.status = status;
 
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned blocks = picard_grid(ks, D, N);
-    const auto correct = ks.correct_any && (off(u_in, 16) || off(u_out, 16)) ? ks.correct_any : ks.correct;
+    const PicardLaunch<double> predict = picard_launch(ks, kPredict, D, N, nt);
+    PicardLaunch<double> correct = picard_launch(ks, kCorrect, D, N, nt);
+    if (ks.correct_any && (off(u_in, 16) || off(u_out, 16))) correct.kernel = ks.correct_any;
     noalloc_arm<<<1, 1, 0, s>>>(dtmin, status);
     double rk_a[3] = {0, 0, 0};
     if (c.rk_order == 2) rk_a[1] = 0.5;
@@ -202,7 +200,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
             A.ua_in = in;
             A.in_slices = in_slices;
             A.ua_out = ua[it % 2];
-            ks.predict<<<blocks, ks.picard_threads, ks.picard_smem[kPredict], s>>>(G, dm, A);
+            predict.kernel<<<predict.blocks, predict.threads, predict.smem, s>>>(G, dm, A);
             in = ua[it % 2];
             in_slices = nt;
         }
@@ -212,7 +210,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
         A.final_stage = 1;
         A.wcv = wcv_out;
         A.dtmin = dtmin;
-        correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
+        correct.kernel<<<correct.blocks, correct.threads, correct.smem, s>>>(G, dm, A);
     } else {
         double* stage_in = work;
         double* u0 = work + (size_t)E * V * NPT;
@@ -234,7 +232,7 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
             A.wcv = wcv_out;
             A.dtmin = dtmin;
             A.dt = dt_inout;
-            correct<<<blocks, ks.picard_threads, ks.picard_smem[kCorrect], s>>>(G, dm, A);
+            correct.kernel<<<correct.blocks, correct.threads, correct.smem, s>>>(G, dm, A);
             cur = u_out;
         }
     }

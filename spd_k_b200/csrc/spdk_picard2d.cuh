@@ -151,26 +151,71 @@ constexpr int kLineBlocksPerSM =
     sizeof(R) == 4 ? (P == 1 ? 8 : P <= 3 ? 6 : P == 4 ? 5 : P == 5 ? 4 : 2)
                    : (P == 1 ? 5 : P <= 4 ? (MODE == kPredict ? 3 : 4) : P == 5 ? (MODE == kPredict ? 2 : 3)
                                                                                : (MODE == kPredict ? 1 : 2));
+// (viscous passes carry the interface's viscous fluxes too)
+template <typename R, int P, int MODE>
+constexpr int kLineBlocksPerSMVisc =
+    sizeof(R) == 4 ? (P == 1 ? 6 : P <= 3 ? 4 : P == 4 ? 4 : P == 5 ? 3 : 2)
+                   : (P == 1 ? 4 : P <= 4 ? (MODE == kPredict ? 2 : 3) : P == 5 ? 2 : 1);
 
-// the values of one line of one variable's point block: x lines are
-// contiguous, y lines strided by n
-template <typename R, int n, int d>
-__device__ __forceinline__ void load_line(const R* src, int tp, R (&u)[n]) {
-    if constexpr (d == 0) row_load<R, n>(src + n * tp, u);
+// The values of one line of one variable's point block: x lines are
+// contiguous, y lines strided by n.
+//
+// The direction of the code below is a value: a compile-time one in the passes
+// of several slices (x lines as vectors, no selects), or one that differs
+// between warps (RT), which halves the code a pass fetches: a single-slice
+// SSP-RK stage runs it once, from a cold instruction cache (64^2 p=2 FP64 RK3
+// steps 41 -> 39 us, 128^2 p=6 304 -> 276 us; the predictor is up to 1.3 times
+// slower so, its slices find the code cached).
+template <bool RT, typename R, int n>
+__device__ __forceinline__ void load_line(int d, const R* src, int tp, R (&u)[n]) {
+    if (!RT && d == 0) row_load<R, n>(src + n * tp, u);
     else {
+        const R* p = src + (d == 0 ? n * tp : tp);
+        const int st = d == 0 ? 1 : n;
 #pragma unroll
-        for (int l = 0; l < n; l++) u[l] = src[tp + n * l];
+        for (int l = 0; l < n; l++) u[l] = p[l * st];
     }
+}
+template <typename R>
+__device__ __forceinline__ R along2(const R* w, int d) { return d == 0 ? w[0] : w[1]; }
+
+// euler_flux and riemann_llf of that direction, and the mirrored state
+template <typename R>
+__device__ __forceinline__ void euler_flux2(const R* u, const R* w, R* f, int d) {
+    const R vn = along2(w + 1, d);
+    f[0] = u[0] * vn;
+#pragma unroll
+    for (int v = 1; v <= 2; v++) f[v] = (v == 1 + d) ? (u[v] * vn + w[3]) : (u[v] * vn);
+    f[3] = (u[3] + w[3]) * vn;
+}
+template <typename R>
+__device__ __forceinline__ void riemann_llf2(R* F, const R* uL, const R* uR, int d, R gm) {
+    R wL[4], wR[4], fL[4], fR[4];
+    primitives<2>(uL, wL, gm);
+    primitives<2>(uR, wR, gm);
+    euler_flux2(uL, wL, fL, d);
+    euler_flux2(uR, wR, fR, d);
+    R cL = sound_speed(wL[0], wL[3], gm) + fabs(along2(wL + 1, d));
+    R cR = sound_speed(wR[0], wR[3], gm) + fabs(along2(wR + 1, d));
+    R cmax = smax(cL, cR);
+#pragma unroll
+    for (int v = 0; v < 4; v++) F[v] = R(0.5) * (fR[v] + fL[v]) - R(0.5) * cmax * (uR[v] - uL[v]);
+}
+template <typename R>
+__device__ __forceinline__ void ghost2(const DevGrid& G, const R* in, R* out, int d) {
+    const bool flip = G.bc[d] == kReflective;
+#pragma unroll
+    for (int v = 0; v < 4; v++) out[v] = (flip && v == 1 + d) ? -in[v] : in[v];
 }
 
 // the state at a line's end: E = 0 low, 1 high
-template <typename R, int P, int d, int END>
-__device__ __forceinline__ void trace2(const DevMatsT<R>& M, const R* src, int tp, R (&t)[4]) {
+template <bool RT, int P, int END, typename R>
+__device__ __forceinline__ void trace2(const DevMatsT<R>& M, int d, const R* src, int tp, R (&t)[4]) {
     constexpr int n = P + 1, NPT = n * n, o = END ? (P + 1) * n : 0;
 #pragma unroll
     for (int v = 0; v < 4; v++) {
         R ul[n];
-        load_line<R, n, d>(src + v * NPT, tp, ul);
+        load_line<RT>(d, src + v * NPT, tp, ul);
         R a = 0;
 #pragma unroll
         for (int l = 0; l < n; l++) a += ul[l] * M.sp_to_fp[o + l];
@@ -181,21 +226,13 @@ __device__ __forceinline__ void trace2(const DevMatsT<R>& M, const R* src, int t
 // interface flux between the states of the two sides: the ghost image at a
 // non-periodic domain edge (src/boundary.cpp:48-113), LLF, and in viscous
 // runs the interface sum of the sides' viscous fluxes (src/hydro.cpp:420-455)
-template <typename R, int P, int d, bool VISC>
-__device__ __forceinline__ void interface2(const DevGrid& G, R (&uL)[4], R (&uR)[4], bool ghostL, bool ghostR, R (&F)[4],
-                                           const R* vg, int eL, int eR, int vt, int tp) {
+template <int P, bool VISC, typename R>
+__device__ __forceinline__ void interface2(const DevGrid& G, int d, R (&uL)[4], R (&uR)[4], bool ghostL, bool ghostR,
+                                           R (&F)[4], const R* vg, int eL, int eR, int vt, int tp) {
     constexpr int V = 4, NTP = P + 1;
-    if (ghostL) {
-#pragma unroll
-        for (int v = 0; v < V; v++) uL[v] = uR[v];
-        if (G.bc[d] == kReflective) uL[1 + d] = -uL[1 + d];
-    }
-    if (ghostR) {
-#pragma unroll
-        for (int v = 0; v < V; v++) uR[v] = uL[v];
-        if (G.bc[d] == kReflective) uR[1 + d] = -uR[1 + d];
-    }
-    riemann_llf<2>(F, uL, uR, d, (R)G.gm);
+    if (ghostL) ghost2(G, uR, uL, d);
+    if (ghostR) ghost2(G, uL, uR, d);
+    riemann_llf2(F, uL, uR, d, (R)G.gm);
     if constexpr (VISC) {
         R gL[V], gR[V];
         if (!ghostL) {
@@ -208,22 +245,14 @@ __device__ __forceinline__ void interface2(const DevGrid& G, R (&uL)[4], R (&uR)
 #pragma unroll
             for (int v = 0; v < V; v++) gR[v] = g[v * NTP];
         }
-        if (ghostL) {
-#pragma unroll
-            for (int v = 0; v < V; v++) gL[v] = gR[v];
-            if (G.bc[d] == kReflective) gL[1 + d] = -gL[1 + d];
-        }
-        if (ghostR) {
-#pragma unroll
-            for (int v = 0; v < V; v++) gR[v] = gL[v];
-            if (G.bc[d] == kReflective) gR[1 + d] = -gR[1 + d];
-        }
+        if (ghostL) ghost2(G, gR, gL, d);
+        if (ghostR) ghost2(G, gL, gR, d);
 #pragma unroll
         for (int v = 0; v < V; v++) F[v] += wind_mix(gR[v], gL[v], R(-0.5));
     }
 }
 
-template <typename R, int P, int TX, int TY, int MODE, bool VISC>
+template <typename R, int P, int TX, int TY, int MODE, bool VISC, bool RT = false>
 __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R>& M, const PicardArgsT<R>& A,
                                               long long bidx) {
     constexpr int D = 2;
@@ -346,11 +375,11 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         const bool check = MODE != kFlux && sizeof(R) == 8 && !G.uniform_pow2;
         const int vt = multi ? t : 0;
         auto line = [&](auto dir, int q) {
-            constexpr int d = decltype(dir)::value;
+            const int d = dir;
             // x lines: 8 elements, then their rows (16-byte loads of 8 lanes
             // fall into distinct banks); y lines: an element's columns first
             int el, r;
-            if constexpr (d == 0 && NE % 8 == 0) { el = (q & 7) + 8 * (q / (8 * n)); r = (q >> 3) % n; }
+            if (NE % 8 == 0 && d == 0) { el = (q & 7) + 8 * (q / (8 * n)); r = (q >> 3) % n; }
             else { el = q / n; r = q % n; }
             const int lx = el % TX, ly = el / TX;
             const int sN = d == 0 ? TL::slot(lx - 1, ly, 0) : TL::slot(lx, ly - 1, 0);
@@ -361,14 +390,14 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             const bool ghostL = edge && gface == 0, ghostR = edge && gface == G.N[d];
             const R* src = Ss + el * SS;
             R* dst = FX + d * NE * FE + el * FE + (d == 0 ? r * nf : r);
-            constexpr int st = d == 0 ? 1 : n;  // stride between the line's flux points
+            const int st = d == 0 ? 1 : n;  // stride between the line's flux points
             // the plain form reads the line again after the interface instead
             // of holding it across, for its registers
             constexpr bool hold = sizeof(R) == 4;
             R ul[V][n];
             auto load = [&]() {
 #pragma unroll
-                for (int v = 0; v < V; v++) load_line<R, n, d>(src + v * NPT, r, ul[v]);
+                for (int v = 0; v < V; v++) load_line<RT>(d, src + v * NPT, r, ul[v]);
             };
             if (hold) load();
             {
@@ -382,10 +411,10 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
                         uR[v] = a;
                     }
                 } else if (!ghostR) {
-                    trace2<R, P, d, 0>(M, src, r, uR);
+                    trace2<RT, P, 0>(M, d, src, r, uR);
                 }
-                if (!ghostL) trace2<R, P, d, 1>(M, Ss + sN * SS, r, uL);
-                interface2<R, P, d, VISC>(G, uL, uR, ghostL, ghostR, F, A.vg[d], VISC ? sl_elem[sN] : 0,
+                if (!ghostL) trace2<RT, P, 1>(M, d, Ss + sN * SS, r, uL);
+                interface2<P, VISC>(G, d, uL, uR, ghostL, ghostR, F, VISC ? along2(A.vg, d) : nullptr, VISC ? sl_elem[sN] : 0,
                                           VISC ? sl_elem[el] : 0, vt, r);
                 R* dl = FX + d * NE * FE + sN * FE + (d == 0 ? r * nf : r) + (nf - 1) * st;
                 const bool inside = d == 0 ? lx > 0 : ly > 0;
@@ -409,7 +438,7 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
                     u[v] = a;
                 }
                 primitives<2>(u, w, (R)G.gm);
-                euler_flux<2>(u, w, f, d);
+                euler_flux2(u, w, f, d);
 #pragma unroll
                 for (int v = 0; v < V; v++) {
                     dst[v * NFP + ll * st] = f[v];
@@ -418,7 +447,7 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             }
         };
         auto edge = [&](auto dir, int q) {
-            constexpr int d = decltype(dir)::value;
+            const int d = dir;
             const int r = q % n, k = q / n;
             const int el = d == 0 ? (TX - 1) + TX * k : k + TX * (TY - 1);
             const int sN = d == 0 ? TL::slot(TX, k, 0) : TL::slot(k, TY, 0);
@@ -426,9 +455,9 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             if (gface > G.N[d] || o[1 - d] + k >= G.N[1 - d]) return;
             const bool ghostR = G.bc[d] != kPeriodic && gface == G.N[d];
             R uL[V], uR[V], F[V];
-            trace2<R, P, d, 1>(M, Ss + el * SS, r, uL);
-            if (!ghostR) trace2<R, P, d, 0>(M, Ss + sN * SS, r, uR);
-            interface2<R, P, d, VISC>(G, uL, uR, false, ghostR, F, A.vg[d], VISC ? sl_elem[el] : 0,
+            trace2<RT, P, 1>(M, d, Ss + el * SS, r, uL);
+            if (!ghostR) trace2<RT, P, 0>(M, d, Ss + sN * SS, r, uR);
+            interface2<P, VISC>(G, d, uL, uR, false, ghostR, F, VISC ? along2(A.vg, d) : nullptr, VISC ? sl_elem[el] : 0,
                                       VISC ? sl_elem[sN] : 0, vt, r);
             R* dst = FX + d * NE * FE + el * FE + (d == 0 ? r * nf + nf - 1 : r + n * (nf - 1));
 #pragma unroll
@@ -439,7 +468,15 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
         };
         using D0 = std::integral_constant<int, 0>;
         using D1 = std::integral_constant<int, 1>;
-        if (tid < LN::LW) {
+        if constexpr (RT) {
+            if (tid < 2 * LN::LW) {
+                const int d = tid >= LN::LW, q = tid - d * LN::LW;
+                if (LN::LW == LN::LINES || q < LN::LINES) line(d, q);
+            } else if (tid < 2 * LN::LW + LN::EDGE0 + LN::EDGE1) {
+                const int q = tid - 2 * LN::LW, d = q >= LN::EDGE0;
+                edge(d, q - d * LN::EDGE0);
+            }
+        } else if (tid < LN::LW) {
             if (LN::LW == LN::LINES || tid < LN::LINES) line(D0{}, tid);
         } else if (tid < 2 * LN::LW) {
             if (LN::LW == LN::LINES || tid < LN::LW + LN::LINES) line(D1{}, tid - LN::LW);
@@ -702,6 +739,9 @@ __device__ __forceinline__ void picard2d_body(const DevGrid& G, const DevMatsT<R
             block_min_dt(dtl, A.dtmin);
         }
     } else {
+        if (A.labels)
+            for (int el = tid; el < NE; el += NTH)
+                if (el_own[el] >= 0) A.labels[el_own[el]] = 0;
         // ---- U_cv = sp_to_cv(U) and the slice-0 FV candidate: a thread
         // averages its rows in x, then, from the rows' x averages, in y ----
         R* Tx = smem;                      // [NE][V][NPT]

@@ -507,6 +507,7 @@ __device__ __forceinline__ void picard3d_body(const DevGrid& G, const DevMatsT<R
                 block_min_dt(dtl, A.dtmin);
             }
         } else {
+            if (A.labels && tid < ne) A.labels[e0 + tid] = 0;
             // ---- U_cv = sp_to_cv(U) and the slice-0 FV candidate ----
             for (int q = tid; q < ne * V * NPT; q += NTH) B0[q] = A.u[(long long)e0 * V * NPT + q];
             __syncthreads();

@@ -84,6 +84,19 @@ def test_ragged_counts_match_the_oracle_3d(p, size):
     against_oracle(ov, *random_state(gpu_config(ov), seed=k), steps=1 if p == 5 else 2)
 
 
+# both sides of the switches between the 2D passes' kernels: small tiles up to 64
+# of them (above p = 4), correctors for few blocks up to 296 (above p = 4: 128)
+LAUNCHES = [(5, (16, 16), "ader"), (5, (17, 16), "ader"), (5, (16, 17), "rk2"), (7, (16, 16), "rk2"), (6, (17, 15), "rk3"),
+            (7, (33, 31), "rk2"), (6, (31, 34), "ader"), (5, (33, 32), "rk2"), (3, (72, 66), "rk2"), (2, (73, 69), "rk3"),
+            (2, (68, 68), "rk2"), (1, (69, 72), "ader"), (4, (46, 50), "ader"), (4, (51, 49), "rk2")]
+
+
+@pytest.mark.parametrize("p,size,integrator", LAUNCHES)
+def test_both_sides_of_every_kernel_switch(p, size, integrator):
+    ov = overrides(p, *size, ("reflective", "periodic"), fallback=False, integrator=integrator)
+    against_oracle(ov, *random_state(gpu_config(ov), seed=p), steps=1)
+
+
 @pytest.mark.parametrize("scale", [1e-160, 1e-300, 1e80])
 def test_fluxes_too_small_or_large_for_the_reciprocal(scale):
     """momenta (and with them flux values) of this size leave the range in
@@ -95,7 +108,7 @@ def test_fluxes_too_small_or_large_for_the_reciprocal(scale):
     against_oracle(ov, mine, ref5, D, steps=1)
 
 
-@pytest.mark.parametrize("p,size", [(2, (7, 6)), (3, (6, 5)), (5, (5, 7))])
+@pytest.mark.parametrize("p,size", [(2, (7, 6)), (3, (6, 5)), (5, (5, 7)), (5, (17, 18)), (7, (5, 6))])
 def test_precision_form_on_ragged_counts(p, size):
     """FP32 round-off only (as the aligned counts): smooth flow, 4 steps"""
     ov = overrides(p, *size, ("periodic", "periodic"), fallback=False) + ["time/cfl=0.4"]
