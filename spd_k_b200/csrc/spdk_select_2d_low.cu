@@ -3,11 +3,11 @@
 
 namespace spdk {
 
-bool select_2d_low(int p, const int[3], KernelSetT<double>* k, bool visc) {
+bool select_2d_low(int p, const int N[3], KernelSetT<double>* k, bool visc) {
     switch (p) {
-    case 1: return pick2<double, 1>(k, visc);
-    case 2: return pick2<double, 2>(k, visc);
-    case 3: return pick2<double, 3>(k, visc);
+    case 1: return pick2<double, 1>(N, k, visc);
+    case 2: return pick2<double, 2>(N, k, visc);
+    case 3: return pick2<double, 3>(N, k, visc);
     }
     return false;
 }

@@ -84,6 +84,14 @@ def test_ragged_counts_match_the_oracle_3d(p, size):
     against_oracle(ov, *random_state(gpu_config(ov), seed=k), steps=1 if p == 5 else 2)
 
 
+# both sides of the switches between the detection's tiles at p = 4 (148 blocks of
+# 2 x 2 elements)
+@pytest.mark.parametrize("size", [(24, 24), (25, 24)])
+def test_both_detection_tiles(size):
+    ov = overrides(4, *size, ("gradfree", "periodic"))
+    against_oracle(ov, *random_state(gpu_config(ov), seed=size[0]), steps=1)
+
+
 # both sides of the switches between the 2D passes' kernels: small tiles up to 64
 # of them (above p = 4), correctors for few blocks up to 296 (above p = 4: 128)
 LAUNCHES = [(5, (16, 16), "ader"), (5, (17, 16), "ader"), (5, (16, 17), "rk2"), (7, (16, 16), "rk2"), (6, (17, 15), "rk3"),
