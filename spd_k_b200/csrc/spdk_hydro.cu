@@ -58,16 +58,42 @@ int dalloc(spdk_hydro* h, void** p, size_t bytes) {
     return 0;
 }
 
-// the distances of consecutive axis positions with their reciprocals
-int upload_widths(spdk_hydro* h, const std::vector<double>& x, Width** out) {
-    std::vector<Width> w(x.size() - 1);
-    for (size_t i = 0; i + 1 < x.size(); i++) {
-        const double d = x[i + 1] - x[i], r = 1.0 / d;
-        w[i] = Width{d, r, std::fma(-d, r, 1.0) * r, 0.0};
+// the FV axes of the active directions (faces, centres, their distances with
+// reciprocals) in one allocation and one upload
+int upload_axes(spdk_hydro* h) {
+    size_t count = 0;
+    for (int d = 0; d < h->D; d++) count += h->ax[d].fv_faces.size() + h->ax[d].fv_centers.size();
+    std::vector<Width> w;                  // widths first: they are 16-byte vectors
+    std::vector<double> x;
+    w.reserve(count);
+    x.reserve(count);
+    size_t first[3][2][2];                 // [direction][faces, centres][in w, in x]
+    for (int d = 0; d < h->D; d++)
+        for (int k = 0; k < 2; k++) {
+            const std::vector<double>& a = k ? h->ax[d].fv_centers : h->ax[d].fv_faces;
+            first[d][k][0] = w.size();
+            first[d][k][1] = x.size();
+            for (size_t i = 0; i + 1 < a.size(); i++) {
+                const double l = a[i + 1] - a[i], r = 1.0 / l;
+                w.push_back(Width{l, r, std::fma(-l, r, 1.0) * r, 0.0});
+            }
+            x.insert(x.end(), a.begin(), a.end());
+        }
+    const size_t wb = w.size() * sizeof(Width), xb = x.size() * sizeof(double);
+    std::vector<char> host(wb + xb);
+    std::memcpy(host.data(), w.data(), wb);
+    std::memcpy(host.data() + wb, x.data(), xb);
+    if (int rc = dalloc(h, &h->axes, host.size())) return rc;
+    if (cudaMemcpy(h->axes, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(SPDK_E_CUDA, "upload axes");
+    const Width* dw = (const Width*)h->axes;
+    const double* dx = (const double*)((const char*)h->axes + wb);
+    for (int d = 0; d < h->D; d++) {
+        h->G.fw[d] = dw + first[d][0][0];
+        h->G.fd[d] = dw + first[d][1][0];
+        h->G.fvf[d] = dx + first[d][0][1];
+        h->G.fvc[d] = dx + first[d][1][1];
     }
-    if (int rc = dalloc(h, (void**)out, w.size() * sizeof(Width))) return rc;
-    if (cudaMemcpy(*out, w.data(), w.size() * sizeof(Width), cudaMemcpyHostToDevice) != cudaSuccess)
-        return fail(SPDK_E_CUDA, "upload widths");
     return 0;
 }
 
@@ -324,24 +350,28 @@ __global__ void narrow_kernel(const double* __restrict__ a, float* __restrict__ 
         b[i] = (float)a[i];
 }
 
-// per-kernel attributes: dynamic shared memory and the full carveout
+// attributes of the kernels that this run launches: dynamic shared memory, and
+// the whole unified L1/shared array as shared memory (residency is limited by
+// shared memory, not by L1: staging goes through TMA)
 template <typename R>
-int set_attributes(const KernelSetT<R>& ks) {
-    const int rc = each_picard_kernel(ks, [](const void* f, size_t smem) {
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(smem) + " bytes");
-        // the whole unified L1/shared array as shared memory: residency is
-        // limited by shared memory, not by L1 (staging goes through TMA)
-        cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        return 0;
-    });
-    if (rc) return rc;
-    const std::pair<const void*, size_t> fv[] = {{(const void*)ks.blend, ks.blend_smem},
-                                                 {(const void*)ks.update, ks.update_smem}};
-    for (const auto& f : fv) {
-        cudaFuncSetAttribute(f.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+int set_attributes(const spdk_hydro* h, const KernelSetT<R>& ks) {
+    std::vector<std::pair<const void*, size_t>> used;
+    auto picard = [&](int mode) {
+        const PicardLaunch<R> L = picard_launch(ks, mode, h->D, h->G.N, h->nt);
+        used.push_back({(const void*)L.kernel, L.smem});
+    };
+    if (h->nt > 1) picard(kPredict);
+    if (h->cfg.fallback) {
+        picard(kFlux);
+        used.push_back({(const void*)ks.blend, ks.blend_smem});
+        used.push_back({(const void*)ks.update, ks.update_smem});
+    } else {
+        picard(kCorrect);
+    }
+    for (const auto& f : used) {
         if (cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second) != cudaSuccess)
             return fail(SPDK_E_CUDA, "shared memory request of " + std::to_string(f.second) + " bytes");
+        cudaFuncSetAttribute(f.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
     return 0;
 }
@@ -352,9 +382,7 @@ void release(spdk_hydro* h) {
     if (h->graph_evolve) cudaGraphExecDestroy(h->graph_evolve);
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     void* ptrs[] = {h->u, h->ua[0], h->ua[1], h->u0, h->ucv[0], h->ucv[1], h->ff[0], h->ff[1], h->ff[2],
-                    h->blend_mark, h->blend_tiles, h->blend_count, h->fw[0], h->fw[1], h->fw[2], h->fd[0], h->fd[1], h->fd[2],
-                    h->wcv, h->dt, h->fvf[0], h->fvf[1], h->fvf[2], h->fvc[0], h->fvc[1], h->fvc[2],
-                    h->rpo, h->rpn, h->trouble, h->theta, h->dtmin, h->status, h->elem_trouble, h->elem_pred,
+                    h->wcv, h->dt, h->axes, h->rpo, h->rpn, h->flags, h->dtmin, h->status, h->elem_pred,
                     h->feat, h->means, h->vg[0], h->vg[1], h->vg[2], h->gate, h->tb, h->stage};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -508,43 +536,26 @@ int spdk_hydro_create(const spdk_hydro_config* cfg, spdk_hydro** out) {
         if (!rc) rc = dalloc(h, (void**)&h->ucv[1], state);
         if (!rc) rc = dalloc(h, (void**)&h->rpo, (size_t)h->E * h->NPT * sizeof(double2));
         if (!rc) rc = dalloc(h, (void**)&h->rpn, (size_t)h->E * h->NPT * sizeof(double2));
-        if (!rc) rc = dalloc(h, (void**)&h->trouble, (size_t)h->E * h->NPT);
-        if (!rc) rc = dalloc(h, (void**)&h->theta, (size_t)h->E * h->NPT);
+        // the blend list and the flags start out zero: one allocation
         const size_t tiles = tile_blocks(D, G.N, h->prec == SPDK_PRECISION_FP32 ? h->ks32.blend_tile : h->ks64.blend_tile);
-        if (!rc) rc = dalloc(h, (void**)&h->blend_mark, tiles * sizeof(int));
-        if (!rc) rc = dalloc(h, (void**)&h->blend_tiles, tiles * sizeof(int));
-        if (!rc) rc = dalloc(h, (void**)&h->blend_count, sizeof(int));
-        if (!rc && (cudaMemset(h->blend_mark, 0, tiles * sizeof(int)) != cudaSuccess ||
-                    cudaMemset(h->blend_count, 0, sizeof(int)) != cudaSuccess))
-            rc = fail(SPDK_E_CUDA, "memset");
-        if (!rc) rc = dalloc(h, (void**)&h->elem_trouble, (size_t)h->E);
-        if (!rc && cudaMemset(h->elem_trouble, 0, (size_t)h->E) != cudaSuccess) rc = fail(SPDK_E_CUDA, "memset");
+        const size_t cells = (size_t)h->E * h->NPT, ints = (2 * tiles + 1) * sizeof(int);
+        const size_t bytes = ints + 2 * cells + (size_t)h->E;
+        if (!rc) rc = dalloc(h, &h->flags, bytes);
+        if (!rc && cudaMemset(h->flags, 0, bytes) != cudaSuccess) rc = fail(SPDK_E_CUDA, "memset");
+        h->blend_mark = (int*)h->flags;
+        h->blend_tiles = h->blend_mark + tiles;
+        h->blend_count = h->blend_tiles + tiles;
+        h->trouble = (uint8_t*)h->flags + ints;
+        h->theta = h->trouble + cells;
+        h->elem_trouble = h->theta + cells;
         G.elem_trouble = h->elem_trouble;
-        for (int d = 0; d < D && !rc; d++) {
-            rc = dalloc(h, (void**)&h->fvf[d], h->ax[d].fv_faces.size() * sizeof(double));
-            if (!rc) rc = dalloc(h, (void**)&h->fvc[d], h->ax[d].fv_centers.size() * sizeof(double));
-            if (!rc && cudaMemcpy(h->fvf[d], h->ax[d].fv_faces.data(), h->ax[d].fv_faces.size() * sizeof(double),
-                                  cudaMemcpyHostToDevice) != cudaSuccess)
-                rc = fail(SPDK_E_CUDA, "upload fv_faces");
-            if (!rc && cudaMemcpy(h->fvc[d], h->ax[d].fv_centers.data(),
-                                  h->ax[d].fv_centers.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
-                rc = fail(SPDK_E_CUDA, "upload fv_centers");
-            G.fvf[d] = h->fvf[d];
-            G.fvc[d] = h->fvc[d];
-            if (!rc) rc = upload_widths(h, h->ax[d].fv_faces, &h->fw[d]);
-            if (!rc) rc = upload_widths(h, h->ax[d].fv_centers, &h->fd[d]);
-            G.fw[d] = h->fw[d];
-            G.fd[d] = h->fd[d];
-        }
-        if (!rc && cudaMemset(h->trouble, 0, (size_t)h->E * h->NPT) != cudaSuccess)
-            rc = fail(SPDK_E_CUDA, "memset");
-        if (!rc && cudaMemset(h->theta, 0, (size_t)h->E * h->NPT) != cudaSuccess) rc = fail(SPDK_E_CUDA, "memset");
+        if (!rc) rc = upload_axes(h);
     }
     if (!rc && c.nu > 0.0) {
         const size_t vgb = (size_t)h->nt * h->E * 2 * h->V * (h->NPT / h->n) * h->esz;
         for (int d = 0; d < D && !rc; d++) rc = dalloc(h, &h->vg[d], vgb);
     }
-    if (!rc) rc = h->prec == SPDK_PRECISION_FP32 ? set_attributes(h->ks32) : set_attributes(h->ks64);
+    if (!rc) rc = h->prec == SPDK_PRECISION_FP32 ? set_attributes(h, h->ks32) : set_attributes(h, h->ks64);
     if (!rc) {
         // initial condition on the host (transcendentals through the same
         // libm as the reference), U_sp and dt on the device in FP64; the

@@ -35,9 +35,9 @@ struct spdk_hydro {
     void *u = nullptr, *ua[2] = {nullptr, nullptr}, *u0 = nullptr, *ucv[2] = {nullptr, nullptr};
     void *ff[3] = {nullptr, nullptr, nullptr}, *wcv = nullptr;
     double* dt = nullptr;
-    double *fvf[3] = {nullptr, nullptr, nullptr}, *fvc[3] = {nullptr, nullptr, nullptr};
-    Width *fw[3] = {nullptr, nullptr, nullptr}, *fd[3] = {nullptr, nullptr, nullptr};
+    void* axes = nullptr;   // the FV axes that G.fvf, fvc, fw and fd point into
     double2 *rpo = nullptr, *rpn = nullptr;
+    void* flags = nullptr;  // the next five, and elem_trouble
     int *blend_mark = nullptr, *blend_tiles = nullptr, *blend_count = nullptr;  // tiles the troubles reach
     uint8_t *trouble = nullptr, *theta = nullptr;
     unsigned long long* dtmin = nullptr;

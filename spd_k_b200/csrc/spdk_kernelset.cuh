@@ -264,21 +264,6 @@ PicardLaunch<R> picard_launch(const KernelSetT<R>& k, int mode, int D, const int
     return {kernel, b, (unsigned)k.picard_threads, k.picard_smem[mode]};
 }
 
-// calls f(kernel, dynamic shared memory) for every Picard kernel of a set
-template <typename R, typename F>
-int each_picard_kernel(const KernelSetT<R>& k, F f) {
-    const struct { void (*kernel)(DevGrid, DevMatsT<R>, PicardArgsT<R>); size_t smem; } all[] = {
-        {k.predict, k.picard_smem[kPredict]}, {k.flux, k.picard_smem[kFlux]},
-        {k.correct, k.picard_smem[kCorrect]}, {k.correct_few, k.picard_smem[kCorrect]},
-        {k.correct_rk, k.picard_smem[kCorrect]}, {k.correct_rk_few, k.picard_smem[kCorrect]},
-        {k.correct_any, k.picard_smem[kCorrect]}, {k.small[0], k.small_smem[0]},
-        {k.small[1], k.small_smem[1]}, {k.small[2], k.small_smem[2]}};
-    for (const auto& a : all)
-        if (a.kernel)
-            if (int rc = f((const void*)a.kernel, a.smem)) return rc;
-    return 0;
-}
-
 // element widths, their reciprocals and powers of two (G.N, D and the box
 // lengths given), and whether every derivative coefficient is zero or far
 // from under- and overflow (div_const)

@@ -70,7 +70,7 @@ __global__ void noalloc_finish(double* dt, unsigned long long* dtmin, const int*
 
 // once per device, with the device current: the device address of
 // g_scratch (its host-side name is only a shadow) and a zero status word
-int setup_device(int dev, const KernelSet& ks, void** base) {
+int setup_device(int dev, const PicardLaunch<double> (&passes)[3], void** base) {
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     if (dev < 0 || dev >= kMaxDevices) return fail(SPDK_E_ARG, "device ordinal out of range");
     if (!g_scratch_ptr[dev]) {
@@ -83,13 +83,12 @@ int setup_device(int dev, const KernelSet& ks, void** base) {
         g_scratch_ptr[dev] = p;
     }
     // per-kernel attributes (idempotent, not an allocation)
-    const int rc = each_picard_kernel(ks, [](const void* f, size_t smem) {
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (const PicardLaunch<double>& l : passes) {
+        if (!l.kernel) continue;
+        cudaError_t e = cudaFuncSetAttribute((const void*)l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
         if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-        cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        return 0;
-    });
-    if (rc) return rc;
+        cudaFuncSetAttribute((const void*)l.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    }
     *base = g_scratch_ptr[dev];
     return 0;
 }
@@ -140,10 +139,17 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
 
     KernelSet ks;
     if (!select_kernels(D, c.p, N, &ks)) return fail(SPDK_E_ARG, "no kernel instantiation for this ndim/p");
+    // a predictor pass, the corrector, and its form for buffers on 8-byte
+    // boundaries, made ready with it: a later call may need it inside a capture
+    const PicardLaunch<double> whole = picard_launch(ks, kCorrect, D, N, nt);
+    const PicardLaunch<double> passes[3] = {picard_launch(ks, kPredict, D, N, nt), whole,
+                                            {ks.correct_any, whole.blocks, whole.threads, whole.smem}};
+    const PicardLaunch<double>& predict = passes[0];
+    const PicardLaunch<double>& correct = ks.correct_any && (off(u_in, 16) || off(u_out, 16)) ? passes[2] : passes[1];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return fail(SPDK_E_CUDA, "cudaGetDevice failed");
     void* base = nullptr;
-    int rc = setup_device(dev, ks, &base);
+    int rc = setup_device(dev, passes, &base);
     if (rc) return rc;
     unsigned long long* dtmin = (unsigned long long*)base;
     int* status = (int*)((char*)base + sizeof(unsigned long long));
@@ -182,9 +188,6 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
     G.status = status;
 
     cudaStream_t s = (cudaStream_t)stream;
-    const PicardLaunch<double> predict = picard_launch(ks, kPredict, D, N, nt);
-    PicardLaunch<double> correct = picard_launch(ks, kCorrect, D, N, nt);
-    if (ks.correct_any && (off(u_in, 16) || off(u_out, 16))) correct.kernel = ks.correct_any;
     noalloc_arm<<<1, 1, 0, s>>>(dtmin, status);
     double rk_a[3] = {0, 0, 0};
     if (c.rk_order == 2) rk_a[1] = 0.5;
