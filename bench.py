@@ -151,9 +151,12 @@ def algorithmic_bytes(info, fallback, esz=8):
     b["predict"] = (first + (nt - 2) * later) / max(nt - 1, 1)
     b["correct"] = nt * S + S + S + S                    # U_ader, U (r+w), W_cv
     b["flux"] = nt * S + S + nt * ff_slice + S + 2 * cells * 16   # U_ader, U, FF, U_cv, candidates
-    b["detect"] = 2 * cells * 16 + cells                  # (rho,p) candidates -> flags
-    b["theta"] = cells + cells
-    b["update"] = S + ff_slice + cells + S + (2 * cells * 16 if True else 0)
+    b["detect"] = 2 * cells * 16 + 2 * cells              # (rho,p) candidates -> flags, theta cleared
+    # "theta" (the blend kernel) has no fixed traffic: it follows the listed tiles
+    # the update, averaged over the slices: U_cv and the slice's faces in; all
+    # but the last also take the next slice's faces and leave U_cv and its
+    # candidates, the last leaves U and W_cv
+    b["update"] = S + ff_slice + ((nt - 1) * (ff_slice + S + 2 * cells * 16) + 2 * S) / nt
     return b
 
 
