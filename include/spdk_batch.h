@@ -7,14 +7,14 @@
  * looks up its problem in a table and runs the single-problem kernel body
  * on it), the groups run concurrently on their own streams, and the whole
  * step is captured once as a CUDA graph and replayed. Each problem keeps its
- * own dt (the step count is shared). The tile shape (elements per block) of
- * each group is chosen by spdk_batch_autotune, which times the candidates on
- * the batch itself.
+ * own dt (the step count is shared). The tile of the detection's blocks (1x1,
+ * 2x2 and, for p <= 3, 4x4 elements, whatever the counts) is chosen for each
+ * group by spdk_batch_autotune, which times the candidates on the batch itself.
  *
- * Supported: 2D, ADER, p in {2, 3, 5}, every element count a multiple of the
- * largest candidate tile that divides all of the group (tiles 1x1, 2x2 and,
- * for p <= 3, 4x4), all problems in one precision, fallback on or off for
- * all, no learned indicator. Results are bit-identical to stepping each
+ * Supported: 2D, ADER, p in {2, 3, 5}, even element counts (odd ones are
+ * refused, although the kernels would take them: batches have always been of
+ * even counts), all problems in one precision, fallback on or off for all, no
+ * learned indicator. Results are bit-identical to stepping each
  * problem alone with spdk_hydro_step (labels included).
  */
 #ifndef SPDK_BATCH_H

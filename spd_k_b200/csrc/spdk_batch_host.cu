@@ -469,7 +469,7 @@ int spdk_batch_autotune(spdk_batch* b, int steps) {
         float best = 1e30f;
         int best_tile = g.tile;
         for (int tile : {1, 2, 4}) {
-            if (select_group(b, g, tile)) continue;  // not instantiated / does not divide
+            if (select_group(b, g, tile)) continue;  // not instantiated (4 x 4 above p = 3)
             restore();
             // one untimed step, then `steps` timed steps of this group
             for (int s = 0; s <= steps && !rc; s++) {

@@ -70,32 +70,6 @@ struct DetectArgs {
     BlendList list;      // blend tiles the troubles reach
 };
 
-template <int D, int P>
-__device__ __forceinline__ long long cell_id(const DevGrid& G, const int a[3]) {
-    constexpr int n = P + 1;
-    int e[3] = {0, 0, 0}, c[3] = {0, 0, 0};
-#pragma unroll
-    for (int d = 0; d < D; d++) {
-        e[d] = a[d] / n;
-        c[d] = a[d] - e[d] * n;
-    }
-    const long long ge = ((long long)e[2] * G.N[1] + e[1]) * G.N[0] + e[0];
-    return ge * Shape<D, P>::NPT + pt_index<n>(c);
-}
-
-// image of a possibly-ghost FV coordinate; flips[d] set for reflective images
-template <int D, int P>
-__device__ __forceinline__ long long cell_image(const DevGrid& G, const int a[3], bool flips[3]) {
-    constexpr int n = P + 1;
-    int m[3] = {0, 0, 0};
-#pragma unroll
-    for (int d = 0; d < D; d++) {
-        flips[d] = false;
-        m[d] = fv_image(a[d], G.N[d] * n, G.bc[d], &flips[d]);
-    }
-    return cell_id<D, P>(G, m);
-}
-
 // Cell numbers of a tile and its halo: the number of cell (x, y, z) of the
 // frame that begins H cells outside the tile is x0[x] + x1[y] + x2[z], each
 // part from the cell's image in that direction; a part is kNoCell where there
@@ -166,9 +140,10 @@ __device__ __forceinline__ bool has_image(const DevGrid& G, const int a[3], int 
 
 __device__ __forceinline__ double rp_var(const double2 v, int k) { return k == 0 ? v.x : v.y; }
 
-// elements of a blend block: 64 to 150 sub-cells, so that nearly every one of
-// the block's phases takes its 256 threads one round: a tile's time is a
-// chain of their latencies (4 x 4 elements at p = 3 took twice as long)
+// elements of a blend block: 64 to 144 sub-cells in 2D and 16 to 216 in 3D, so
+// that nearly every one of the block's phases takes its 256 threads one round: a
+// tile's time is a chain of their latencies (4 x 4 elements at p = 3 took twice
+// as long)
 template <int D, int P>
 struct BlendTile {
     static constexpr int X = D == 2 ? (P <= 3 ? 4 : 2) : (P <= 3 ? 2 : 1);
@@ -322,14 +297,6 @@ static __device__ __noinline__ void sed_al_tile_2d(const SedGeom S, const double
 // blocks uncapped: KH 16^3 p=5 FP64 step 11.40 -> 11.28 ms at 3).
 template <int D>
 constexpr int kDetectBlocksPerSM = D == 2 ? 4 : 3;
-// 3D tiles whose candidates on the tile + 3 halo fit the static shared
-// memory beside W_old's tile + 1 halo stage them for the SED stencils
-// (a flagged cell otherwise reads its 45 candidates per variable from
-// global memory); the larger ones keep the global reads
-template <int D, int P, int TX, int TY, int TZ>
-constexpr bool kSedStage3 =
-    D == 3 && ((size_t)(TX * (P + 1) + 6) * (TY * (P + 1) + 6) * (TZ * (P + 1) + 6) +
-               (size_t)(TX * (P + 1) + 2) * (TY * (P + 1) + 2) * (TZ * (P + 1) + 2)) * sizeof(double2) <= 46 * 1024;
 // flagged threads of a block above which it evaluates every alpha of its
 // tile once instead of each flagged cell evaluating its own six
 constexpr int kSedTileThreshold = 24;
@@ -345,13 +312,15 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const De
     constexpr int CPT = (NC + kThreads - 1) / kThreads;  // cells per thread
     static_assert(CPT <= 16, "NAD flag bits");
     constexpr int E3x = Bx + 6, E3y = By + 6, E3z = D == 3 ? Bz + 6 : 1;
-    constexpr bool stage3 = kSedStage3<D, P, TX, TY, TZ>;
+    // (a flagged cell would otherwise read its 45 candidates per variable from global memory)
+    static_assert(D == 2 || (size_t)(E3x * E3y * E3z + E1x * E1y * E1z) * sizeof(double2) <= 46 * 1024,
+                  "the candidates on the tile + 3 halo fit the static shared memory beside W_old's tile + 1 halo");
     const double2* __restrict__ rpo = A.rpo;
     const double2* __restrict__ rpn = A.rpn;
     __shared__ int el_any[NE];
     for (int e = threadIdx.x; e < NE; e += blockDim.x) el_any[e] = 0;
     __shared__ double2 Ro[E1x * E1y * E1z];
-    __shared__ double2 Rn[D == 2 ? E3x * E3y : (stage3 ? E3x * E3y * E3z : 1)];
+    __shared__ double2 Rn[E3x * E3y * E3z];
     __shared__ double Al[D == 2 ? 4 * E1x * E1y : 1];
     __shared__ CellMap<D, P, TX, TY, TZ, 3> map;
     const int dz = D == 3 ? 1 : 0;
@@ -443,29 +412,23 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const De
             if (un > hi || un < lo) nad |= 1u << (2 * r + k);
         }
     }
-    // SED relaxation of the NAD flags (it can only clear one). In 2D, and
-    // in 3D where it fits, the block stages the candidates of the tile + 3
-    // halo once when any of its cells needs it, so a flagged cell reads its
-    // stencils from shared memory instead of a chain of global loads.
+    // SED relaxation of the NAD flags (it can only clear one). The block stages
+    // the candidates of the tile + 3 halo once when any of its cells needs it, so
+    // a flagged cell reads its stencils from shared memory instead of a chain of
+    // global loads.
     const int nflag = G.use_sed ? __syncthreads_count(nad != 0) : 0;
     if (nflag) {
-        if (D == 2 || stage3) {
-            for (int q = threadIdx.x; q < E3x * E3y * E3z; q += blockDim.x) {
-                // (three cells outside a non-periodic boundary: never read)
-                const int id = map.cell(q % E3x, (q / E3x) % E3y, q / (E3x * E3y));
-                Rn[q] = id >= 0 ? rpn[id] : make_double2(0.0, 0.0);
-            }
-            __syncthreads();
+        for (int q = threadIdx.x; q < E3x * E3y * E3z; q += blockDim.x) {
+            // (three cells outside a non-periodic boundary: never read)
+            const int id = map.cell(q % E3x, (q / E3x) % E3y, q / (E3x * E3y));
+            Rn[q] = id >= 0 ? rpn[id] : make_double2(0.0, 0.0);
         }
+        __syncthreads();
         const SedGeom SG = sed_geom<D, P>(G);
-        auto global = [&](const int b[3], int k) {
-            bool fl[3];
-            return rp_var(rpn[cell_image<D, P>(G, b, fl)], k);
-        };
         const bool tile = D == 2 && nflag > kSedTileThreshold;
-        const bool tile3 = stage3 && nflag > kSedTileThreshold;
+        const bool tile3 = D == 3 && nflag > kSedTileThreshold;
         if (tile3) {
-            if constexpr (stage3) {
+            if constexpr (D == 3) {
                 // many flagged cells: every alpha of the tile once per
                 // variable, in the W_old tile's storage (free after NAD),
                 // then each flagged cell takes the min of its own and its
@@ -531,14 +494,8 @@ __device__ __forceinline__ void fv_detect_kernel_body(const DevGrid& G, const De
                         alpha = smin(m0, m1);
                     } else if (D == 2) {
                         alpha = sed_alpha_staged_2d(SG, Rn, E3x, o[0], o[1], a[0], a[1], k);
-                    } else if (stage3) {
-                        alpha = sed_alpha_staged_3d(SG, Rn, E3x, E3y, o, a, k);
                     } else {
-#pragma unroll
-                        for (int d = 0; d < D; d++) {
-                            const double m3 = sed_component(SG, global, a, d, k);
-                            alpha = d == 0 ? m3 : smin(alpha, m3);
-                        }
+                        alpha = sed_alpha_staged_3d(SG, Rn, E3x, E3y, o, a, k);
                     }
                     if (!(alpha < 1)) nad &= ~(1u << (2 * r + k));
                 }

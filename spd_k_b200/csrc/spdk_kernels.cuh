@@ -269,8 +269,9 @@ __device__ __forceinline__ bool div_range(double x) {
 }
 __device__ __forceinline__ bool div_range(float) { return true; }
 
-// x / h for a width of the sub-cell grid: the division's own bits in FP64, a
-// product with the reciprocal in FP32
+// x / h for a width of the sub-cell grid: the division's own bits in FP64 (-0 may
+// come out as +0, a sign that no state, flag or dt depends on), a product with the
+// reciprocal in FP32
 __device__ __forceinline__ double div_width(const DevGrid& G, double x, const Width& w) {
     double q = div_const(x, w.h, w.ih, w.ihl);
     if (!div_range(x) || !G.safe_div) q = x / w.h;

@@ -317,18 +317,18 @@ bool pick3(KernelSetT<R>* k, bool visc) {
 // compiled without FMA contraction (reference rounding), the FP32 units with it
 bool select_2d_low(int p, const int N[3], KernelSetT<double>* k, bool visc);   // p = 1..3
 bool select_2d_high(int p, const int N[3], KernelSetT<double>* k, bool visc);  // p = 4..7
-bool select_3d(int p, const int N[3], KernelSetT<double>* k, bool visc);       // p = 1..5
+bool select_3d(int p, KernelSetT<double>* k, bool visc);                       // p = 1..5
 bool select_f32_2d(int p, const int N[3], KernelSetT<float>* k, bool visc);    // p = 1..7
-bool select_f32_3d(int p, const int N[3], KernelSetT<float>* k, bool visc);    // p = 1..5
+bool select_f32_3d(int p, KernelSetT<float>* k, bool visc);                    // p = 1..5
 
 inline bool select_kernels(int D, int p, const int N[3], KernelSetT<double>* k, bool visc = false) {
     if (D == 2) return p <= 3 ? select_2d_low(p, N, k, visc) : select_2d_high(p, N, k, visc);
-    if (D == 3) return select_3d(p, N, k, visc);
+    if (D == 3) return select_3d(p, k, visc);
     return false;
 }
 inline bool select_kernels(int D, int p, const int N[3], KernelSetT<float>* k, bool visc = false) {
     if (D == 2) return select_f32_2d(p, N, k, visc);
-    if (D == 3) return select_f32_3d(p, N, k, visc);
+    if (D == 3) return select_f32_3d(p, k, visc);
     return false;
 }
 

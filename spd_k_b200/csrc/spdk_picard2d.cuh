@@ -1,7 +1,8 @@
 // Fused Picard pass of 2D runs: one thread per solution-point line.
 //
-// Same inputs, outputs and FP64 arithmetic as picard_kernel_body
-// (spdk_kernels.cuh), organised by lines:
+// Of the slices of U_ader (PicardArgsT): the fluxes at the flux points, LLF at
+// the interfaces, then the predictor's next slices, the corrected state or the
+// FV face fluxes, organised by lines:
 //
 // * Phase A (fluxes at the flux points of one slice). A thread takes one x or
 //   y line of an element, all variables: the line's low interface (its own

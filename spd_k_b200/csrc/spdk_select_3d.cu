@@ -3,7 +3,7 @@
 
 namespace spdk {
 
-bool select_3d(int p, const int[3], KernelSetT<double>* k, bool visc) {
+bool select_3d(int p, KernelSetT<double>* k, bool visc) {
     switch (p) {
     case 1: return pick3<double, 1>(k, visc);
     case 2: return pick3<double, 2>(k, visc);

@@ -4,7 +4,7 @@
 
 namespace spdk {
 
-bool select_f32_3d(int p, const int[3], KernelSetT<float>* k, bool visc) {
+bool select_f32_3d(int p, KernelSetT<float>* k, bool visc) {
     switch (p) {
     case 1: return pick3<float, 1>(k, visc);
     case 2: return pick3<float, 2>(k, visc);

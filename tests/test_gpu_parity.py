@@ -137,12 +137,12 @@ RANDOM_CASES = {
                        "mesh/x3_bc=reflective"],
     "3d_p3_rk2": ["job/fallback=false", "mesh/nx1=2", "mesh/nx2=3", "mesh/nx3=2", "time/integrator=rk2",
                   "hydro/g3=0.3"],
-    # 3D tiles of 2x1x1 elements (p <= 3, even nx1), with the fallback
+    # counts below, at and past the 3D passes' 4 (p = 2) and 2 (p = 3) consecutive
+    # elements and the 2x2x1 detection tiles, with the fallback
     "3d_p3_fallback_tile2": ["job/fallback=true", "mesh/nx1=2", "mesh/nx2=3", "mesh/nx3=2", "mesh/x2_bc=reflective"],
     "3d_p2_fallback_tile2": ["job/fallback=true", "mesh/p=2", "mesh/nx1=4", "mesh/nx2=3", "mesh/nx3=2",
                              "mesh/x1_bc=gradfree"],
-    # FP64 tiles of 2x2x1 elements (p = 2, 3, even nx1 and nx2), with and
-    # without the fallback
+    # whole 2x2x1 detection tiles, with and without the fallback
     "3d_p2_ader_tile22_423": ["job/fallback=false", "mesh/p=2", "mesh/nx1=4", "mesh/nx2=2", "mesh/nx3=3"],
     "3d_p2_fallback_tile22_443": ["job/fallback=true", "mesh/p=2", "mesh/nx1=4", "mesh/nx2=4", "mesh/nx3=3",
                                   "mesh/x2_bc=reflective"],
