@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, kBlendBlocksPerSM<R, D>)
 }
 
 template <typename R, int D, int P>
-__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D>)
+__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D, P>)
     update_batched(const BatchItem<FallbackArgsT<R>>* __restrict__ items, int n, DevMatsT<R> M) {
     long long b;
     const BatchItem<FallbackArgsT<R>>& it = batch_item(items, n, &b, blockIdx.x);

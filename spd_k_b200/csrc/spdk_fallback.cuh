@@ -883,9 +883,13 @@ __global__ void __launch_bounds__(kThreads, kBlendBlocksPerSM<R, D>) fv_blend_ke
 }
 
 // resident blocks the update kernel's registers are sized for (48 registers a
-// thread in FP32, 64 in FP64: no spills in 2D)
-template <typename R, int D>
-constexpr int kUpdateBlocksPerSM = sizeof(R) == 4 ? 5 : 4;
+// thread in FP32, 64 in FP64: 16 bytes of spills at most where the inputs arrive
+// as bulk copies). The 3D orders that gather them, p = 2 and 4, spill 212 to 260
+// bytes there: in FP32 the spills cost more than the fifth block gains (24^3 p=4
+// steps 5576 us at 5 blocks, 5384 us at 4), in FP64 less than the fourth (11454 us
+// at 4, 11690 us at 3)
+template <typename R, int D, int P>
+constexpr int kUpdateBlocksPerSM = sizeof(R) == 8 || (D == 3 && P % 2 == 0) ? 4 : 5;
 
 // elements of an update block: consecutive ones (no neighbour is read), as
 // many as give every thread a sub-cell
@@ -1123,7 +1127,7 @@ __device__ __forceinline__ void fv_update_kernel_body(const DevGrid& G, const De
 }
 
 template <typename R, int D, int P>
-__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D>) fv_update_kernel(DevGrid G, DevMatsT<R> M, FallbackArgsT<R> A) {
+__global__ void __launch_bounds__(kThreads, kUpdateBlocksPerSM<R, D, P>) fv_update_kernel(DevGrid G, DevMatsT<R> M, FallbackArgsT<R> A) {
     pdl_wait();
     if (gate_closed(G)) return;
     fv_update_kernel_body<R, D, P>(G, M, A, blockIdx.x);
