@@ -125,3 +125,25 @@ def test_batch_labels_match_single_solvers():
             nb.record_labels(True)
         finally:
             nb.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_counts_that_hang_over_every_tile(precision):
+    """counts of 2 mod 4 (and of 2 alone), steps before and after the autotuner
+    has tried every detection tile: the single solvers' bits"""
+    import spd_k_b200 as S
+    import spd_k_b200.batch as B
+    cs = [dict(quadrant(N, p, 7 + i), precision=precision)
+          for i, (N, p) in enumerate([((6, 10), 2), ((2, 14), 2), ((10, 6), 3), ((18, 2), 3), ((6, 6), 5), ((14, 10), 5)])]
+    b = B.Batch(cs)
+    singles = [S.HydroSolver(c) for c in cs]
+    for n in (2, 2):
+        b.steps(n)
+        b.sync()
+        for i, s in enumerate(singles):
+            for _ in range(n):
+                s.step()
+            assert same_bits(b.member(i).read(0), s.read(0)) and b.member(i).dt() == s.dt(), (i, n)
+        b.autotune(2)
+    b.close()

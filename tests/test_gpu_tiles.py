@@ -128,3 +128,38 @@ def test_precision_form_on_ragged_counts(p, size):
     assert max(np.abs(b[v] - a[v]).sum() / np.abs(a[v]).sum() for v in range(4)) < 3e-6
     g64.close()
     g32.close()
+
+
+@pytest.mark.parametrize("p,size", [(1, (5, 3)), (2, (5, 7)), (3, (6, 5)), (4, (3, 6)), (5, (5, 3)), (7, (3, 5)),
+                                    (2, (3, 2, 5)), (3, (5, 3, 2)), (4, (3, 2, 3)), (5, (2, 3, 3))])
+def test_precision_form_does_not_see_where_a_tile_ends(p, size):
+    """FP32 with the fallback, from a random state: a periodic box on counts that
+    hang over its tiles against the same box repeated to whole tiles, whose
+    elements then sit elsewhere in theirs. Spacings are 1/8, so that only the
+    sub-cell widths round differently (the last FP64 bit of a difference of
+    faces, seldom one of its FP32 value): a flux difference of relative 6e-8 a
+    step, on values of order one."""
+    D = len(size)
+    reps = (4,) * D if D == 2 else (2,) * D
+
+    def run(N, u):
+        ov = [f"mesh/p={p}", "time/cfl=0.4", "job/fallback=true"]
+        for d in range(3):
+            ov += [f"mesh/nx{d + 1}={N[d] if d < D else 1}", f"mesh/x{d + 1}_bc=periodic",
+                   f"mesh/x{d + 1}len={N[d] / 8 if d < D else 1}"]
+        g = solver(ov, precision="fp32")
+        if u is None:
+            from test_gpu_precision import random_u
+            u = random_u(g, seed=p).astype(np.float32).astype(np.float64)
+        g.write_u(u)
+        for _ in range(2):
+            g.step()
+        out = g.read(0).reshape(*N[::-1], -1)
+        flagged = g.read(4).any()
+        g.close()
+        return u.reshape(*N[::-1], -1), out, flagged
+    start, small, flagged = run(size, None)
+    k = reps[::-1] + (1,)
+    _, large, _ = run(tuple(n * r for n, r in zip(size, reps)), np.tile(start, k))
+    assert flagged
+    assert np.abs(large - np.tile(small, k)).max() <= 2 * 16 * 6e-8 * np.abs(small).max()
