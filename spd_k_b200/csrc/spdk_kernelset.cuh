@@ -244,8 +244,8 @@ struct PicardLaunch {
 // gives each an SM of its own (24^2, 144 blocks: p=5 FP64 186 / 214 us).
 // Few blocks: a corrector compiled for two blocks per SM (above p = 4: one), without
 // spills (32^2 p=3 FP64, 8 steps: 272 -> 262 us; 32^2 p=5 RK3 42.5 -> 41 us), up to
-// what is resident at once; from there the other one's occupancy counts (64 x 72
-// and 80^2, p=3 RK3: 48 / 58 us and 47 / 65 us).
+// what is resident at once; from there the other one's occupancy counts (68 x 72
+// and 80^2, p=3 RK3: 47 / 59 us and 47 / 65 us).
 template <typename R>
 PicardLaunch<R> picard_launch(const KernelSetT<R>& k, int mode, int D, const int N[3], int nt) {
     if (k.small[0] && mode != kFlux) {
