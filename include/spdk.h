@@ -256,8 +256,9 @@ int spdk_fv_faces(int N, int p, double L, int active, double* out, size_t count)
  * SPDK_NOALLOC_SCRATCH_BYTES bytes, held on every GPU that loads the library
  * until exit; problems that need more (ADER: 2(p+1) states, RK: 2 states)
  * are rejected with SPDK_E_ARG. The first call on a device, with that device
- * current, resolves the array's device address and sets kernel attributes:
- * make it before any stream capture. Calls share the array, so calls that
+ * current, resolves the array's device address, and the first of each ndim and
+ * p sets the attributes of the kernels that such steps take: make those before
+ * any stream capture. Calls share the array, so calls that
  * overlap on the GPU race; order them on one stream. No call allocates.
  * Buffers are aligned to their 8-byte values; u_in and u_out start on 16-byte
  * boundaries in 2D at odd p, and u_in in every ADER step in 2D or at odd p

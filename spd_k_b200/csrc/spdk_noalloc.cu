@@ -20,10 +20,10 @@
 //
 // In host code g_scratch names a host-side shadow, not a device address.
 // The first call on each device, with that device current, resolves the
-// real address with cudaGetSymbolAddress and sets the kernels' shared-memory
-// attributes; make that first call before any stream capture. After that a
-// call only enqueues kernels and device-to-device copies on the caller's
-// stream; no call allocates.
+// real address with cudaGetSymbolAddress, and the first of each dimension and
+// order sets its kernels' shared-memory attributes; make those before any
+// stream capture. After that a call only enqueues kernels and device-to-device
+// copies on the caller's stream; no call allocates.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -69,8 +69,12 @@ __global__ void noalloc_finish(double* dt, unsigned long long* dtmin, const int*
 }
 
 // once per device, with the device current: the device address of
-// g_scratch (its host-side name is only a shadow) and a zero status word
-int setup_device(int dev, const PicardLaunch<double> (&passes)[3], void** base) {
+// g_scratch (its host-side name is only a shadow) and a zero status word; and
+// once per device, dimension and order: the attributes of every kernel a step
+// may take, whatever its element counts and buffers, so that no later call
+// readies one (inside a capture, say)
+int setup_device(int dev, int D, int p, const KernelSet& ks, void** base) {
+    static bool ready[kMaxDevices][2][kMaxP + 1] = {};
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     if (dev < 0 || dev >= kMaxDevices) return fail(SPDK_E_ARG, "device ordinal out of range");
     if (!g_scratch_ptr[dev]) {
@@ -82,12 +86,20 @@ int setup_device(int dev, const PicardLaunch<double> (&passes)[3], void** base) 
         if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("scratch status reset: ") + cudaGetErrorString(e));
         g_scratch_ptr[dev] = p;
     }
-    // per-kernel attributes (idempotent, not an allocation)
-    for (const PicardLaunch<double>& l : passes) {
-        if (!l.kernel) continue;
-        cudaError_t e = cudaFuncSetAttribute((const void*)l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
-        if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-        cudaFuncSetAttribute((const void*)l.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (!ready[dev][D - 2][p]) {
+        const size_t c = ks.picard_smem[kCorrect];
+        const struct { void (*kernel)(DevGrid, DevMatsT<double>, PicardArgsT<double>); size_t smem; } all[] = {
+            {ks.predict, ks.picard_smem[kPredict]}, {ks.correct, c}, {ks.correct_few, c}, {ks.correct_rk, c},
+            {ks.correct_rk_few, c}, {ks.correct_any, c}, {ks.small[0], ks.small_smem[0]},
+            {ks.small[1], ks.small_smem[1]}, {ks.small[2], ks.small_smem[2]}};
+        for (const auto& a : all) {
+            if (!a.kernel) continue;
+            const void* f = (const void*)a.kernel;
+            cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.smem);
+            if (e != cudaSuccess) return fail(SPDK_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+            cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        }
+        ready[dev][D - 2][p] = true;
     }
     *base = g_scratch_ptr[dev];
     return 0;
@@ -139,17 +151,13 @@ extern "C" int spdk_hydro_step_noalloc(const spdk_hydro_config* cfg, const doubl
 
     KernelSet ks;
     if (!select_kernels(D, c.p, N, &ks)) return fail(SPDK_E_ARG, "no kernel instantiation for this ndim/p");
-    // a predictor pass, the corrector, and its form for buffers on 8-byte
-    // boundaries, made ready with it: a later call may need it inside a capture
-    const PicardLaunch<double> whole = picard_launch(ks, kCorrect, D, N, nt);
-    const PicardLaunch<double> passes[3] = {picard_launch(ks, kPredict, D, N, nt), whole,
-                                            {ks.correct_any, whole.blocks, whole.threads, whole.smem}};
-    const PicardLaunch<double>& predict = passes[0];
-    const PicardLaunch<double>& correct = ks.correct_any && (off(u_in, 16) || off(u_out, 16)) ? passes[2] : passes[1];
+    const PicardLaunch<double> predict = picard_launch(ks, kPredict, D, N, nt);
+    PicardLaunch<double> correct = picard_launch(ks, kCorrect, D, N, nt);
+    if (ks.correct_any && (off(u_in, 16) || off(u_out, 16))) correct.kernel = ks.correct_any;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return fail(SPDK_E_CUDA, "cudaGetDevice failed");
     void* base = nullptr;
-    int rc = setup_device(dev, passes, &base);
+    int rc = setup_device(dev, D, c.p, ks, &base);
     if (rc) return rc;
     unsigned long long* dtmin = (unsigned long long*)base;
     int* status = (int*)((char*)base + sizeof(unsigned long long));

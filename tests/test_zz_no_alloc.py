@@ -155,3 +155,41 @@ def test_buffers_that_start_on_an_8_byte_boundary(case):
     assert torch.equal(u, start)
     assert pool[1][:oo].count_nonzero() == 0 and pool[1][oo + start.numel():].count_nonzero() == 0
     ref.close()
+
+
+@pytest.mark.parametrize("p,first,later,integ", [(3, (16, 8), (60, 68), "ader"), (2, (8, 8), (74, 76), "rk2"),
+                                                 (5, (4, 4), (20, 18), "ader")])
+def test_a_capture_needs_no_first_call_of_its_own_size(p, first, later, integ):
+    """a step of a small grid readies the order's kernels; a larger grid, which
+    takes others of them, is then captured without a call of its own"""
+    import torch
+
+    import spd_k_b200 as S
+    from spd_k_b200.api import apply_overrides, config_from_params, make_config
+
+    lib = S.load_library()
+    step = bind(lib)
+    stream = torch.cuda.Stream()
+    for N, capture in ((first, False), (later, True)):
+        c = config_from_params(apply_overrides({}, ["job/fallback=false", f"mesh/p={p}", f"mesh/nx1={N[0]}",
+                                                    f"mesh/nx2={N[1]}", "mesh/nx3=1", f"time/integrator={integ}",
+                                                    "problem/problem=kelvin_helmholtz"]))
+        ref, cfg = S.HydroSolver(c), make_config(c)
+        u = torch.from_numpy(ref.read(S.FIELD_U_SP)).cuda()
+        dt = torch.tensor([ref.dt()], dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            return step(ctypes.addressof(cfg), u.data_ptr(), u.data_ptr(), None, dt.data_ptr(), stream.cuda_stream)
+        if capture:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                assert call() == 0, lib.spdk_last_error().decode()
+            with torch.cuda.stream(stream):
+                g.replay()
+        else:
+            assert call() == 0, lib.spdk_last_error().decode()
+        stream.synchronize()
+        ref.step()
+        assert np.array_equal(u.cpu().numpy(), ref.read(S.FIELD_U_SP)) and float(dt.item()) == ref.dt()
+        ref.close()
