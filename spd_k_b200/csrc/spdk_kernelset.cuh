@@ -122,8 +122,6 @@ static __global__ void evolve_advance_kernel(double* dt, unsigned long long* dtm
 }
 
 constexpr unsigned kSMs = 148;
-// blocks of small tiles at most (picard_launch)
-constexpr unsigned kSmallBlocks = 64;
 
 // ---------------------------------------------------------------------------
 // kernel table of one (R, D, P, tile) instantiation
@@ -139,11 +137,12 @@ struct KernelSetT {
     void (*correct_rk_few)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*correct_rk)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     unsigned few_blocks = 0;
-    // passes on small tiles, for at most kSmallBlocks of them (null: none);
+    // passes on small tiles, for at most small_blocks of them (null: none);
     // [predict, corrector of an ADER step, of an SSP-RK stage]
     void (*small[3])(DevGrid, DevMatsT<R>, PicardArgsT<R>) = {nullptr, nullptr, nullptr};
     size_t small_smem[3] = {0, 0, 0};
     int small_threads = 0, small_tile[3] = {1, 1, 1};
+    unsigned small_blocks = 0;
     // the corrector on state buffers that start on no 16-byte boundary (null:
     // `correct` takes them if n is odd, and nothing does if n is even)
     void (*correct_any)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
@@ -181,14 +180,17 @@ KernelSetT<R> make_set() {
             k.few_blocks = P <= 4 ? 2 * kSMs : 128;
         }
         if constexpr (f64) k.correct_rk = picard2d_kernel<R, P, PX, PY, kCorrect, VISC, true, picard_blocks<R, 2, P, kCorrect, VISC>()>;
-        if constexpr (P > 4) {
-            k.small[0] = picard2d_kernel<R, P, 2, 2, kPredict, VISC, false, 1>;
-            k.small[1] = picard2d_kernel<R, P, 2, 2, kCorrect, VISC, false, 1>;
-            k.small[2] = picard2d_kernel<R, P, 2, 2, kCorrect, VISC, f64, 1>;
-            k.small_smem[0] = Line2<R, P, 2, 2, kPredict>::bytes;
-            k.small_smem[1] = k.small_smem[2] = Line2<R, P, 2, 2, kCorrect>::bytes;
-            k.small_threads = Line2<R, P, 2, 2, kPredict>::threads;
-            k.small_tile[0] = k.small_tile[1] = 2;
+        if constexpr (P > 4 || (!f64 && (P == 2 || P == 3))) {
+            constexpr int SX = P > 4 ? 2 : 4, SY = 2, blocks = P > 4 ? 1 : 4;
+            k.small[0] = picard2d_kernel<R, P, SX, SY, kPredict, VISC, false, blocks>;
+            k.small[1] = picard2d_kernel<R, P, SX, SY, kCorrect, VISC, false, blocks>;
+            k.small[2] = picard2d_kernel<R, P, SX, SY, kCorrect, VISC, f64, blocks>;
+            k.small_smem[0] = Line2<R, P, SX, SY, kPredict>::bytes;
+            k.small_smem[1] = k.small_smem[2] = Line2<R, P, SX, SY, kCorrect>::bytes;
+            k.small_threads = Line2<R, P, SX, SY, kPredict>::threads;
+            k.small_tile[0] = SX;
+            k.small_tile[1] = SY;
+            k.small_blocks = P > 4 ? 64 : 512;
         }
     }
     if constexpr (D == 3 && sizeof(R) == 8 && P % 2 == 1 && !VISC) k.correct_any = correct_any_kernel<R, P>;
@@ -241,7 +243,9 @@ struct PicardLaunch {
 // few blocks is a chain of latencies that grows with the elements of a block;
 // 16^2 steps without the fallback on 4 x 2 / 2 x 2 tiles: p=5 FP64 154 / 137 us,
 // p=7 FP64 362 / 317 us, p=5 FP32 97 / 74 us; beyond 64 blocks the device no longer
-// gives each an SM of its own (24^2, 144 blocks: p=5 FP64 186 / 214 us).
+// gives each an SM of its own (24^2, 144 blocks: p=5 FP64 186 / 214 us). In FP32 at
+// p = 2 and 3, whose blocks are shortest, 4 x 2 tiles up to 512 blocks (64^2 on 4 x 4 /
+// 4 x 2: p=2 33 / 28.5 us, RK3 34 / 30.5 us, p=3 50 / 43.5 us; 768 blocks, 96 x 64: p=3 56 / 61 us).
 // Few blocks: a corrector compiled for two blocks per SM (above p = 4: one), without
 // spills (32^2 p=3 FP64, 8 steps: 272 -> 262 us; 32^2 p=5 RK3 42.5 -> 41 us), up to
 // what is resident at once; from there the other one's occupancy counts (68 x 72
@@ -251,7 +255,7 @@ PicardLaunch<R> picard_launch(const KernelSetT<R>& k, int mode, int D, const int
     if (k.small[0] && mode != kFlux) {
         const unsigned b = tile_blocks(D, N, k.small_tile);
         const int i = mode == kPredict ? 0 : (nt > 1 ? 1 : 2);
-        if (b <= kSmallBlocks) return {k.small[i], b, (unsigned)k.small_threads, k.small_smem[i]};
+        if (b <= k.small_blocks) return {k.small[i], b, (unsigned)k.small_threads, k.small_smem[i]};
     }
     const long long E = (long long)N[0] * N[1] * N[2];
     const unsigned b = k.picard_elems ? (unsigned)((E + k.picard_elems - 1) / k.picard_elems)

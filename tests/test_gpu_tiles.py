@@ -116,7 +116,8 @@ def test_fluxes_too_small_or_large_for_the_reciprocal(scale):
     against_oracle(ov, mine, ref5, D, steps=1)
 
 
-@pytest.mark.parametrize("p,size", [(2, (7, 6)), (3, (6, 5)), (5, (5, 7)), (5, (17, 18)), (7, (5, 6))])
+@pytest.mark.parametrize("p,size", [(2, (7, 6)), (3, (6, 5)), (5, (5, 7)), (5, (17, 18)), (7, (5, 6)),
+                                    (2, (63, 63)), (2, (66, 62)), (3, (65, 63))])
 def test_precision_form_on_ragged_counts(p, size):
     """FP32 round-off only (as the aligned counts): smooth flow, 4 steps"""
     ov = overrides(p, *size, ("periodic", "periodic"), fallback=False) + ["time/cfl=0.4"]
