@@ -438,6 +438,16 @@ __global__ void __launch_bounds__(Line2<R, P, TX, TY, MODE>::threads, BLOCKS)
     picard2d_body<R, P, TX, TY, MODE, VISC, RT>(G, M, A, blockIdx.x);
 }
 
+// The 3D pass with all the registers of one block per SM, for launches of at most
+// that many
+template <typename R, int P, int MODE, bool VISC>
+__global__ void __launch_bounds__(Line3<R, P, MODE>::threads, 1)
+    picard3d_kernel(DevGrid G, DevMatsT<R> M, PicardArgsT<R> A) {
+    pdl_wait();
+    if (gate_closed(G)) return;
+    picard3d_body<R, P, MODE, VISC>(G, M, A, blockIdx.x);
+}
+
 // The 3D corrector on a caller's buffers that start on no 16-byte boundary
 template <typename R, int P>
 __global__ void __launch_bounds__(picard_threads<R, 3, P, 1, 1>(), picard_blocks<R, 3, P, kCorrect>())

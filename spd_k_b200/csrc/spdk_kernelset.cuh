@@ -137,7 +137,8 @@ struct KernelSetT {
     void (*correct_rk_few)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     void (*correct_rk)(DevGrid, DevMatsT<R>, PicardArgsT<R>) = nullptr;
     unsigned few_blocks = 0;
-    // passes on small tiles, for at most small_blocks of them (null: none);
+    // passes on small tiles (3D: blocks compiled for one per SM), for at most
+    // small_blocks of them (null: none);
     // [predict, corrector of an ADER step, of an SSP-RK stage]
     void (*small[3])(DevGrid, DevMatsT<R>, PicardArgsT<R>) = {nullptr, nullptr, nullptr};
     size_t small_smem[3] = {0, 0, 0};
@@ -197,7 +198,19 @@ KernelSetT<R> make_set() {
     k.picard_threads = picard_threads<R, D, P, PX, PY>();
     k.picard_tile[0] = PX;
     k.picard_tile[1] = PY;
-    if constexpr (D == 3) k.picard_elems = Line3<R, P, kFlux>::EB;
+    if constexpr (D == 3) {
+        using L3 = Line3<R, P, kFlux>;
+        k.picard_elems = L3::EB;
+        if constexpr (P == 5 || (P == 4 && sizeof(R) == 4)) {
+            static_assert(L3::EB == 1, "blocks of one element, as tile_blocks counts them");
+            k.small[0] = picard3d_kernel<R, P, kPredict, VISC>;
+            k.small[1] = k.small[2] = picard3d_kernel<R, P, kCorrect, VISC>;
+            k.small_smem[0] = Line3<R, P, kPredict>::bytes;
+            k.small_smem[1] = k.small_smem[2] = Line3<R, P, kCorrect>::bytes;
+            k.small_threads = L3::threads;
+            k.small_blocks = kSMs;
+        }
+    }
     k.detect = fv_detect_kernel<R, D, P, TX, TY, TZ>;
     using BT = BlendTile<D, P>;
     k.blend = fv_blend_kernel<R, D, P, BT::X, BT::Y, BT::Z>;
@@ -246,6 +259,9 @@ struct PicardLaunch {
 // gives each an SM of its own (24^2, 144 blocks: p=5 FP64 186 / 214 us). In FP32 at
 // p = 2 and 3, whose blocks are shortest, 4 x 2 tiles up to 512 blocks (64^2 on 4 x 4 /
 // 4 x 2: p=2 33 / 28.5 us, RK3 34 / 30.5 us, p=3 50 / 43.5 us; 768 blocks, 96 x 64: p=3 56 / 61 us).
+// In 3D at p = 5 (FP32 also p = 4) the same blocks of one element compiled for one per
+// SM, while there are no more (4^3: p=5 FP64 226 / 200 us, FP32 129 / 112 us, p=4 FP32
+// 112 / 85 us; 6^3, 216 blocks: p=5 FP64 360 / 513 us).
 // Few blocks: a corrector compiled for two blocks per SM (above p = 4: one), without
 // spills (32^2 p=3 FP64, 8 steps: 272 -> 262 us; 32^2 p=5 RK3 42.5 -> 41 us), up to
 // what is resident at once; from there the other one's occupancy counts (68 x 72

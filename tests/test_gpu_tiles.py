@@ -84,6 +84,15 @@ def test_ragged_counts_match_the_oracle_3d(p, size):
     against_oracle(ov, *random_state(gpu_config(ov), seed=k), steps=1 if p == 5 else 2)
 
 
+# both sides of the switch to one block per SM in 3D (148 elements)
+@pytest.mark.parametrize("p,size,integrator,extra", [(5, (6, 5, 5), "ader", "hydro/g3=-0.3"), (5, (7, 7, 3), "rk2", "hydro/nu=0.01"),
+                                                     (5, (5, 5, 5), "rk3", "hydro/g1=0.2"), (5, (3, 4, 5), "ader", "hydro/nu=0.01")])
+def test_both_3d_launches(p, size, integrator, extra):
+    ov = overrides(p, size[0], size[1], ("gradfree", "reflective"), fallback=False, integrator=integrator) + [extra]
+    ov[3] = f"mesh/nx3={size[2]}"
+    against_oracle(ov, *random_state(gpu_config(ov), seed=p), steps=1)
+
+
 # both sides of the switches between the detection's tiles at p = 4 (148 blocks of
 # 2 x 2 elements)
 @pytest.mark.parametrize("size", [(24, 24), (25, 24)])
@@ -132,7 +141,7 @@ def test_precision_form_on_ragged_counts(p, size):
 
 
 @pytest.mark.parametrize("p,size", [(1, (5, 3)), (2, (5, 7)), (3, (6, 5)), (4, (3, 6)), (5, (5, 3)), (7, (3, 5)),
-                                    (2, (3, 2, 5)), (3, (5, 3, 2)), (4, (3, 2, 3)), (5, (2, 3, 3))])
+                                    (2, (3, 2, 5)), (3, (5, 3, 2)), (4, (3, 2, 3)), (5, (2, 3, 3)), (4, (5, 6, 5))])
 def test_precision_form_does_not_see_where_a_tile_ends(p, size):
     """FP32 with the fallback, from a random state: a periodic box on counts that
     hang over its tiles against the same box repeated to whole tiles, whose
